@@ -1,0 +1,32 @@
+"""The FP64 bond kernels of small lattices (vpd_box64.cu) against the per-slot kernels, bit for bit:
+both sum every point's bonds in slot order with the same operations."""
+import numpy as np
+import pytest
+
+import vpd
+from vpd.case import PRECISION_FP64, tensile_bar
+
+pytestmark = pytest.mark.gpu
+
+FIELDS = ("displacement", "velocity", "stress_corotational", "state", "damage_index", "force_density")
+
+
+# boxes of 32, 64 and 128 points, ragged in every direction; lattices thinner than the stencil; the longest
+# reach whose region fits (6) and the first that does not (7: the tiled kernels); beyond the default's range
+@pytest.mark.parametrize("dims,ratio", [((9, 2, 3), 3.015), ((13, 5, 7), 4.015), ((41, 10, 11), 3.0), ((31, 13, 17), 4.015),
+                                        ((40, 17, 19), 3.015), ((12, 37, 70), 4.015), ((17, 9, 8), 6.015),
+                                        ((17, 9, 8), 7.015)])
+@pytest.mark.parametrize("damage", [0, 1])
+def test_box_kernels_match_slot_kernels_bitwise(monkeypatch, dims, ratio, damage):
+    nx, ny, nz = dims
+    case = tensile_bar(3, nx=nx, ny=ny, nz=nz, horizon=ratio * 0.1, damage_mode=damage, damage_initiation=0.004,
+                       precision=PRECISION_FP64)
+    out = {}
+    for kind in ("slot", "box", "tiles", ""):
+        monkeypatch.setenv("VPD_BOND_KERNEL", kind)
+        with vpd.Simulation(case) as sim:
+            rows = sim.step(150)
+            out[kind] = {f: sim.field(f) for f in FIELDS} | {"rows": rows}
+    for kind in ("box", "tiles", ""):
+        for f, want in out["slot"].items():
+            assert np.array_equal(out[kind][f], want), (kind, f)

@@ -480,11 +480,12 @@ int create_impl(vpd_handle *h, const vpd_case *c, const double *positions, const
   {
     // VPD_BOND_KERNEL=slot selects the per-slot bond kernels (both precisions), scalar the
     // two-point tiled mixed kernels in scalar FP32, tiled2 the two-point FP64 force kernel,
-    // staged the TMA-staged FP64 force kernel (default: tiled; packed pairs when mixed, four
-    // points per thread reading through L1 in the FP64 force)
+    // staged the TMA-staged FP64 force kernel, tiles the tiled FP64 kernels at any size, box the
+    // small-lattice FP64 kernels at any size (default: boxes on small lattices, kBoxPoints, else tiled;
+    // packed pairs when mixed)
     const char *bk = getenv("VPD_BOND_KERNEL");
     const std::string kind = bk ? bk : "";
-    p.tiled = kind == "slot" ? 0 : kind == "scalar" ? 1 : kind == "tiled2" ? 3 : kind == "staged" ? 6 : 2;
+    p.tiled = kind == "slot" ? 0 : kind == "scalar" ? 1 : kind == "tiled2" ? 3 : kind == "staged" ? 6 : kind == "tiles" ? 4 : kind == "box" ? 7 : 2;
     // VPD_RETURN_MAP=bisection: the material kernel evaluates every bisection iteration (the
     // default decides most of them from two anchor evaluations; the results are the same)
     const char *rm = getenv("VPD_RETURN_MAP");
@@ -494,6 +495,8 @@ int create_impl(vpd_handle *h, const vpd_case *c, const double *positions, const
                   (c->precision != VPD_PRECISION_MIXED && (rc = dalloc(h, &p.fmap, 3 * n)))))
     return rc;
   if (p.st.nw && p.fmap && p.tiled == 6 && (rc = setup_staged_force64(p, p.st.rx, p.st.ry, p.st.rz)))
+    return rc;
+  if (p.st.nw && p.fmap && (p.tiled == 7 || (p.tiled == 2 && n <= (c->damage_mode == VPD_DAMAGE_CRITICAL_STRETCH ? kBoxPointsDamage : kBoxPoints))) && (rc = setup_box64(p)))
     return rc;
   p.nstatev = c->nstatev;
   p.flags = h->flags, p.obsw = h->obsw;

@@ -43,6 +43,15 @@ struct StagedTiles {
   uint32_t bytes = 0;                  // box bytes: 3 rows x by x bz x 32
 };
 
+// Boxes of the small-lattice FP64 bond kernels (vpd_box64.cu); threads == 0: not in use.
+struct BoxTiles {
+  int tx = 0, ty = 0, tz = 0;            // a block's box of points
+  int ex = 0, ey = 0, ez = 0, sz = 0;    // its staged region (box plus reach), and its row stride along z
+  int tiles_y = 0, tiles_z = 0, threads = 0;
+  int64_t tiles = 0;
+  int records = 0;                       // of the region, with the row padding
+};
+
 // Lattice-stencil bond layout (vpd_stencil.cu). nw == 0: not in use.
 struct StencilLayout {
   int slots = 0, nw = 0, ngroups = 0;
@@ -71,7 +80,7 @@ struct StepParams {
   double lat_h;               // lattice spacing
   int tiled;                  // bond kernels: 0 per slot; mixed 1 tiled scalar, else packed pairs; FP64
                               // tiled with the 4-point force, 3 with the 2-point force, 6 with the
-                              // TMA-staged force
+                              // TMA-staged force, 4 never the small-lattice boxes, 7 always
   int literal_bisection;      // 1: k_material runs the VUMAT's bisection literally (every iteration
                               // evaluated), 0: jc_return_map (same results)
   // kinematic state
@@ -85,6 +94,7 @@ struct StepParams {
   // fmap[r * n + i] = (VM_r0, VM_r1, VM_r2, X_r), so one bond reads three 32-byte records
   double4 *fmap;
   double4 *vxi;               // sum over all bonds of V_j xi (FP64, set once; stencil layout)
+  BoxTiles box;               // the small-lattice FP64 kernels' boxes
   StagedTiles staged;         // the TMA-staged FP64 force kernel's tiles and box
   CUtensorMap fmap_tmap;      // ... and its tensor map over fmap (lane, z, y, x, row)
   // mixed precision (VPD_PRECISION_MIXED): FP32 copies gathered by the bond kernels
@@ -175,6 +185,16 @@ int launch_force_tiled(const StepParams &p, cudaStream_t s);
 // tiled FP64 bond kernels (vpd_tiled64.cu)
 int launch_deformation_tiled64(const StepParams &p, cudaStream_t s);
 int launch_force_tiled64(const StepParams &p, cudaStream_t s);
+// FP64 bond kernels of small lattices (vpd_box64.cu): setup fills p.box (threads stays 0 when no
+// box's neighbourhood fits shared memory). Default up to kBoxPoints points: beyond, the tiled kernels
+// have enough blocks. Per increment in microseconds, tiled against boxes, at horizons 3.015 h | 4.015 h:
+// 4,000 points 92/43 | 158/62, 10,605 112/57 | 204/91, 20,400 99/95 | 174/154 (168 with 128-point boxes),
+// 27,000 99/98 | 166/167, 54,000 100/138 | 171/241. With bond damage the boxes' stretch tests cost less
+// than the tiles': 4,000 points 117/49 | 208/70, 27,000 128/107 | 223/189, 54,000 126/156 | 224/275.
+constexpr int64_t kBoxPoints = 20000, kBoxPointsDamage = 32000;
+int setup_box64(StepParams &p);
+int launch_deformation_box64(const StepParams &p, cudaStream_t s);
+int launch_force_box64(const StepParams &p, cudaStream_t s);
 // TMA-staged FP64 force kernel (vpd_staged64.cu): setup fills p.staged and p.fmap_tmap (left
 // unused when the box does not fit or the driver lacks tensor maps)
 int setup_staged_force64(StepParams &p, int rx, int ry, int rz);
