@@ -421,7 +421,7 @@ int create_impl(vpd_handle *h, const vpd_case *c, const double *positions, const
   {
     NeighborScratch scr;
     NeighborGrid grid;
-    if ((rc = neighbor_scratch_alloc(scr, n)) == VPD_OK) {
+    if ((rc = neighbor_scratch_alloc(scr, n, s)) == VPD_OK) {
       trace.mark("neighbour scratch");
       if ((rc = neighbor_count(h->xv, n, c->horizon, h->row_ptr, grid, scr, s)) == VPD_OK) {
         VPD_CUDA(cudaMemcpyAsync(&h->nbonds, h->row_ptr + n, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
@@ -783,8 +783,10 @@ int vpd_create(const vpd_case *c, const double *positions, const double *volumes
 }
 
 int vpd_destroy(vpd_handle *h) {
-  if (h)
+  if (h) {
     destroy_impl(h);
+    workspace_trim();
+  }
   return VPD_OK;
 }
 

@@ -21,6 +21,40 @@ int cuda_error(cudaError_t e, const char *what);
       return ::vpd::cuda_error(e_, #call);                                                  \
   } while (0)
 
+// ---- temporary device memory (vpd_workspace.cu) ----
+// Device memory that a call needs only until the work it queues on `stream` has run: taken from a
+// memory pool of this library (one per device, stream-ordered, so safe with any streams and
+// threads) and returned to it in stream order. The pool keeps at most kWorkspaceKeep bytes of idle
+// memory at the next synchronisation; vpd_destroy gives that back too (workspace_trim).
+constexpr uint64_t kWorkspaceKeep = uint64_t(256) << 20;
+int workspace_alloc(void **p, size_t bytes, cudaStream_t stream);
+void workspace_trim();
+inline void workspace_free(void *p, cudaStream_t stream) {
+  if (p)
+    cudaFreeAsync(p, stream);
+}
+struct Workspace {
+  explicit Workspace(cudaStream_t s) : stream(s) {}
+  Workspace(const Workspace &) = delete;
+  Workspace &operator=(const Workspace &) = delete;
+  ~Workspace() {
+    for (int k = 0; k < used; ++k)
+      workspace_free(ptrs[k], stream);
+  }
+  template <typename T> int alloc(T **p, size_t count) {
+    if (used == kMax)
+      return set_error(VPD_ERR_CAPACITY, "workspace slots exhausted");
+    const int rc = workspace_alloc(&ptrs[used], (count ? count : 1) * sizeof(T), stream);
+    if (rc == VPD_OK)
+      *p = static_cast<T *>(ptrs[used++]);
+    return rc;
+  }
+  static constexpr int kMax = 32;
+  cudaStream_t stream;
+  void *ptrs[kMax];
+  int used = 0;
+};
+
 // ---- device status word bits (ORed by kernels, read by the host) ----
 enum : unsigned int {
   STATUS_SINGULAR_K = 1u,
@@ -43,6 +77,7 @@ enum : uint8_t {
 // ---- neighbour build (vpd_neighbors.cu) ----
 // Scratch for one build; every pointer is device memory.
 struct NeighborScratch {
+  cudaStream_t stream = nullptr;     // of every allocation (workspace_alloc)
   long long *cell_coords = nullptr;  // 3n
   int32_t *cell_of = nullptr;        // n
   int32_t *cell_count = nullptr;     // ncells (+1)
@@ -81,7 +116,7 @@ int neighbor_count(const double4 *xv, int64_t n, double horizon, int64_t *row_pt
                    NeighborGrid &grid, NeighborScratch &scr, cudaStream_t s);
 int neighbor_fill(const double4 *xv, int64_t n, const int64_t *row_ptr, int32_t *col,
                   const NeighborGrid &grid, const NeighborScratch &scr, cudaStream_t s);
-int neighbor_scratch_alloc(NeighborScratch &scr, int64_t n);
+int neighbor_scratch_alloc(NeighborScratch &scr, int64_t n, cudaStream_t s);
 int neighbor_scratch_alloc_cells(NeighborScratch &scr, int64_t ncells);
 void neighbor_scratch_free(NeighborScratch &scr);
 

@@ -385,15 +385,15 @@ extern "C" int vpd_mlp_forward(const uint16_t *weights, const float *biases, con
   if (!weights || !biases || !x || !out || batch < 1)
     return set_error(VPD_ERR_INVALID, "vpd_mlp_forward: invalid argument");
   cudaStream_t s = (cudaStream_t)stream;
+  Workspace ws(s);
   unsigned *derr = nullptr;
-  VPD_CUDA(cudaMalloc(&derr, sizeof(unsigned)));
+  int rc = ws.alloc(&derr, 1);
+  if (rc)
+    return rc;
   VPD_CUDA(cudaMemsetAsync(derr, 0, sizeof(unsigned), s));
   const MlpWeights w = mlp_weights(reinterpret_cast<const __nv_bfloat16 *>(weights), biases);
-  int rc = mlp_forward(w, x, batch, out, MlpActs{}, derr, s);
-  if (rc == VPD_OK)
-    rc = check_err(derr, s);
-  cudaFree(derr);
-  return rc;
+  rc = mlp_forward(w, x, batch, out, MlpActs{}, derr, s);
+  return rc == VPD_OK ? check_err(derr, s) : rc;
 }
 
 extern "C" int vpd_mlp_gradients(const uint16_t *weights, const float *biases, const float *x,
@@ -407,7 +407,10 @@ extern "C" int vpd_mlp_gradients(const uint16_t *weights, const float *biases, c
   const size_t blocks = (size_t)mlp_backward_blocks(batch);
   const size_t bytes = nb * kMlpIn * 2 + nb * kMlpHidden * (4 * 3 + 2 * 3) + nb * kMlpOut * 4 + 256 +
                        sizeof(float) * blocks * kMlpParams + sizeof(uint16_t) * kMlpWeights;
-  VPD_CUDA(cudaMalloc(&buf, bytes));
+  Workspace ws(s);
+  int rc = ws.alloc(&buf, bytes);
+  if (rc)
+    return rc;
   MlpActs a;
   unsigned char *q = buf;
   a.y0 = reinterpret_cast<__nv_bfloat16 *>(q), q += nb * kMlpIn * 2;
@@ -423,7 +426,6 @@ extern "C" int vpd_mlp_gradients(const uint16_t *weights, const float *biases, c
   MlpBackwardScratch scr;
   scr.partials = reinterpret_cast<float *>(q), q += sizeof(float) * blocks * kMlpParams;
   scr.wt = reinterpret_cast<__nv_bfloat16 *>(q);
-  int rc = VPD_OK;
   cudaError_t e = cudaMemsetAsync(derr, 0, sizeof(unsigned), s);
   if (e == cudaSuccess)
     e = cudaMemsetAsync(grad, 0, sizeof(float) * kMlpParams, s);
@@ -435,6 +437,5 @@ extern "C" int vpd_mlp_gradients(const uint16_t *weights, const float *biases, c
     rc = mlp_backward(w, a, gout, batch, grad, scr, derr, s);
   if (rc == VPD_OK)
     rc = check_err(derr, s);
-  cudaFree(buf);
   return rc;
 }

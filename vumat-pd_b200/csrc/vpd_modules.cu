@@ -309,12 +309,15 @@ int vpd_build_neighbor_list(const double *positions, int64_t n, double horizon, 
   if (!positions || !row_ptr || !total || n <= 0)
     return set_error(VPD_ERR_INVALID, "vpd_build_neighbor_list: invalid argument");
   cudaStream_t s = (cudaStream_t)stream;
+  Workspace ws(s);
   double4 *xv = nullptr;
-  VPD_CUDA(cudaMalloc(&xv, sizeof(double4) * n));
+  int rc = ws.alloc(&xv, n);
+  if (rc)
+    return rc;
   k_pack_positions<<<blocks(n), 128, 0, s>>>(positions, n, xv);
   NeighborScratch scr;
   NeighborGrid grid;
-  int rc = neighbor_scratch_alloc(scr, n);
+  rc = neighbor_scratch_alloc(scr, n, s);
   if (rc == VPD_OK)
     rc = neighbor_count(xv, n, horizon, row_ptr, grid, scr, s);
   if (rc == VPD_OK) {
@@ -327,7 +330,6 @@ int vpd_build_neighbor_list(const double *positions, int64_t n, double horizon, 
   if (rc == VPD_OK && col)
     rc = neighbor_fill(xv, n, row_ptr, col, grid, scr, s);
   neighbor_scratch_free(scr);
-  cudaFree(xv);
   return rc;
 }
 
@@ -360,15 +362,16 @@ int vpd_force_density(const double *positions, const double *volumes, int64_t n,
   unsigned *st = thread_status();
   if (!st)
     return set_error(VPD_ERR_CUDA, "status word allocation failed");
+  Workspace ws(s);
   double *M = nullptr;
-  VPD_CUDA(cudaMalloc(&M, sizeof(double) * 9 * std::max<int64_t>(n, 1)));
+  const int rc = ws.alloc(&M, 9 * std::max<int64_t>(n, 1));
+  if (rc)
+    return rc;
   VPD_CUDA(cudaMemsetAsync(st, 0, sizeof(unsigned), s));
   k_csr_force_map<<<blocks(n), 128, 0, s>>>(cauchy_stress, defgrad, kinv, n, M, st);
   k_csr_force<<<blocks(n), 128, 0, s>>>(positions, volumes, n, row_ptr, col, M, bond_damage, force);
-  cudaError_t e = cudaGetLastError();
-  const int rc = e == cudaSuccess ? check_status(st, s) : cuda_error(e, "force density");
-  cudaFree(M);
-  return rc;
+  VPD_CUDA(cudaGetLastError());
+  return check_status(st, s);
 }
 
 int vpd_corotational_update(int64_t n, const double *defgrad_old, const double *defgrad_new,

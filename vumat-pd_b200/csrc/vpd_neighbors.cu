@@ -358,26 +358,34 @@ __global__ void k_nb_fill(const double4 *xv, int64_t n, const long long *cc, Gri
 }
 
 // ------------------------------------------------------------------ host orchestration
-int neighbor_scratch_alloc(NeighborScratch &scr, int64_t n) {
-  VPD_CUDA(cudaMalloc(&scr.cell_coords, sizeof(long long) * 3 * (size_t)std::max<int64_t>(n, 1)));
-  VPD_CUDA(cudaMalloc(&scr.cell_of, sizeof(int32_t) * (size_t)std::max<int64_t>(n, 1)));
-  VPD_CUDA(cudaMalloc(&scr.sorted, sizeof(int32_t) * (size_t)std::max<int64_t>(n, 1)));
-  VPD_CUDA(cudaMalloc(&scr.len, sizeof(int32_t) * (size_t)std::max<int64_t>(n, 1)));
-  VPD_CUDA(cudaMalloc(&scr.reduce, sizeof(unsigned long long) * kReduceWords));
+template <typename T> static int scratch(NeighborScratch &scr, T **p, int64_t count) {
+  return workspace_alloc(reinterpret_cast<void **>(p), sizeof(T) * (size_t)std::max<int64_t>(count, 1), scr.stream);
+}
+
+int neighbor_scratch_alloc(NeighborScratch &scr, int64_t n, cudaStream_t s) {
+  scr.stream = s;
+  int rc;
+  if ((rc = scratch(scr, &scr.cell_coords, 3 * n)) || (rc = scratch(scr, &scr.cell_of, n)) ||
+      (rc = scratch(scr, &scr.sorted, n)) || (rc = scratch(scr, &scr.len, n)) ||
+      (rc = scratch(scr, &scr.reduce, kReduceWords)))
+    return rc;
   return VPD_OK;
 }
 
 int neighbor_scratch_alloc_cells(NeighborScratch &scr, int64_t ncells) {
   const int64_t tmp = std::max(scan_tmp_elems(ncells), scan_tmp_elems(0)) + 8;
-  VPD_CUDA(cudaMalloc(&scr.cell_count, sizeof(int32_t) * (size_t)(ncells + 1)));
-  VPD_CUDA(cudaMalloc(&scr.cell_start, sizeof(int64_t) * (size_t)(ncells + 1)));
-  VPD_CUDA(cudaMalloc(&scr.scan_tmp, sizeof(int64_t) * (size_t)tmp));
+  int rc;
+  if ((rc = scratch(scr, &scr.cell_count, ncells + 1)) || (rc = scratch(scr, &scr.cell_start, ncells + 1)) ||
+      (rc = scratch(scr, &scr.scan_tmp, tmp)))
+    return rc;
   return VPD_OK;
 }
 
 void neighbor_scratch_free(NeighborScratch &scr) {
-  cudaFree(scr.cell_coords), cudaFree(scr.cell_of), cudaFree(scr.sorted), cudaFree(scr.len);
-  cudaFree(scr.reduce), cudaFree(scr.cell_count), cudaFree(scr.cell_start), cudaFree(scr.scan_tmp);
+  void *const all[] = {scr.cell_coords, scr.cell_of,    scr.sorted,     scr.len,
+                       scr.reduce,      scr.cell_count, scr.cell_start, scr.scan_tmp};
+  for (void *p : all)
+    workspace_free(p, scr.stream);
   scr = NeighborScratch{};
 }
 
@@ -453,14 +461,14 @@ int neighbor_count(const double4 *xv, int64_t n, double horizon, int64_t *row_pt
   int64_t *tmp = scr.scan_tmp;
   int64_t *own = nullptr;
   if (scan_tmp_elems(n) > std::max(scan_tmp_elems(grid.ncells), scan_tmp_elems(0)) + 8) {
-    VPD_CUDA(cudaMalloc(&own, sizeof(int64_t) * (size_t)scan_tmp_elems(n)));
+    if ((rc = scratch(scr, &own, scan_tmp_elems(n))))
+      return rc;
     tmp = own;
   }
   rc = scan_exclusive_i32(scr.len, n, row_ptr, tmp, s);
   VPD_CUDA(cudaMemcpyAsync(red, scr.reduce, sizeof red, cudaMemcpyDeviceToHost, s));
   VPD_CUDA(cudaStreamSynchronize(s));
-  if (own)
-    cudaFree(own);
+  workspace_free(own, s);
   if (rc)
     return rc;
   grid.max_len = (int)red[8];

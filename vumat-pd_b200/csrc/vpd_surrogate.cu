@@ -189,22 +189,6 @@ __global__ void k_to_bf16(const float *p, __nv_bfloat16 *q, int64_t n) {
 
 namespace {
 
-// Device buffers of one training run, freed on every exit path.
-struct TrainBuffers {
-  std::vector<void *> ptrs;
-  ~TrainBuffers() {
-    for (void *p : ptrs)
-      cudaFree(p);
-  }
-  template <typename T> int alloc(T **p, size_t count) {
-    void *q = nullptr;
-    VPD_CUDA(cudaMalloc(&q, std::max<size_t>(count, 1) * sizeof(T)));
-    ptrs.push_back(q);
-    *p = static_cast<T *>(q);
-    return VPD_OK;
-  }
-};
-
 struct StreamGuard {
   cudaStream_t s = nullptr;
   cudaEvent_t e0 = nullptr, e1 = nullptr;
@@ -261,7 +245,7 @@ int train_surrogate(const vpd_surrogate_config &cfg, uint16_t *w_out, float *b_o
   VPD_CUDA(cudaEventCreate(&g.e0));
   VPD_CUDA(cudaEventCreate(&g.e1));
   cudaStream_t s = g.s;
-  TrainBuffers buf;
+  Workspace buf(s);  // given back before the stream goes
   float *X = nullptr, *Y = nullptr, *Xb = nullptr, *Yb = nullptr, *out = nullptr, *gout = nullptr;
   float *z1 = nullptr, *z2 = nullptr, *z3 = nullptr, *P = nullptr, *M = nullptr, *Vm = nullptr, *G = nullptr;
   float *loss = nullptr, *vout = nullptr;
@@ -664,7 +648,7 @@ extern "C" int vpd_surrogate_samples(const double *props, uint64_t seed, int64_t
     if (!std::isfinite(props[k]))
       return set_error(VPD_ERR_INVALID, "vpd_surrogate_samples: non-finite material property");
   const JcParams jc = make_jc_params(props);
-  TrainBuffers buf;
+  Workspace buf(0);
   float *X = nullptr, *Y = nullptr;
   double *R = nullptr;
   int rc;

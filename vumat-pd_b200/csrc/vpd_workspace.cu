@@ -1,0 +1,63 @@
+// The memory pool behind the temporary device memory of the module entry points, the neighbour search
+// and the training run.
+//
+// cudaMalloc and cudaFree of a few megabytes cost 0.3 to 0.5 ms each and synchronise the device:
+// 0.85 of the 0.9 ms of a gradient call at batch 8192, 4 of the 10 ms of a 250,000-point neighbour
+// search, a third of the 21 ms of a 60-step training run. A stream-ordered pool hands the same memory
+// out again in a few microseconds.
+#include "vpd_internal.h"
+
+#include <mutex>
+
+namespace vpd {
+
+namespace {
+constexpr int kMaxDevices = 64;
+std::mutex g_pool_mutex;
+cudaMemPool_t g_pools[kMaxDevices] = {nullptr};  // kept until the process ends
+
+int device_pool(cudaMemPool_t *out) {
+  int dev = 0;
+  VPD_CUDA(cudaGetDevice(&dev));
+  if (dev < 0 || dev >= kMaxDevices)
+    return set_error(VPD_ERR_UNSUPPORTED, "device ordinal beyond 64");
+  std::lock_guard<std::mutex> lock(g_pool_mutex);
+  if (!g_pools[dev]) {
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    cudaMemPool_t pool = nullptr;
+    VPD_CUDA(cudaMemPoolCreate(&pool, &props));
+    uint64_t keep = kWorkspaceKeep;
+    const cudaError_t e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    if (e != cudaSuccess) {
+      cudaMemPoolDestroy(pool);
+      return cuda_error(e, "cudaMemPoolSetAttribute");
+    }
+    g_pools[dev] = pool;
+  }
+  *out = g_pools[dev];
+  return VPD_OK;
+}
+}  // namespace
+
+int workspace_alloc(void **p, size_t bytes, cudaStream_t stream) {
+  cudaMemPool_t pool = nullptr;
+  const int rc = device_pool(&pool);
+  if (rc)
+    return rc;
+  VPD_CUDA(cudaMallocFromPoolAsync(p, bytes, pool, stream));
+  return VPD_OK;
+}
+
+void workspace_trim() {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices)
+    return;
+  std::lock_guard<std::mutex> lock(g_pool_mutex);
+  if (g_pools[dev])
+    cudaMemPoolTrimTo(g_pools[dev], 0);
+}
+
+}  // namespace vpd
