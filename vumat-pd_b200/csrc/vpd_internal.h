@@ -74,6 +74,12 @@ enum : uint8_t {
   FLAG_LATERAL_POS = 32,
 };
 
+// ---- CSR force density (vpd_modules.cu): the force map into M (9 n doubles, 16-byte aligned),
+// then the bond sum ----
+int launch_csr_force(const double *positions, const double *volumes, int64_t n, const int64_t *row_ptr,
+                     const int32_t *col, const double *kinv, const double *defgrad, const double *cauchy_stress,
+                     const double *bond_damage, double *force, double *M, unsigned *status, cudaStream_t s);
+
 // ---- neighbour build (vpd_neighbors.cu) ----
 // Scratch for one build; every pointer is device memory.
 struct NeighborScratch {

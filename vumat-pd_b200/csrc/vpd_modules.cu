@@ -1,7 +1,7 @@
 // Module-level entry points of libvpd_gpu.so: the reference's C++ module functions on
 // caller-owned device arrays in the reference's point-major layout (Tensor3 row-major,
 // neighbour lists as CSR), and the VUMAT plugin entry vumat_adapter_call evaluated on the GPU.
-// Each kernel is one thread per point.
+// The bond sums run eight threads per point, the pointwise kernels one.
 #include "vpd_math.cuh"
 #include "vpd_step.cuh"
 
@@ -18,24 +18,120 @@ __global__ void k_pack_positions(const double *pos, int64_t n, double4 *xv) {
     xv[i] = make_double4(pos[3 * i], pos[3 * i + 1], pos[3 * i + 2], 0.0);
 }
 
-// PdCorrespondenceSkeleton::initialize (:149-170)
-__global__ void k_csr_shape_inverse(const double *pos, const double *vol, int64_t n,
-                                    const int64_t *row_ptr, const int32_t *col, double *kinv,
-                                    unsigned *status) {
+// ------------------------------------------------------------------ CSR bond sums
+// Eight lanes per point (kRowLanes), each taking every eighth bond of the point's row; a fixed shuffle
+// tree joins the eight partial sums. The lanes of a row read its neighbour indices (and bond damage) as
+// consecutive words, and its sorted neighbours, mostly runs of consecutive points, from a few cache
+// lines; the next bond's index is read before the current bond's gathers are used. With one thread per
+// point every lane of a warp read another row's index, 32 lines per load that L1 could not hold until
+// their next use, and a few thousand points were too few warps.
+// What bounds them now is L1 (93 % of its wavefronts): the gathers of 32 bonds touch about eight lines a
+// load in any arrangement tried (records of 32 bytes, one array per component, lane = point with the
+// indices transposed through shared memory, which jitter misaligns: 1.1 to 1.8 times slower).
+// Kernel times on a B200, one thread per point | now: 154,000 jittered points, horizon 4.015 h (33M bonds): deformation
+// 254 | 200 us, damage 466 | 230, force 732 | 385; 4,000 points at 3.015 h: 28 | 7, 78 | 9, 60 | 11 us.
+constexpr int kRowLanes = 8;
+constexpr int kRowThreads = 256;
+
+static unsigned row_blocks(int64_t n) { return (unsigned)((n * kRowLanes + kRowThreads - 1) / kRowThreads); }
+
+// The eight lanes' sum, in every lane.
+__device__ __forceinline__ double row_sum(double v) {
+#pragma unroll
+  for (int o = kRowLanes / 2; o > 0; o >>= 1)
+    v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// The calling lane's row; a lane past the end takes an empty one, so that whole warps take part in the shuffles.
+struct RowPoint {
+  int64_t i, begin, end;
+  int lane;
+  bool valid;
+};
+__device__ __forceinline__ RowPoint row_point(int64_t n, const int64_t *row_ptr) {
+  const int64_t k = ((int64_t)blockIdx.x * kRowThreads + threadIdx.x) / kRowLanes;
+  RowPoint r;
+  r.valid = k < n;
+  r.i = r.valid ? k : 0;
+  r.begin = r.valid ? row_ptr[k] : 0, r.end = r.valid ? row_ptr[k + 1] : 0;
+  r.lane = threadIdx.x & (kRowLanes - 1);
+  return r;
+}
+
+// Calls bond(q, j) for the calling lane's bonds q of its row and their neighbours j.
+template <typename F> __device__ __forceinline__ void for_row(const RowPoint &r, const int32_t *col, F &&bond) {
+  int64_t q = r.begin + r.lane;
+  int32_t j = q < r.end ? __ldg(col + q) : 0;
+#pragma unroll 2
+  for (; q < r.end; q += kRowLanes) {
+    const int32_t next = q + kRowLanes < r.end ? __ldg(col + q + kRowLanes) : 0;
+    bond(q, (int64_t)j);
+    j = next;
+  }
+}
+
+// Where the bond sums read the points: the caller's arrays, or 32-byte records packed in temporary memory
+// first, one load per vector.
+struct PointsPlain {
+  const double *pos, *vol;
+  __device__ __forceinline__ double4 xv(int64_t j) const {
+    return make_double4(__ldg(pos + 3 * j), __ldg(pos + 3 * j + 1), __ldg(pos + 3 * j + 2), __ldg(vol + j));
+  }
+};
+// The displacement u (deformation) or the current position x + u (damage) of a point.
+template <bool CURRENT> struct VectorsPlain {
+  const double *pos, *disp;
+  __device__ __forceinline__ double4 at(int64_t j) const {
+    double v[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+      v[c] = CURRENT ? __dadd_rn(__ldg(pos + 3 * j + c), __ldg(disp + 3 * j + c)) : __ldg(disp + 3 * j + c);
+    return make_double4(v[0], v[1], v[2], 0.0);
+  }
+};
+struct Packed {
+  const double4 *rec;
+  __device__ __forceinline__ double4 xv(int64_t j) const { return ldg256(rec + j); }
+  __device__ __forceinline__ double4 at(int64_t j) const { return ldg256(rec + j); }
+};
+
+template <bool CURRENT>
+__global__ void k_pack_points(const double *pos, const double *vol, const double *disp, int64_t n, double4 *xv,
+                              double4 *vec) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n)
     return;
-  double K[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-  for (int64_t q = row_ptr[i]; q < row_ptr[i + 1]; ++q) {
-    const int64_t j = col[q];
-    const double e[3] = {pos[3 * j] - pos[3 * i], pos[3 * j + 1] - pos[3 * i + 1],
-                         pos[3 * j + 2] - pos[3 * i + 2]};
-#pragma unroll
-    for (int a = 0; a < 3; ++a)
-#pragma unroll
-      for (int b = 0; b < 3; ++b)
-        K[3 * a + b] += vol[j] * e[a] * e[b];
-  }
+  st256(xv + i, PointsPlain{pos, vol}.xv(i));
+  if (vec)
+    st256(vec + i, VectorsPlain<CURRENT>{pos, disp}.at(i));
+}
+
+// From these many points on the records pay for their pass. Calls at horizon 4.015 h, plain | packed:
+// damage 16,000 points 34 | 30 us, 36,000 73 | 64, 154,000 295 | 238; deformation 36,000 51 | 53, 154,000
+// 203 | 203, 250,000 345 | 324; shape tensors 154,000 165 | 158, 250,000 251 | 226. (Not in the force
+// sum: its nine words of M a bond outweigh the four of the point, 644 | 659 us at 250,000.)
+constexpr int64_t kPackDamage = 16000, kPackSums = 150000;
+
+// PdCorrespondenceSkeleton::initialize (:149-170)
+template <typename Points>
+__global__ void __launch_bounds__(kRowThreads) k_csr_shape_inverse(Points points, int64_t n, const int64_t *row_ptr,
+                                                                   const int32_t *col, double *kinv,
+                                                                   unsigned *status) {
+  const RowPoint r = row_point(n, row_ptr);
+  const double4 x = points.xv(r.i);
+  double k00 = 0, k01 = 0, k02 = 0, k11 = 0, k12 = 0, k22 = 0;
+  for_row(r, col, [&](int64_t, int64_t j) {
+    const double4 p = points.xv(j);
+    const double e0 = p.x - x.x, e1 = p.y - x.y, e2 = p.z - x.z, v = p.w, w0 = v * e0, w1 = v * e1;
+    k00 += w0 * e0, k01 += w0 * e1, k02 += w0 * e2;
+    k11 += w1 * e1, k12 += w1 * e2, k22 += v * e2 * e2;
+  });
+  k00 = row_sum(k00), k01 = row_sum(k01), k02 = row_sum(k02);
+  k11 = row_sum(k11), k12 = row_sum(k12), k22 = row_sum(k22);
+  if (!r.valid || r.lane != 0)
+    return;
+  const double K[9] = {k00, k01, k02, k01, k11, k12, k02, k12, k22};
   double Ki[9];
   if (!m_inv(K, Ki)) {
     atomicOr(status, STATUS_SINGULAR_K);
@@ -43,37 +139,44 @@ __global__ void k_csr_shape_inverse(const double *pos, const double *vol, int64_
       Ki[c] = 0.0;
   }
   for (int c = 0; c < 9; ++c)
-    kinv[9 * i + c] = Ki[c];
+    kinv[9 * r.i + c] = Ki[c];
 }
 
 // computeDeformationGradients (:172-197), in displacement-gradient form
 // F = I + [sum_j V_j (u_j - u_i) (x) xi] K^-1.
-__global__ void k_csr_deformation(const double *pos, const double *disp, const double *vol,
-                                  int64_t n, const int64_t *row_ptr, const int32_t *col,
-                                  const double *kinv, double *F) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n)
-    return;
+template <typename Points, typename Vectors>
+__global__ void __launch_bounds__(kRowThreads) k_csr_deformation(Points points, Vectors disp, int64_t n,
+                                                                 const int64_t *row_ptr, const int32_t *col,
+                                                                 const double *kinv, double *F) {
+  const RowPoint r = row_point(n, row_ptr);
+  const double4 x = points.xv(r.i), u = disp.at(r.i);
   double G[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-  for (int64_t q = row_ptr[i]; q < row_ptr[i + 1]; ++q) {
-    const int64_t j = col[q];
-    double e[3], d[3];
-    for (int c = 0; c < 3; ++c) {
-      e[c] = pos[3 * j + c] - pos[3 * i + c];
-      d[c] = vol[j] * (disp[3 * j + c] - disp[3 * i + c]);
-    }
+  for_row(r, col, [&](int64_t, int64_t j) {
+    const double4 p = points.xv(j), uj = disp.at(j);
+    const double e[3] = {p.x - x.x, p.y - x.y, p.z - x.z};
+    const double d[3] = {p.w * (uj.x - u.x), p.w * (uj.y - u.y), p.w * (uj.z - u.z)};
+#pragma unroll
     for (int a = 0; a < 3; ++a)
+#pragma unroll
       for (int b = 0; b < 3; ++b)
         G[3 * a + b] += d[a] * e[b];
-  }
-  double K[9], GK[9];
+  });
+#pragma unroll
   for (int c = 0; c < 9; ++c)
-    K[c] = kinv[9 * i + c];
-  m_mul(G, K, GK);
-  for (int c = 0; c < 9; ++c)
-    F[9 * i + c] = ((c % 4 == 0) ? 1.0 : 0.0) + GK[c];
+    G[c] = row_sum(G[c]);
+  const int a = r.lane;  // lanes 0..2 write rows 0..2 of F
+  if (!r.valid || a >= 3)
+    return;
+  const double g0 = a == 0 ? G[0] : (a == 1 ? G[3] : G[6]), g1 = a == 0 ? G[1] : (a == 1 ? G[4] : G[7]),
+               g2 = a == 0 ? G[2] : (a == 1 ? G[5] : G[8]);
+  const double *K = kinv + 9 * r.i;
+#pragma unroll
+  for (int b = 0; b < 3; ++b)
+    F[9 * r.i + 3 * a + b] = (a == b ? 1.0 : 0.0) + (g0 * K[b] + g1 * K[3 + b] + g2 * K[6 + b]);
 }
 
+// The force map M = J sigma F^-T K^-1 of every point as the bond sum gathers it: entries 0..7 as four
+// arrays of pairs, then entry 8 (9 n doubles in all).
 __global__ void k_csr_force_map(const double *sigma, const double *F, const double *kinv,
                                 int64_t n, double *M, unsigned *status) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -87,33 +190,40 @@ __global__ void k_csr_force_map(const double *sigma, const double *F, const doub
     for (int c = 0; c < 9; ++c)
       m[c] = 0.0;
   }
-  for (int c = 0; c < 9; ++c)
-    M[9 * i + c] = m[c];
+  double2 *pairs = reinterpret_cast<double2 *>(M);
+#pragma unroll
+  for (int c = 0; c < 4; ++c)
+    pairs[c * n + i] = make_double2(m[2 * c], m[2 * c + 1]);
+  M[8 * n + i] = m[8];
 }
 
 // computeForceDensity (:199-230): f_i = sum (1 - clamp(d)) (M_i + M_j) xi V_j
-__global__ void k_csr_force(const double *pos, const double *vol, int64_t n,
-                            const int64_t *row_ptr, const int32_t *col, const double *M,
-                            const double *bond_damage, double *force) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n)
-    return;
-  double f[3] = {0, 0, 0};
-  const double *Mi = M + 9 * i;
-  for (int64_t q = row_ptr[i]; q < row_ptr[i + 1]; ++q) {
-    const int64_t j = col[q];
-    const double *Mj = M + 9 * j;
-    const double e[3] = {pos[3 * j] - pos[3 * i], pos[3 * j + 1] - pos[3 * i + 1],
-                         pos[3 * j + 2] - pos[3 * i + 2]};
-    double dmg = bond_damage ? bond_damage[q] : 0.0;
+__global__ void __launch_bounds__(kRowThreads) k_csr_force(PointsPlain points, int64_t n, const int64_t *row_ptr,
+                                                           const int32_t *col, const double *M,
+                                                           const double *bond_damage, double *force) {
+  const RowPoint r = row_point(n, row_ptr);
+  const double2 *pairs = reinterpret_cast<const double2 *>(M);
+  const double4 x = points.xv(r.i);
+  const double2 ai = __ldg(pairs + r.i), bi = __ldg(pairs + n + r.i), ci = __ldg(pairs + 2 * n + r.i),
+                di = __ldg(pairs + 3 * n + r.i);
+  const double m8i = __ldg(M + 8 * n + r.i);
+  double f0 = 0, f1 = 0, f2 = 0;
+  for_row(r, col, [&](int64_t q, int64_t j) {
+    const double4 p = points.xv(j);
+    const double e0 = p.x - x.x, e1 = p.y - x.y, e2 = p.z - x.z;
+    double dmg = bond_damage ? __ldg(bond_damage + q) : 0.0;
     dmg = dmg < 0.0 ? 0.0 : (dmg > 1.0 ? 1.0 : dmg);
-    const double w = (1.0 - dmg) * vol[j];
-    for (int a = 0; a < 3; ++a)
-      f[a] += w * ((Mi[3 * a] + Mj[3 * a]) * e[0] + (Mi[3 * a + 1] + Mj[3 * a + 1]) * e[1] +
-                   (Mi[3 * a + 2] + Mj[3 * a + 2]) * e[2]);
-  }
-  for (int a = 0; a < 3; ++a)
-    force[3 * i + a] = f[a];
+    const double w = (1.0 - dmg) * p.w;
+    const double2 a = __ldg(pairs + j), b = __ldg(pairs + n + j), c = __ldg(pairs + 2 * n + j),
+                  d = __ldg(pairs + 3 * n + j);
+    const double m8 = __ldg(M + 8 * n + j);
+    f0 += w * ((ai.x + a.x) * e0 + (ai.y + a.y) * e1 + (bi.x + b.x) * e2);
+    f1 += w * ((bi.y + b.y) * e0 + (ci.x + c.x) * e1 + (ci.y + c.y) * e2);
+    f2 += w * ((di.x + d.x) * e0 + (di.y + d.y) * e1 + (m8i + m8) * e2);
+  });
+  f0 = row_sum(f0), f1 = row_sum(f1), f2 = row_sum(f2);
+  if (r.valid && r.lane == 0)
+    force[3 * r.i] = f0, force[3 * r.i + 1] = f1, force[3 * r.i + 2] = f2;
 }
 
 __global__ void k_corotational(int64_t n, const double *fN, const double *fNP1, const double *vN,
@@ -212,37 +322,58 @@ __global__ void k_jc_return_map(int64_t n, JcParams jc, double dt, const double 
 }
 
 // PdSimpleDamage::update critical_stretch (:51-82) with the reference's rounding, and the
-// damage index (:23-36).
-__global__ void k_csr_damage(const double *pos, const double *disp, const double *vol, int64_t n,
-                             const int64_t *row_ptr, const int32_t *col, double initiation,
-                             double failure, int use_compression, double *bond_damage,
-                             double *damage_index) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n)
-    return;
-  double yi[3];
-  for (int c = 0; c < 3; ++c)
-    yi[c] = __dadd_rn(pos[3 * i + c], disp[3 * i + c]);
-  double damaged = 0.0, total = 0.0;
-  for (int64_t q = row_ptr[i]; q < row_ptr[i + 1]; ++q) {
-    const int64_t j = col[q];
-    double e[3], y[3];
-    for (int c = 0; c < 3; ++c) {
-      e[c] = __dsub_rn(pos[3 * j + c], pos[3 * i + c]);
-      y[c] = __dsub_rn(__dadd_rn(pos[3 * j + c], disp[3 * j + c]), yi[c]);
+// damage index (:23-36). A bond whose squared lengths lie clear of both thresholds (by 1e-9 of them,
+// against roundings of 1e-15) is decided from those; the others, and lengths whose squares may not be
+// normal numbers, take the reference's square roots and division.
+struct StretchTest {
+  double initiation, failure, tension2, compression2;  // thresholds on the stretch and on (1 + it)^2
+  int use_compression;
+};
+__device__ __forceinline__ bool stretch_breaks(const StretchTest &t, const double (&e)[3], const double (&y)[3]) {
+  const double xx =
+      __dadd_rn(__dadd_rn(__dmul_rn(e[0], e[0]), __dmul_rn(e[1], e[1])), __dmul_rn(e[2], e[2]));
+  const double yy =
+      __dadd_rn(__dadd_rn(__dmul_rn(y[0], y[0]), __dmul_rn(y[1], y[1])), __dmul_rn(y[2], y[2]));
+  if (xx > 1.0e-200 && xx < 1.0e200 && yy > 1.0e-200 && yy < 1.0e200) {
+    const double tt = t.tension2 * xx;
+    if (yy > tt * (1.0 + 1.0e-9))
+      return true;
+    if (yy < tt * (1.0 - 1.0e-9)) {
+      if (!t.use_compression)
+        return false;
+      const double c = t.compression2 * xx;
+      if (yy < c * (1.0 - 1.0e-9))
+        return true;
+      if (yy > c * (1.0 + 1.0e-9))
+        return false;
     }
-    const double initial =
-        __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(e[0], e[0]), __dmul_rn(e[1], e[1])), __dmul_rn(e[2], e[2])));
-    const double cur =
-        __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(y[0], y[0]), __dmul_rn(y[1], y[1])), __dmul_rn(y[2], y[2])));
-    const double stretch = __ddiv_rn(__dsub_rn(cur, initial), initial);
-    if (stretch > initiation || (use_compression && stretch < -failure))
-      bond_damage[q] = 1.0;
-    damaged += bond_damage[q] * vol[j];
-    total += vol[j];
   }
-  if (damage_index)
-    damage_index[i] = total > 0.0 ? damaged / total : 0.0;
+  const double initial = __dsqrt_rn(xx);
+  const double stretch = __ddiv_rn(__dsub_rn(__dsqrt_rn(yy), initial), initial);
+  return stretch > t.initiation || (t.use_compression && stretch < -t.failure);
+}
+
+template <typename Points, typename Vectors>
+__global__ void __launch_bounds__(kRowThreads) k_csr_damage(Points points, Vectors current, int64_t n,
+                                                            const int64_t *row_ptr, const int32_t *col,
+                                                            StretchTest test, double *bond_damage,
+                                                            double *damage_index) {
+  const RowPoint r = row_point(n, row_ptr);
+  const double4 x = points.xv(r.i), yi = current.at(r.i);
+  double damaged = 0.0, total = 0.0;
+  for_row(r, col, [&](int64_t q, int64_t j) {
+    const double4 p = points.xv(j), yj = current.at(j);
+    const double e[3] = {__dsub_rn(p.x, x.x), __dsub_rn(p.y, x.y), __dsub_rn(p.z, x.z)};
+    const double y[3] = {__dsub_rn(yj.x, yi.x), __dsub_rn(yj.y, yi.y), __dsub_rn(yj.z, yi.z)};
+    double d = bond_damage[q];
+    if (stretch_breaks(test, e, y) && d != 1.0)
+      bond_damage[q] = d = 1.0;
+    damaged += d * p.w;
+    total += p.w;
+  });
+  damaged = row_sum(damaged), total = row_sum(total);
+  if (damage_index && r.valid && r.lane == 0)
+    damage_index[r.i] = total > 0.0 ? damaged / total : 0.0;
 }
 
 // Johnson-Cook on one column-major block (the plugin ABI).
@@ -298,6 +429,16 @@ static unsigned *thread_status() {
 
 static unsigned blocks(int64_t n) { return (unsigned)std::max<int64_t>(1, (n + 127) / 128); }
 
+int launch_csr_force(const double *positions, const double *volumes, int64_t n, const int64_t *row_ptr,
+                     const int32_t *col, const double *kinv, const double *defgrad, const double *cauchy_stress,
+                     const double *bond_damage, double *force, double *M, unsigned *status, cudaStream_t s) {
+  k_csr_force_map<<<blocks(n), 128, 0, s>>>(cauchy_stress, defgrad, kinv, n, M, status);
+  k_csr_force<<<row_blocks(n), kRowThreads, 0, s>>>(PointsPlain{positions, volumes}, n, row_ptr, col, M, bond_damage,
+                                                    force);
+  VPD_CUDA(cudaGetLastError());
+  return VPD_OK;
+}
+
 }  // namespace vpd
 
 using namespace vpd;
@@ -339,8 +480,21 @@ int vpd_shape_tensor_inverse(const double *positions, const double *volumes, int
   unsigned *st = thread_status();
   if (!st)
     return set_error(VPD_ERR_CUDA, "status word allocation failed");
+  if (n <= 0)
+    return VPD_OK;
   VPD_CUDA(cudaMemsetAsync(st, 0, sizeof(unsigned), s));
-  k_csr_shape_inverse<<<blocks(n), 128, 0, s>>>(positions, volumes, n, row_ptr, col, kinv, st);
+  Workspace ws(s);
+  if (n >= kPackSums) {
+    double4 *rec = nullptr;
+    const int rc = ws.alloc(&rec, n);
+    if (rc)
+      return rc;
+    k_pack_points<false><<<blocks(n), 128, 0, s>>>(positions, volumes, nullptr, n, rec, nullptr);
+    k_csr_shape_inverse<<<row_blocks(n), kRowThreads, 0, s>>>(Packed{rec}, n, row_ptr, col, kinv, st);
+  } else {
+    k_csr_shape_inverse<<<row_blocks(n), kRowThreads, 0, s>>>(PointsPlain{positions, volumes}, n, row_ptr, col, kinv,
+                                                              st);
+  }
   VPD_CUDA(cudaGetLastError());
   return check_status(st, s);
 }
@@ -348,8 +502,23 @@ int vpd_shape_tensor_inverse(const double *positions, const double *volumes, int
 int vpd_deformation_gradients(const double *positions, const double *displacement, const double *volumes,
                               int64_t n, const int64_t *row_ptr, const int32_t *col, const double *kinv,
                               double *defgrad, void *stream) {
-  k_csr_deformation<<<blocks(n), 128, 0, (cudaStream_t)stream>>>(positions, displacement, volumes, n,
-                                                                  row_ptr, col, kinv, defgrad);
+  if (n <= 0)
+    return VPD_OK;
+  cudaStream_t s = (cudaStream_t)stream;
+  Workspace ws(s);
+  if (n >= kPackSums) {
+    double4 *rec = nullptr;
+    const int rc = ws.alloc(&rec, 2 * n);
+    if (rc)
+      return rc;
+    k_pack_points<false><<<blocks(n), 128, 0, s>>>(positions, volumes, displacement, n, rec, rec + n);
+    k_csr_deformation<<<row_blocks(n), kRowThreads, 0, s>>>(Packed{rec}, Packed{rec + n}, n, row_ptr, col, kinv,
+                                                            defgrad);
+  } else {
+    k_csr_deformation<<<row_blocks(n), kRowThreads, 0, s>>>(PointsPlain{positions, volumes},
+                                                            VectorsPlain<false>{positions, displacement}, n, row_ptr,
+                                                            col, kinv, defgrad);
+  }
   VPD_CUDA(cudaGetLastError());
   return VPD_OK;
 }
@@ -362,15 +531,17 @@ int vpd_force_density(const double *positions, const double *volumes, int64_t n,
   unsigned *st = thread_status();
   if (!st)
     return set_error(VPD_ERR_CUDA, "status word allocation failed");
+  if (n <= 0)
+    return VPD_OK;
   Workspace ws(s);
   double *M = nullptr;
-  const int rc = ws.alloc(&M, 9 * std::max<int64_t>(n, 1));
+  int rc = ws.alloc(&M, 9 * n);
   if (rc)
     return rc;
   VPD_CUDA(cudaMemsetAsync(st, 0, sizeof(unsigned), s));
-  k_csr_force_map<<<blocks(n), 128, 0, s>>>(cauchy_stress, defgrad, kinv, n, M, st);
-  k_csr_force<<<blocks(n), 128, 0, s>>>(positions, volumes, n, row_ptr, col, M, bond_damage, force);
-  VPD_CUDA(cudaGetLastError());
+  if ((rc = launch_csr_force(positions, volumes, n, row_ptr, col, kinv, defgrad, cauchy_stress, bond_damage, force, M,
+                             st, s)))
+    return rc;
   return check_status(st, s);
 }
 
@@ -435,10 +606,26 @@ int vpd_damage_update(const double *positions, const double *displacement, const
                       double *bond_damage, double *damage_index, void *stream) {
   if (!(initiation > 0.0))
     return set_error(VPD_ERR_INVALID, "critical_stretch requires initiation > 0.");
+  if (n <= 0)
+    return VPD_OK;
   const int use_compression = failure > 0.0 && std::isfinite(failure);
-  k_csr_damage<<<blocks(n), 128, 0, (cudaStream_t)stream>>>(positions, displacement, volumes, n, row_ptr, col,
-                                                            initiation, failure, use_compression, bond_damage,
-                                                            damage_index);
+  const StretchTest test{initiation, failure, (1.0 + initiation) * (1.0 + initiation),
+                         failure < 1.0 ? (1.0 - failure) * (1.0 - failure) : 0.0, use_compression};
+  cudaStream_t s = (cudaStream_t)stream;
+  Workspace ws(s);
+  if (n >= kPackDamage) {
+    double4 *rec = nullptr;
+    const int rc = ws.alloc(&rec, 2 * n);
+    if (rc)
+      return rc;
+    k_pack_points<true><<<blocks(n), 128, 0, s>>>(positions, volumes, displacement, n, rec, rec + n);
+    k_csr_damage<<<row_blocks(n), kRowThreads, 0, s>>>(Packed{rec}, Packed{rec + n}, n, row_ptr, col, test,
+                                                       bond_damage, damage_index);
+  } else {
+    k_csr_damage<<<row_blocks(n), kRowThreads, 0, s>>>(PointsPlain{positions, volumes},
+                                                       VectorsPlain<true>{positions, displacement}, n, row_ptr, col,
+                                                       test, bond_damage, damage_index);
+  }
   VPD_CUDA(cudaGetLastError());
   return VPD_OK;
 }

@@ -28,15 +28,6 @@
 
 #include <mutex>
 
-namespace vpd {
-// The module kernels of vpd_modules.cu: the force map M = J sigma F^-T K^-1 and the bond sum.
-__global__ void k_csr_force_map(const double *sigma, const double *F, const double *kinv,
-                                int64_t n, double *M, unsigned *status);
-__global__ void k_csr_force(const double *pos, const double *vol, int64_t n,
-                            const int64_t *row_ptr, const int32_t *col, const double *M,
-                            const double *bond_damage, double *force);
-}  // namespace vpd
-
 namespace {
 
 constexpr int64_t kNoAllocMaxPoints = 65536;
@@ -92,10 +83,9 @@ extern "C" int vpd_force_density_noalloc(const double *positions, const double *
   unsigned *status = reinterpret_cast<unsigned *>(scratch + kStatusOffset);
   cudaStream_t s = (cudaStream_t)stream;
   VPD_CUDA(cudaMemsetAsync(status, 0, sizeof(unsigned), s));
-  const unsigned blocks = (unsigned)((n + 127) / 128);
-  k_csr_force_map<<<blocks, 128, 0, s>>>(cauchy_stress, defgrad, kinv, n, M, status);
-  k_csr_force<<<blocks, 128, 0, s>>>(positions, volumes, n, row_ptr, col, M, bond_damage, force);
-  VPD_CUDA(cudaGetLastError());
+  if ((rc = launch_csr_force(positions, volumes, n, row_ptr, col, kinv, defgrad, cauchy_stress, bond_damage, force, M,
+                             status, s)))
+    return rc;
   unsigned st = 0;
   VPD_CUDA(cudaMemcpyAsync(&st, status, sizeof st, cudaMemcpyDeviceToHost, s));
   VPD_CUDA(cudaStreamSynchronize(s));
