@@ -1,97 +1,178 @@
-// The surrogate network's forward and backward passes on the tensor cores.
+// The surrogate network's forward pass and gradients on the tensor cores.
 //
 // Network: 10 -> 128 -> 128 -> 128 -> 7 with SiLU activations, BF16 weights and activations,
 // FP32 accumulation. Inputs and outputs are padded to 16 columns (zero weights outside).
-// Each CTA takes a tile of 128 batch rows with 128 threads, thread t owning row t: its row of
-// every accumulator sits in TMEM lane t, so the epilogue (bias, SiLU, BF16 conversion, writing
-// the next layer's operand into shared memory) is row-local. The MMAs are tcgen05.mma
-// kind::f16 (BF16 x BF16 -> FP32 in TMEM), issued by one thread, completion signalled through
-// an mbarrier (tcgen05.commit); every wait is bounded and reports a timeout in *err.
-//
-// Backward (same tiling): dZ = dY * SiLU'(Z); dW = dZ^T Y_prev is a 128 x 128 (or 128 x 16)
-// product over the tile's rows, accumulated into FP32 gradient buffers with atomics; dY_prev =
-// dZ W. Operands that the products need transposed are staged transposed into shared memory.
+// A tile is 128 batch rows; its rows are TMEM lanes. The MMAs are tcgen05.mma kind::f16 (BF16 x BF16 ->
+// FP32 in TMEM), issued by one thread, completion signalled through an mbarrier (tcgen05.commit);
+// every wait is bounded and reports a timeout in *err.
 #include "vpd_mlp_tile.cuh"
+#include "vpd_surrogate.cuh"
 
 #include <algorithm>
 #include <vector>
 
 namespace vpd {
 
-// ------------------------------------------------------------------ forward
-// smem: W1 (128x16) | W2 (128x128) | W3 | W4 (16x128) | A (128x128) | X0 (128x16) | barrier |
-//       biases
-constexpr size_t kFwdSmem = 4096 + 32768 + 32768 + 4096 + 32768 + 4096 + 64 + 4 * kBiasFloats;
-
-__device__ __forceinline__ void stage_weights_fwd(unsigned char *s, const MlpWeights &w) {
-  stage_rowmajor(s, w.w1, kMlpHidden, kMlpIn);
-  stage_rowmajor(s + 4096, w.w2, kMlpHidden, kMlpHidden);
-  stage_rowmajor(s + 4096 + 32768, w.w3, kMlpHidden, kMlpHidden);
-  stage_rowmajor(s + 4096 + 65536, w.w4, kMlpOut, kMlpHidden);
+// W1 (128x16) | W2 (128x128) | W3 | W4 (16x128), as staged by both kernels
+constexpr int kWeightBytes = 4096 + 32768 + 32768 + 4096;
+struct StagedWeights {
+  unsigned char *w1, *w2, *w3, *w4;
+};
+__device__ __forceinline__ StagedWeights stage_weights(unsigned char *s, const MlpWeights &w) {
+  const StagedWeights sw{s, s + 4096, s + 4096 + 32768, s + 4096 + 65536};
+  stage_rowmajor(sw.w1, w.w1, kMlpHidden, kMlpIn);
+  stage_rowmajor(sw.w2, w.w2, kMlpHidden, kMlpHidden);
+  stage_rowmajor(sw.w3, w.w3, kMlpHidden, kMlpHidden);
+  stage_rowmajor(sw.w4, w.w4, kMlpOut, kMlpHidden);
+  return sw;
 }
 
-__global__ void __launch_bounds__(128, 1) k_mlp_forward(MlpWeights w, const float *x, int64_t B, float *out,
-                                                        MlpActs acts, unsigned *err) {
+// ------------------------------------------------------------------ forward
+// Persistent blocks, one per SM: the weights are staged once, and four groups of 128 threads run a tile each
+// (thread t of a group = row t = TMEM lane t), with their own operand tile, 128 TMEM columns, mbarrier and
+// named barrier. A tile's four products and epilogues are a serial chain; the four groups of a block
+// overlap theirs. What bounds it is the epilogue: 384 tanh per row at 16 per SM and clock, 83 us for 1M rows,
+// against 43 us of tensor work and 20 us of memory traffic. Measured on a B200: 161 us for 1M rows (490 with a
+// block per tile that staged the 72 KB of weights each time), the tanh unit about half busy; the rest is the chain's
+// waits (barriers, TMEM loads) at 16 warps.
+constexpr int kGroups = 4;
+constexpr size_t kFwdSmem = kWeightBytes + kGroups * 32768 + kGroups * 16 + 4 * kBiasFloats;
+
+// Four consecutive floats; the callers' arrays may start at any multiple of 4 bytes (vec: at one of 16).
+__device__ __forceinline__ float4 load4(const float *p, bool vec) {
+  return vec ? __ldg(reinterpret_cast<const float4 *>(p)) : make_float4(__ldg(p), __ldg(p + 1), __ldg(p + 2), __ldg(p + 3));
+}
+__device__ __forceinline__ void store4(float *p, float4 v, bool vec) {
+  if (vec)
+    *reinterpret_cast<float4 *>(p) = v;
+  else
+    p[0] = v.x, p[1] = v.y, p[2] = v.z, p[3] = v.w;
+}
+__device__ __forceinline__ bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+
+// Barrier and vote of one group's 128 threads.
+__device__ __forceinline__ void group_sync(int g) { asm volatile("bar.sync %0, 128;" ::"r"(g + 1) : "memory"); }
+__device__ __forceinline__ bool group_all(int g, bool v) {
+  uint32_t r;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.u32 p, %1, 0;\n\t"
+      "bar.red.and.pred q, %2, 128, p;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t}\n"
+      : "=r"(r)
+      : "r"((uint32_t)v), "r"(g + 1)
+      : "memory");
+  return r != 0;
+}
+
+__global__ void __launch_bounds__(128 * kGroups, 1) k_mlp_forward(MlpWeights w, const float *x, int64_t B, float *out,
+                                                                  unsigned *err) {
   extern __shared__ __align__(1024) unsigned char smem[];
-  unsigned char *sW1 = smem, *sW2 = smem + 4096, *sW3 = sW2 + 32768, *sW4 = sW3 + 32768;
-  unsigned char *sA = sW4 + 4096, *sX = sA + 32768;
-  uint64_t *mbar = reinterpret_cast<uint64_t *>(sX + 4096);
-  float *sBias = reinterpret_cast<float *>(sX + 4096 + 64);
+  unsigned char *sAll = smem + kWeightBytes;
+  uint64_t *mbars = reinterpret_cast<uint64_t *>(sAll + kGroups * 32768);
+  float *sBias = reinterpret_cast<float *>(sAll + kGroups * 32768 + kGroups * 16);
   __shared__ uint32_t s_tmem;
-  const int t = threadIdx.x;
-  const int64_t row = (int64_t)blockIdx.x * 128 + t;
-  if (t < 32)
-    umma::tmem_alloc(&s_tmem, 128);
+  const int g = threadIdx.x >> 7, t = threadIdx.x & 127;
+  if (threadIdx.x < 32)
+    umma::tmem_alloc(&s_tmem, 128 * kGroups);
   if (t == 0)
-    umma::mbar_init(mbar, 1);
-  stage_weights_fwd(smem, w);
+    umma::mbar_init(mbars + 2 * g, 1);
+  const StagedWeights sw = stage_weights(smem, w);
   stage_biases(sBias, w);
-  float xin[kMlpIn];
-#pragma unroll
-  for (int c = 0; c < kMlpIn; ++c)
-    xin[c] = row < B ? x[row * kMlpIn + c] : 0.0f;
-#pragma unroll
-  for (int c = 0; c < kMlpIn; ++c)
-    st_bf16(sX, t, c, kMlpIn, xin[c]);
-  if (acts.y0 && row < B)
-#pragma unroll
-    for (int c = 0; c < kMlpIn; ++c)
-      acts.y0[row * kMlpIn + c] = __float2bfloat16(xin[c]);
   stage_wait();
+  umma::fence_proxy_async();
   umma::fence_before_sync();
   __syncthreads();
   umma::fence_after_sync();
-  const uint32_t tmem = s_tmem;
+  unsigned char *sA = sAll + g * 32768;  // the layer's input rows (the 16 features in its first 4 KB)
+  uint64_t *mbar = mbars + 2 * g;
+  const uint32_t tmem = s_tmem + 128u * g;
   const uint32_t trow = tmem + ((uint32_t)(t & ~31) << 16);  // this warp's TMEM lanes
-  Sync sy{mbar, 0u, err, 1u, true};
-  const bool keep = row < B;
-  gemm(sy, tmem, sX, sW1, kMlpIn, kMlpHidden);
-  hidden_epilogue(trow, sBias, sA, keep && acts.z1 ? acts.z1 + row * kMlpHidden : nullptr,
-                  keep && acts.y1 ? acts.y1 + row * kMlpHidden : nullptr);
-  gemm(sy, tmem, sA, sW2, kMlpHidden, kMlpHidden);
-  hidden_epilogue(trow, sBias + kMlpHidden, sA, keep && acts.z2 ? acts.z2 + row * kMlpHidden : nullptr,
-                  keep && acts.y2 ? acts.y2 + row * kMlpHidden : nullptr);
-  gemm(sy, tmem, sA, sW3, kMlpHidden, kMlpHidden);
-  hidden_epilogue(trow, sBias + 2 * kMlpHidden, sA, keep && acts.z3 ? acts.z3 + row * kMlpHidden : nullptr,
-                  keep && acts.y3 ? acts.y3 + row * kMlpHidden : nullptr);
-  gemm(sy, tmem, sA, sW4, kMlpHidden, kMlpOut);
-  float v[16];
-  if (sy.ok)
-    umma::tmem_ld16(trow, v);
-  if (keep)
+  uint32_t phase = 0;
+  bool ok = true;
+  // D = A B^T by the group's first thread, awaited by the group
+  auto product = [&](const unsigned char *b, int K, int N) {
+    umma::fence_proxy_async();
+    umma::fence_before_sync();
+    group_sync(g);
+    if (t == 0) {
+      umma::fence_after_sync();
+      umma::gemm_issue(tmem, umma::k_major(sA, K), umma::k_major(b, K), K, N);
+      umma::commit(mbar);
+    }
+    ok = group_all(g, umma::mbar_wait(mbar, phase, kWaitLimit));
+    phase ^= 1u;
+    umma::fence_after_sync();
+  };
+  const int64_t tiles = (B + 127) / 128;
+  const bool vecx = aligned16(x), veco = aligned16(out);
+  float4 next[4];
+  auto load = [&](int64_t tile) {
+    const int64_t row = tile * 128 + t;
 #pragma unroll
-    for (int c = 0; c < kMlpOut; ++c)
-      out[row * kMlpOut + c] = sy.ok ? v[c] + w.b4[c] : 0.0f;
+    for (int c = 0; c < 4; ++c)
+      next[c] = row < B ? load4(x + row * kMlpIn + 4 * c, vecx) : make_float4(0.f, 0.f, 0.f, 0.f);
+  };
+  // group g of block b takes tiles b + (g + kGroups k) gridDim: few tiles spread over the blocks first
+  const int64_t stride = (int64_t)kGroups * gridDim.x;
+  int64_t tile = blockIdx.x + (int64_t)g * gridDim.x;
+  if (tile < tiles)
+    load(tile);
+  for (; tile < tiles && ok; tile += stride) {
+    __align__(16) __nv_bfloat16 xb[16];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      xb[4 * c] = __float2bfloat16(next[c].x), xb[4 * c + 1] = __float2bfloat16(next[c].y);
+      xb[4 * c + 2] = __float2bfloat16(next[c].z), xb[4 * c + 3] = __float2bfloat16(next[c].w);
+    }
+    *reinterpret_cast<uint4 *>(sA + kmajor_offset(t, 0, kMlpIn)) = *reinterpret_cast<const uint4 *>(xb);
+    *reinterpret_cast<uint4 *>(sA + kmajor_offset(t, 8, kMlpIn)) = *reinterpret_cast<const uint4 *>(xb + 8);
+    if (tile + stride < tiles)
+      load(tile + stride);
+    product(sw.w1, kMlpIn, kMlpHidden);
+    if (ok)
+      hidden_epilogue(trow, sBias, sA, t), product(sw.w2, kMlpHidden, kMlpHidden);
+    if (ok)
+      hidden_epilogue(trow, sBias + kMlpHidden, sA, t), product(sw.w3, kMlpHidden, kMlpHidden);
+    if (ok)
+      hidden_epilogue(trow, sBias + 2 * kMlpHidden, sA, t), product(sw.w4, kMlpHidden, kMlpOut);
+    const int64_t row = tile * 128 + t;
+    float v[16];
+    if (ok)
+      umma::tmem_ld16(trow, v);
+    if (row < B) {
+#pragma unroll
+      for (int c = 0; c < kMlpOut; c += 4) {
+        const float4 bb = *reinterpret_cast<const float4 *>(sBias + 3 * kMlpHidden + c);
+        store4(out + row * kMlpOut + c,
+               ok ? make_float4(v[c] + bb.x, v[c + 1] + bb.y, v[c + 2] + bb.z, v[c + 3] + bb.w)
+                  : make_float4(0.f, 0.f, 0.f, 0.f),
+               veco);
+      }
+    }
+  }
+  if (!ok && t == 0)
+    atomicOr(err, 1u);
   umma::fence_before_sync();
   __syncthreads();
-  if (t < 32)
-    umma::tmem_dealloc(tmem, 128);
+  if (threadIdx.x < 32)
+    umma::tmem_dealloc(s_tmem, 128 * kGroups);
 }
 
-// ------------------------------------------------------------------ backward
-// smem: Wt2 (128x128) | Wt3 | Wt4 (128x16) | A (dZ, 128x128) | At (dZ^T, 128x128) |
-//       Bt (Y_prev^T, 128x128) | small (dZ4^T 16x128) | barrier
-constexpr size_t kBwdSmem = 32768 * 2 + 4096 + 32768 * 3 + 4096 + 64;
+// ------------------------------------------------------------------ gradients
+// Forward and backward of one 128-row tile per block, everything between in shared memory and TMEM (the two
+// passes as kernels of their own wrote and read 2.3 KB a row of pre-activations and activations, a third kernel
+// transposed the weights, and 128 threads ran every epilogue of the tile alone). 512 threads: warp w holds the TMEM
+// lanes (rows) of its quarter w % 4 and the 32 columns of its group w / 4.
+//   forward   Z1 = X W1^T, Y1 = silu(Z1 + b1) ... Y3; Z2 and Z3 stay in TMEM, Z1 (one K = 16 product) is formed again
+//   backward  dZ = dY * silu'(Z); dW = dZ^T Y_prev and dY_prev = dZ W. The products that need an operand the other
+//             way round read the forward pass's own tiles through MN-major descriptors.
+// The tile's weight and bias gradients go to the block's slice of `partials`; the slices are summed in block
+// order, so the gradient does not depend on the order the blocks run in. Batch 8192 on a B200: 27 us and 3.5 us for
+// the sum (46 + 60 + 6 us in the separate kernels); eight dependent stages at one block on 64 SMs, so latency.
+constexpr int kGradThreads = 512;
+// weights | Y0 (128x16) | Y1 | Y2 | Y3 | dZ (128x128) | dZ4 (128x16) | mbarrier | biases
+constexpr size_t kGradSmem = kWeightBytes + 4096 + 4 * 32768 + 4096 + 64 + 4 * kBiasFloats;
 
 // Column sums of a 16-column slab over the 32 lanes of a warp, by halving: each step a lane
 // keeps half of its columns and adds the partner's copy of them (16 shuffles in all). Lane l
@@ -115,251 +196,274 @@ __device__ __forceinline__ float warp_column_sums16(const float (&v)[16], int la
   return e;
 }
 
-// Thread t copies its batch row of a row-major bf16 matrix [rows][kin] into column t of a
-// K-major tile whose rows are the kin inputs (K = the 128 batch rows): 16-byte row loads,
-// and the 2-byte stores of a warp fall in four 16-byte runs.
-__device__ __forceinline__ void stage_row_as_column(unsigned char *tile, const __nv_bfloat16 *src, int64_t row,
-                                                    int64_t rows, int kin) {
-  const int t = threadIdx.x;
-  for (int c8 = 0; c8 < kin; c8 += 8) {
-    uint4 q = make_uint4(0u, 0u, 0u, 0u);
-    if (row < rows)
-      q = *reinterpret_cast<const uint4 *>(src + row * kin + c8);
-    const __nv_bfloat16 *e = reinterpret_cast<const __nv_bfloat16 *>(&q);
-#pragma unroll
-    for (int j = 0; j < 8; ++j)
-      *reinterpret_cast<__nv_bfloat16 *>(tile + kmajor_offset(c8 + j, t, 128)) = e[j];
-  }
-}
-
-// One 128-row batch tile per block. The weight gradients of the tile (tensor-core products in
-// TMEM) and its bias gradients (warp column sums) are written to the block's slice of
-// `partials` [gridDim.x][kMlpParams]; k_sum_partials adds the slices in block order, so the
-// result does not depend on the order the blocks run in. wt holds W2^T, W3^T and W4^T
-// (row-major [in][out]), made once per pass by k_transpose_weights.
-__global__ void __launch_bounds__(128, 1) k_mlp_backward(MlpWeights w, const __nv_bfloat16 *wt, MlpActs acts,
-                                                         const float *gout, int64_t B, float *partials,
-                                                         unsigned *err) {
+template <bool TRAIN>
+__global__ void __launch_bounds__(kGradThreads, 1) k_mlp_gradient(MlpWeights w, MlpBatch batch, int64_t B, float *partials,
+                                                                  unsigned *err) {
   extern __shared__ __align__(1024) unsigned char smem[];
-  unsigned char *sWt2 = smem, *sWt3 = smem + 32768, *sWt4 = smem + 65536;
-  unsigned char *sA = sWt4 + 4096, *sAt = sA + 32768, *sBt = sAt + 32768, *sSm = sBt + 32768;
-  uint64_t *mbar = reinterpret_cast<uint64_t *>(sSm + 4096);
+  unsigned char *sY0 = smem + kWeightBytes, *sY1 = sY0 + 4096, *sY2 = sY1 + 32768, *sY3 = sY2 + 32768;
+  unsigned char *sDZ = sY3 + 32768, *sDZ4 = sDZ + 32768;
+  uint64_t *mbar = reinterpret_cast<uint64_t *>(sDZ4 + 4096);
+  float *sBias = reinterpret_cast<float *>(sDZ4 + 4096 + 64);
   __shared__ uint32_t s_tmem;
   __shared__ float s_db[4][kMlpHidden];
-  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, quarter = warp & 3, group = warp >> 2;
+  const int t = quarter * 32 + lane;  // the thread's row (of the tile, and of dW)
+  const int c0 = group * 32;          // ... and its first column
   const int64_t row0 = (int64_t)blockIdx.x * 128, row = row0 + t;
   const bool keep = row < B;
-  const MlpGrads g = mlp_grads(partials + (size_t)blockIdx.x * kMlpParams);
-  if (t < 32)
-    umma::tmem_alloc(&s_tmem, 256);
-  if (t == 0)
+  const MlpGrads grad = mlp_grads(partials + (size_t)blockIdx.x * kMlpParams);
+  if (warp == 0)
+    umma::tmem_alloc(&s_tmem, 512);
+  if (threadIdx.x == 0)
     umma::mbar_init(mbar, 1);
-  // transposed weights: B operand rows = layer inputs, K = layer outputs
-  stage_rowmajor(sWt2, wt, kMlpHidden, kMlpHidden);
-  stage_rowmajor(sWt3, wt + 16384, kMlpHidden, kMlpHidden);
-  stage_rowmajor(sWt4, wt + 32768, kMlpHidden, kMlpOut);
+  const StagedWeights sw = stage_weights(smem, w);
+  stage_biases(sBias, w);
+  // the batch row's place in the arrays it is read from
+  auto source = [&](int64_t r) {
+    return TRAIN ? (int64_t)((batch.mul * (uint64_t)(batch.first + r) + batch.add) % (uint64_t)batch.rows) : r;
+  };
+  {  // inputs: four threads a row
+    const int rr = threadIdx.x >> 2, part = threadIdx.x & 3;
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (row0 + rr < B)
+      v = load4(batch.x + source(row0 + rr) * kMlpIn + 4 * part, aligned16(batch.x));
+    __align__(8) __nv_bfloat16 xb[4] = {__float2bfloat16(v.x), __float2bfloat16(v.y), __float2bfloat16(v.z),
+                                        __float2bfloat16(v.w)};
+    *reinterpret_cast<uint2 *>(sY0 + kmajor_offset(rr, 4 * part, kMlpIn)) = *reinterpret_cast<const uint2 *>(xb);
+  }
   stage_wait();
   umma::fence_before_sync();
   __syncthreads();
   umma::fence_after_sync();
-  const uint32_t tmem = s_tmem;
-  const uint32_t lane_base = (uint32_t)(t & ~31) << 16;
-  const uint32_t tdy = tmem + lane_base, tdw = tmem + 128 + lane_base;
+  const uint32_t tmem = s_tmem, lanes = (uint32_t)(quarter * 32) << 16;
+  // four accumulators of 128 columns
+  const uint32_t T0 = tmem, T1 = tmem + 128, T2 = tmem + 256, T3 = tmem + 384;
   Sync sy{mbar, 0u, err, 1u, true};
-
-  // ---- output layer: dZ4 = gout
-  float dz4[kMlpOut];
-#pragma unroll
-  for (int c = 0; c < kMlpOut; ++c)
-    dz4[c] = keep ? gout[row * kMlpOut + c] : 0.0f;
-#pragma unroll
-  for (int c = 0; c < kMlpOut; ++c) {
-    st_bf16(sA, t, c, kMlpOut, dz4[c]);          // A for dY3: rows x K=16
-    st_bf16(sSm, c, t, 128, dz4[c]);             // B for dW4^T: N=16 rows x K=128 rows
-  }
-  {
-    int col;
-    const float sum = warp_column_sums16(dz4, lane, col);
-    if (!(lane & 1))
-      s_db[warp][col] = sum;
-  }
-  stage_row_as_column(sBt, acts.y3, row, B, kMlpHidden);  // Y3^T (rows = 128 inputs, K = batch rows)
-  // dW4^T [in][out] = Y3^T dZ4 ; dY3 = dZ4 W4
-  umma::fence_proxy_async();
-  umma::fence_before_sync();
-  __syncthreads();
-  umma::fence_after_sync();
-  if (t < kMlpOut)
-    g.b4[t] = s_db[0][t] + s_db[1][t] + s_db[2][t] + s_db[3][t];
-  if (t == 0) {
-    umma::gemm_issue(tmem + 128, smem_u32(sBt), smem_u32(sSm), 128, kMlpOut, false);
-    umma::gemm_issue(tmem, smem_u32(sA), smem_u32(sWt4), kMlpOut, kMlpHidden, false);
-    umma::commit(mbar);
-  }
-  sy.wait();
-  if (sy.ok) {
-    // thread t holds dW4^T row t (input t): grad_w4[out][t]
-    float v[16];
-    umma::tmem_ld16(tdw, v);
-#pragma unroll
-    for (int c = 0; c < kMlpOut; ++c)
-      g.w4[(size_t)c * kMlpHidden + t] = v[c];
-  }
-
-  // ---- hidden layers 3, 2, 1
-  for (int layer = 3; layer >= 1 && sy.ok; --layer) {
-    const float *z = layer == 3 ? acts.z3 : (layer == 2 ? acts.z2 : acts.z1);
-    const __nv_bfloat16 *yprev = layer == 3 ? acts.y2 : (layer == 2 ? acts.y1 : acts.y0);
-    const int kin = layer == 1 ? kMlpIn : kMlpHidden;
-    float *gw = layer == 3 ? g.w3 : (layer == 2 ? g.w2 : g.w1);
-    float *gb = layer == 3 ? g.b3 : (layer == 2 ? g.b2 : g.b1);
-    // dZ = dY * SiLU'(Z): this thread's row of dY from TMEM
-    for (int c0 = 0; c0 < kMlpHidden; c0 += 16) {
-      float v[16];
-      umma::tmem_ld16(tdy + c0, v);
-      __align__(16) __nv_bfloat16 zb[16];
-#pragma unroll
-      for (int c = 0; c < 16; ++c) {
-        v[c] = keep ? v[c] * silu_grad(z[row * kMlpHidden + c0 + c]) : 0.0f;
-        zb[c] = __float2bfloat16(v[c]);
-        *reinterpret_cast<__nv_bfloat16 *>(sAt + kmajor_offset(c0 + c, t, 128)) = zb[c];  // dW's A
-      }
-      // A for dY_prev: rows x K=128 outputs, two 16-byte rows of core matrices
-      *reinterpret_cast<uint4 *>(sA + kmajor_offset(t, c0, kMlpHidden)) = *reinterpret_cast<const uint4 *>(zb);
-      *reinterpret_cast<uint4 *>(sA + kmajor_offset(t, c0 + 8, kMlpHidden)) =
-          *reinterpret_cast<const uint4 *>(zb + 8);
-      int col;
-      const float sum = warp_column_sums16(v, lane, col);
-      if (!(lane & 1))
-        s_db[warp][c0 + col] = sum;
-    }
-    stage_row_as_column(sBt, yprev, row, B, kin);  // Y_prev^T (rows = inputs, K = batch rows)
+  // The stage's products, issued by one thread once every thread's operands are in place, awaited by all.
+  auto stage = [&](auto issue) {
     umma::fence_proxy_async();
     umma::fence_before_sync();
     __syncthreads();
-    umma::fence_after_sync();
-    gb[t] = s_db[0][t] + s_db[1][t] + s_db[2][t] + s_db[3][t];
-    if (t == 0) {
-      umma::gemm_issue(tmem + 128, smem_u32(sAt), smem_u32(sBt), 128, kin, false);  // dW [out][in]
-      if (layer > 1)
-        umma::gemm_issue(tmem, smem_u32(sA), smem_u32(layer == 3 ? sWt3 : sWt2), kMlpHidden, kMlpHidden,
-                         false);  // dY_prev
+    if (threadIdx.x == 0) {
+      umma::fence_after_sync();
+      issue();
       umma::commit(mbar);
     }
     sy.wait();
-    if (sy.ok)
-      for (int c0 = 0; c0 < kin; c0 += 16) {  // this thread's row of dW [out][in]
+  };
+  auto hidden = [&](uint32_t acc, const float *bias, unsigned char *Y) {
+    float v[32];
+    umma::tmem_ld32(acc + lanes + c0, v);
+    hidden_columns(v, bias, Y, t, c0);
+  };
+  const int H = kMlpHidden;
+
+  // ---- forward
+  stage([&] { umma::gemm_issue(T0, umma::k_major(sY0, kMlpIn), umma::k_major(sw.w1, kMlpIn), kMlpIn, H); });
+  if (sy.ok)
+    hidden(T0, sBias, sY1);
+  stage([&] { umma::gemm_issue(T1, umma::k_major(sY1, H), umma::k_major(sw.w2, H), H, H); });
+  if (sy.ok)
+    hidden(T1, sBias + H, sY2);
+  stage([&] { umma::gemm_issue(T2, umma::k_major(sY2, H), umma::k_major(sw.w3, H), H, H); });
+  if (sy.ok)
+    hidden(T2, sBias + 2 * H, sY3);
+  if (TRAIN)
+    stage([&] { umma::gemm_issue(T3, umma::k_major(sY3, H), umma::k_major(sw.w4, H), H, kMlpOut); });
+
+  // ---- output layer: dZ4 = gout, a row per thread of the first group
+  if (group == 0) {
+    float dz4[kMlpOut];
+    if (TRAIN) {
+      // weighted MSE over the 7 targets (row weight in target column 15, target 0 weighted 4)
+      float o[16], l = 0.0f;
+      if (sy.ok)
+        umma::tmem_ld16(T3 + lanes, o);
+      const float *target = batch.target + (keep ? source(row) : 0) * 16;
+      const float wr = keep ? target[15] : 0.0f, norm = 1.0f / (float)(B * SURROGATE_TARGETS);
+#pragma unroll
+      for (int c = 0; c < kMlpOut; ++c) {
+        const float cw = c == 0 ? 4.0f : 1.0f;
+        const float d = keep && sy.ok && c < SURROGATE_TARGETS ? (o[c] + sBias[3 * H + c]) - target[c] : 0.0f;
+        dz4[c] = 2.0f * wr * cw * d * norm;
+        l += wr * cw * d * d * norm;
+      }
+#pragma unroll
+      for (int k = 16; k > 0; k >>= 1)
+        l += __shfl_xor_sync(0xffffffffu, l, k);
+      if (lane == 0)
+        atomicAdd(batch.loss, l);
+    } else {
+#pragma unroll
+      for (int c = 0; c < kMlpOut; ++c)
+        dz4[c] = keep ? batch.gout[row * kMlpOut + c] : 0.0f;
+    }
+    __align__(16) __nv_bfloat16 zb[16];
+#pragma unroll
+    for (int c = 0; c < kMlpOut; ++c)
+      zb[c] = __float2bfloat16(dz4[c]);
+    *reinterpret_cast<uint4 *>(sDZ4 + kmajor_offset(t, 0, kMlpOut)) = *reinterpret_cast<const uint4 *>(zb);
+    *reinterpret_cast<uint4 *>(sDZ4 + kmajor_offset(t, 8, kMlpOut)) = *reinterpret_cast<const uint4 *>(zb + 8);
+    int col;
+    const float sum = warp_column_sums16(dz4, lane, col);
+    if (!(lane & 1))
+      s_db[quarter][col] = sum;
+  }
+  // dW4^T [in][out] = Y3^T dZ4 ; dY3 = dZ4 W4
+  stage([&] {
+    umma::gemm_issue(T0, umma::mn_major(sY3, H), umma::mn_major(sDZ4, kMlpOut), 128, kMlpOut);
+    umma::gemm_issue(T3, umma::k_major(sDZ4, kMlpOut), umma::mn_major(sw.w4, H), kMlpOut, H);
+  });
+  if (threadIdx.x < kMlpOut)
+    grad.b4[threadIdx.x] =
+        s_db[0][threadIdx.x] + s_db[1][threadIdx.x] + s_db[2][threadIdx.x] + s_db[3][threadIdx.x];
+  if (group == 0 && sy.ok) {  // thread t holds dW4^T row t (input t): grad_w4[out][t]
+    float v[16];
+    umma::tmem_ld16(T0 + lanes, v);
+#pragma unroll
+    for (int c = 0; c < kMlpOut; ++c)
+      grad.w4[(size_t)c * H + t] = v[c];
+  }
+  __syncthreads();  // s_db is written again below
+
+  // ---- hidden layers 3, 2, 1
+#pragma unroll 1  // one copy of the code: every instruction is fetched once per layer otherwise
+  for (int layer = 3; layer >= 1; --layer) {
+    if (!sy.ok)
+      break;
+    const uint32_t Z = layer == 3 ? T2 : (layer == 2 ? T1 : T0);
+    const float *bias = sBias + (layer - 1) * H;
+    // dZ = dY * SiLU'(Z): the thread's columns of its row
+    {
+      float v[32], z[32];
+      umma::tmem_ld32(T3 + lanes + c0, v);
+      umma::tmem_ld32(Z + lanes + c0, z);
+      __align__(16) __nv_bfloat16 zb[32];
+#pragma unroll
+      for (int c = 0; c < 32; ++c) {
+        v[c] = keep ? v[c] * silu_grad(z[c] + bias[c0 + c]) : 0.0f;
+        zb[c] = __float2bfloat16(v[c]);
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        *reinterpret_cast<uint4 *>(sDZ + kmajor_offset(t, c0 + 8 * k, H)) = *reinterpret_cast<const uint4 *>(zb + 8 * k);
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        float slab[16];
+#pragma unroll
+        for (int c = 0; c < 16; ++c)
+          slab[c] = v[16 * h + c];
+        int col;
+        const float sum = warp_column_sums16(slab, lane, col);
+        if (!(lane & 1))
+          s_db[quarter][c0 + 16 * h + col] = sum;
+      }
+    }
+    // dW [out][in] = dZ^T Y_prev over Z's columns, dY_prev = dZ W over dY's
+    stage([&] {
+      if (layer > 1) {
+        umma::gemm_issue(Z, umma::mn_major(sDZ, H), umma::mn_major(layer == 3 ? sY2 : sY1, H), 128, H);
+        umma::gemm_issue(T3, umma::k_major(sDZ, H), umma::mn_major(layer == 3 ? sw.w3 : sw.w2, H), H, H);
+      } else {
+        umma::gemm_issue(Z, umma::mn_major(sDZ, H), umma::mn_major(sY0, kMlpIn), 128, kMlpIn);
+      }
+      if (layer == 2)  // Z1 again
+        umma::gemm_issue(T0, umma::k_major(sY0, kMlpIn), umma::k_major(sw.w1, kMlpIn), kMlpIn, H);
+    });
+    float *gb = layer == 3 ? grad.b3 : (layer == 2 ? grad.b2 : grad.b1);
+    if (threadIdx.x < H)
+      gb[threadIdx.x] =
+          s_db[0][threadIdx.x] + s_db[1][threadIdx.x] + s_db[2][threadIdx.x] + s_db[3][threadIdx.x];
+    if (sy.ok) {
+      if (layer > 1) {  // this thread's 32 columns of row t of dW [out][in]
+        float v[32];
+        umma::tmem_ld32(Z + lanes + c0, v);
+        float4 *dst = reinterpret_cast<float4 *>((layer == 3 ? grad.w3 : grad.w2) + (size_t)t * H + c0);
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+          dst[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+      } else if (group == 0) {
         float v[16];
-        umma::tmem_ld16(tdw + c0, v);
-        float4 *dst = reinterpret_cast<float4 *>(gw + (size_t)t * kin + c0);
+        umma::tmem_ld16(Z + lanes, v);
+        float4 *dst = reinterpret_cast<float4 *>(grad.w1 + (size_t)t * kMlpIn);
 #pragma unroll
         for (int q = 0; q < 4; ++q)
           dst[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
       }
+    }
+    __syncthreads();  // s_db is written again by the next layer
   }
   umma::fence_before_sync();
   __syncthreads();
-  if (t < 32)
-    umma::tmem_dealloc(tmem, 256);
+  if (warp == 0)
+    umma::tmem_dealloc(tmem, 512);
 }
 
-// W2^T, W3^T and W4^T (row-major [in][out]) for the backward pass's B operands.
-__global__ void k_transpose_weights(MlpWeights w, __nv_bfloat16 *wt) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e < 2 * 16384) {
-    const int l = e >> 14, r = (e >> 7) & 127, c = e & 127;  // wt[l][r = in][c = out]
-    wt[e] = (l ? w.w3 : w.w2)[c * 128 + r];
-  } else if (e < 2 * 16384 + 2048) {
-    const int f = e - 2 * 16384, r = f >> 4, c = f & 15;  // [in 128][out 16]
-    wt[e] = w.w4[c * 128 + r];
-  }
+// sum over blocks b (in order) of partials[b][i]
+__device__ __forceinline__ float partial_sum(const float *partials, int nblocks, int i) {
+  float s = 0.0f;
+#pragma unroll 32
+  for (int b = 0; b < nblocks; ++b)
+    s += partials[(size_t)b * kMlpParams + i];
+  return s;
 }
-
-// grad[i] = sum over blocks b (in order) of partials[b][i].
 __global__ void k_sum_partials(const float *partials, int nblocks, float *grad) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < kMlpParams)
+    grad[i] = partial_sum(partials, nblocks, i);
+}
+
+// One Adam step on the summed gradient; the weights (the first kMlpWeights parameters) also to their BF16 copy.
+__global__ void k_adam(const float *partials, int nblocks, float *p, float *m, float *v, __nv_bfloat16 *pb, float lr,
+                       float b1, float b2, float eps, float c1, float c2) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= kMlpParams)
     return;
-  float s = 0.0f;
-  for (int b = 0; b < nblocks; ++b)
-    s += partials[(size_t)b * kMlpParams + i];
-  grad[i] = s;
-}
-
-// ------------------------------------------------------------------ Adam and helpers
-__global__ void k_adam(float *p, float *m, float *v, float *grad, __nv_bfloat16 *pb, int64_t n, float lr,
-                       float b1, float b2, float eps, float c1, float c2) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n)
-    return;
-  const float g = grad[i];
+  const float g = partial_sum(partials, nblocks, i);
   const float mi = b1 * m[i] + (1.0f - b1) * g;
   const float vi = b2 * v[i] + (1.0f - b2) * g * g;
   m[i] = mi, v[i] = vi;
   const float pi = p[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
   p[i] = pi;
-  if (pb)
+  if (i < kMlpWeights)
     pb[i] = __float2bfloat16(pi);
-  grad[i] = 0.0f;
 }
 
-// MSE gradient and loss over the first `cols` outputs: gout = 2 (out - target) / (B cols).
-__global__ void k_mse_grad(const float *out, const float *target, int64_t B, int cols, float *gout,
-                           float *loss) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  float l = 0.0f;
-  if (i < B)
-    for (int c = 0; c < kMlpOut; ++c) {
-      const float d = c < cols ? out[i * kMlpOut + c] - target[i * kMlpOut + c] : 0.0f;
-      gout[i * kMlpOut + c] = 2.0f * d / (float)(B * cols);
-      l += d * d;
-    }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1)
-    l += __shfl_xor_sync(0xffffffffu, l, o);
-  if ((threadIdx.x & 31) == 0)
-    atomicAdd(loss, l / (float)(B * cols));
-}
-
-int mlp_forward(const MlpWeights &w, const float *x, int64_t B, float *out, const MlpActs &acts, unsigned *err,
-                cudaStream_t s) {
-  static bool configured = false;
-  if (!configured) {
-    VPD_CUDA(cudaFuncSetAttribute(k_mlp_forward, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFwdSmem));
-    VPD_CUDA(cudaFuncSetAttribute(k_mlp_backward, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBwdSmem));
-    configured = true;
-  }
-  k_mlp_forward<<<(unsigned)((B + 127) / 128), 128, kFwdSmem, s>>>(w, x, B, out, acts, err);
+int mlp_forward(const MlpWeights &w, const float *x, int64_t B, float *out, unsigned *err, cudaStream_t s) {
+  int dev = 0, sms = 0;
+  VPD_CUDA(cudaGetDevice(&dev));
+  VPD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  VPD_CUDA(cudaFuncSetAttribute(k_mlp_forward, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFwdSmem));
+  const int64_t grid = std::min<int64_t>((B + 127) / 128, sms);
+  k_mlp_forward<<<(unsigned)grid, 128 * kGroups, kFwdSmem, s>>>(w, x, B, out, err);
   VPD_CUDA(cudaGetLastError());
   return VPD_OK;
 }
 
-int64_t mlp_backward_blocks(int64_t B) { return (B + 127) / 128; }
+int64_t mlp_gradient_blocks(int64_t B) { return (B + 127) / 128; }
 
-int mlp_backward(const MlpWeights &w, const MlpActs &acts, const float *gout, int64_t B, float *grad,
-                 const MlpBackwardScratch &scr, unsigned *err, cudaStream_t s) {
-  const int64_t nb = mlp_backward_blocks(B);
-  k_transpose_weights<<<(2 * 16384 + 2048 + 255) / 256, 256, 0, s>>>(w, scr.wt);
-  VPD_CUDA(cudaGetLastError());
-  k_mlp_backward<<<(unsigned)nb, 128, kBwdSmem, s>>>(w, scr.wt, acts, gout, B, scr.partials, err);
-  VPD_CUDA(cudaGetLastError());
-  k_sum_partials<<<(unsigned)((kMlpParams + 255) / 256), 256, 0, s>>>(scr.partials, (int)nb, grad);
+int mlp_gradient_partials(const MlpWeights &w, const MlpBatch &batch, int64_t B, float *partials, unsigned *err,
+                          cudaStream_t s) {
+  auto *kernel = batch.gout ? k_mlp_gradient<false> : k_mlp_gradient<true>;
+  VPD_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGradSmem));
+  kernel<<<(unsigned)mlp_gradient_blocks(B), kGradThreads, kGradSmem, s>>>(w, batch, B, partials, err);
   VPD_CUDA(cudaGetLastError());
   return VPD_OK;
 }
 
-int mlp_adam(float *p, float *m, float *v, float *grad, __nv_bfloat16 *pb, int64_t n, float lr, int step,
-             cudaStream_t s) {
+constexpr unsigned kParamBlocks = (unsigned)((kMlpParams + 127) / 128);
+
+int mlp_sum_partials(const float *partials, int64_t blocks, float *grad, cudaStream_t s) {
+  k_sum_partials<<<kParamBlocks, 128, 0, s>>>(partials, (int)blocks, grad);
+  VPD_CUDA(cudaGetLastError());
+  return VPD_OK;
+}
+
+int mlp_adam(const float *partials, int64_t blocks, float *p, float *m, float *v, __nv_bfloat16 *wb, float lr,
+             int step, cudaStream_t s) {
   const float b1 = 0.9f, b2 = 0.999f;
   const float c1 = 1.0f - powf(b1, (float)step), c2 = 1.0f - powf(b2, (float)step);
-  k_adam<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(p, m, v, grad, pb, n, lr, b1, b2, 1e-8f, c1, c2);
-  VPD_CUDA(cudaGetLastError());
-  return VPD_OK;
-}
-
-int mlp_mse_grad(const float *out, const float *target, int64_t B, int cols, float *gout, float *loss,
-                 cudaStream_t s) {
-  k_mse_grad<<<(unsigned)((B + 255) / 256), 256, 0, s>>>(out, target, B, cols, gout, loss);
+  k_adam<<<kParamBlocks, 128, 0, s>>>(partials, (int)blocks, p, m, v, wb, lr, b1, b2, 1e-8f, c1, c2);
   VPD_CUDA(cudaGetLastError());
   return VPD_OK;
 }
@@ -392,7 +496,7 @@ extern "C" int vpd_mlp_forward(const uint16_t *weights, const float *biases, con
     return rc;
   VPD_CUDA(cudaMemsetAsync(derr, 0, sizeof(unsigned), s));
   const MlpWeights w = mlp_weights(reinterpret_cast<const __nv_bfloat16 *>(weights), biases);
-  rc = mlp_forward(w, x, batch, out, MlpActs{}, derr, s);
+  rc = mlp_forward(w, x, batch, out, derr, s);
   return rc == VPD_OK ? check_err(derr, s) : rc;
 }
 
@@ -402,40 +506,18 @@ extern "C" int vpd_mlp_gradients(const uint16_t *weights, const float *biases, c
     return set_error(VPD_ERR_INVALID, "vpd_mlp_gradients: invalid argument");
   cudaStream_t s = (cudaStream_t)stream;
   const MlpWeights w = mlp_weights(reinterpret_cast<const __nv_bfloat16 *>(weights), biases);
-  unsigned char *buf = nullptr;
-  const size_t nb = (size_t)batch;
-  const size_t blocks = (size_t)mlp_backward_blocks(batch);
-  const size_t bytes = nb * kMlpIn * 2 + nb * kMlpHidden * (4 * 3 + 2 * 3) + nb * kMlpOut * 4 + 256 +
-                       sizeof(float) * blocks * kMlpParams + sizeof(uint16_t) * kMlpWeights;
+  const int64_t blocks = mlp_gradient_blocks(batch);
   Workspace ws(s);
-  int rc = ws.alloc(&buf, bytes);
-  if (rc)
+  unsigned *derr = nullptr;
+  float *partials = nullptr;
+  int rc;
+  if ((rc = ws.alloc(&derr, 1)) || (rc = ws.alloc(&partials, (size_t)blocks * kMlpParams)))
     return rc;
-  MlpActs a;
-  unsigned char *q = buf;
-  a.y0 = reinterpret_cast<__nv_bfloat16 *>(q), q += nb * kMlpIn * 2;
-  a.z1 = reinterpret_cast<float *>(q), q += nb * kMlpHidden * 4;
-  a.z2 = reinterpret_cast<float *>(q), q += nb * kMlpHidden * 4;
-  a.z3 = reinterpret_cast<float *>(q), q += nb * kMlpHidden * 4;
-  a.y1 = reinterpret_cast<__nv_bfloat16 *>(q), q += nb * kMlpHidden * 2;
-  a.y2 = reinterpret_cast<__nv_bfloat16 *>(q), q += nb * kMlpHidden * 2;
-  a.y3 = reinterpret_cast<__nv_bfloat16 *>(q), q += nb * kMlpHidden * 2;
-  float *out = reinterpret_cast<float *>(q), *derrf = out + nb * kMlpOut;
-  unsigned *derr = reinterpret_cast<unsigned *>(derrf);
-  q = reinterpret_cast<unsigned char *>(derrf) + 256;
-  MlpBackwardScratch scr;
-  scr.partials = reinterpret_cast<float *>(q), q += sizeof(float) * blocks * kMlpParams;
-  scr.wt = reinterpret_cast<__nv_bfloat16 *>(q);
-  cudaError_t e = cudaMemsetAsync(derr, 0, sizeof(unsigned), s);
-  if (e == cudaSuccess)
-    e = cudaMemsetAsync(grad, 0, sizeof(float) * kMlpParams, s);
-  if (e != cudaSuccess)
-    rc = cuda_error(e, "vpd_mlp_gradients");
-  if (rc == VPD_OK)
-    rc = mlp_forward(w, x, batch, out, a, derr, s);
-  if (rc == VPD_OK)
-    rc = mlp_backward(w, a, gout, batch, grad, scr, derr, s);
-  if (rc == VPD_OK)
-    rc = check_err(derr, s);
-  return rc;
+  VPD_CUDA(cudaMemsetAsync(derr, 0, sizeof(unsigned), s));
+  MlpBatch rows{};
+  rows.x = x, rows.gout = gout;
+  if ((rc = mlp_gradient_partials(w, rows, batch, partials, derr, s)) ||
+      (rc = mlp_sum_partials(partials, blocks, grad, s)))
+    return rc;
+  return check_err(derr, s);
 }

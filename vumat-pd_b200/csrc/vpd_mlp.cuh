@@ -22,13 +22,6 @@ struct MlpWeights {
   const float *b1, *b2, *b3, *b4;
 };
 
-// Activations kept for the backward pass (any pointer may be null in inference).
-struct MlpActs {
-  __nv_bfloat16 *y0;              // [B][16] inputs as fed
-  float *z1, *z2, *z3;            // [B][128] pre-activations
-  __nv_bfloat16 *y1, *y2, *y3;    // [B][128] activations
-};
-
 struct MlpGrads {  // FP32 accumulators, same shapes as the parameters
   float *w1, *w2, *w3, *w4, *b1, *b2, *b3, *b4;
 };
@@ -42,21 +35,26 @@ __host__ __device__ inline MlpGrads mlp_grads(float *g) {
                   g + kMlpWeights, g + kMlpWeights + 128, g + kMlpWeights + 256, g + kMlpWeights + 384};
 }
 
-int mlp_forward(const MlpWeights &w, const float *x, int64_t B, float *out, const MlpActs &acts,
-                unsigned *err, cudaStream_t s);
-// Scratch of one backward pass: the transposed weights (VPD_MLP_WEIGHTS - 2048 bf16) and one
-// partial gradient per 128-row block (mlp_backward_blocks(B) x kMlpParams floats).
-struct MlpBackwardScratch {
-  __nv_bfloat16 *wt;
-  float *partials;
+// out [B][16] = network(x [B][16]).
+int mlp_forward(const MlpWeights &w, const float *x, int64_t B, float *out, unsigned *err, cudaStream_t s);
+
+// One pass for the gradient of a batch: partial gradients of sum(out * gout) per 128-row block into `partials`
+// (mlp_gradient_blocks(B) x kMlpParams floats). Rows are x's own, with gout given, or gathered from the training
+// set with gout of the weighted MSE (MlpBatch).
+int64_t mlp_gradient_blocks(int64_t B);
+struct MlpBatch {
+  const float *x, *gout;  // [B][16]; gout null: training rows, and the rest of this struct
+  const float *target;    // [rows][16], row weight in column 15; x is then [rows][16] too
+  int64_t rows, first;    // row r of the batch is row (mul (first + r) + add) % rows
+  uint64_t mul, add;
+  float *loss;            // += the batch's mean loss
 };
-int64_t mlp_backward_blocks(int64_t B);
-// grad [kMlpParams] = d/dparams of sum(out * gout) over the batch (overwritten, not accumulated).
-int mlp_backward(const MlpWeights &w, const MlpActs &acts, const float *gout, int64_t B, float *grad,
-                 const MlpBackwardScratch &scr, unsigned *err, cudaStream_t s);
-int mlp_adam(float *p, float *m, float *v, float *grad, __nv_bfloat16 *pb, int64_t n, float lr,
+int mlp_gradient_partials(const MlpWeights &w, const MlpBatch &batch, int64_t B, float *partials, unsigned *err,
+                          cudaStream_t s);
+// grad [kMlpParams] = the partials' sum in block order.
+int mlp_sum_partials(const float *partials, int64_t blocks, float *grad, cudaStream_t s);
+// The same sum taken straight into one Adam step on the parameters p (m, v: moments); wb: the weights' BF16 copy.
+int mlp_adam(const float *partials, int64_t blocks, float *p, float *m, float *v, __nv_bfloat16 *wb, float lr,
              int step, cudaStream_t s);
-int mlp_mse_grad(const float *out, const float *target, int64_t B, int cols, float *gout,
-                 float *loss, cudaStream_t s);
 
 }  // namespace vpd

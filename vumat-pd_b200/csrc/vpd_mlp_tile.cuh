@@ -26,6 +26,12 @@ __device__ __forceinline__ float silu(float z) {
   const float h = 0.5f * z;
   return fmaf(h, tanh_approx(h), h);
 }
+// silu(v + bias) of two columns as packed pairs, rounded to BF16: each lane with silu's operations.
+__device__ __forceinline__ __nv_bfloat162 silu2(float2 v, float2 bias) {
+  const float2 h = __fmul2_rn(__fadd2_rn(v, bias), make_float2(0.5f, 0.5f));
+  const float2 y = __ffma2_rn(h, make_float2(tanh_approx(h.x), tanh_approx(h.y)), h);
+  return __floats2bfloat162_rn(y.x, y.y);
+}
 __device__ __forceinline__ float silu_grad(float z) {
   const float s = fmaf(0.5f, tanh_approx(0.5f * z), 0.5f);
   return s * fmaf(z, 1.0f - s, 1.0f);
@@ -93,37 +99,29 @@ __device__ __forceinline__ void stage_biases(float *dst, const MlpWeights &w) {
                                                                         : w.b4[c - 3 * kMlpHidden]));
 }
 
-// Hidden-layer epilogue for the calling thread's row, 32 columns per TMEM load: bias, SiLU,
-// next operand (bf16) in A; optionally the pre-activation and activation to global memory.
-// `bias` points at the layer's 128 biases (shared or global memory, 16-byte aligned).
-__device__ __forceinline__ void hidden_epilogue(uint32_t trow, const float *bias, unsigned char *A, float *z_out,
-                                                __nv_bfloat16 *y_out) {
-  const int t = threadIdx.x;
+// Bias, SiLU and the BF16 rounding of 32 accumulator columns c0.. of the calling thread's row into the next
+// layer's operand A [128][128] (row t). `bias`: the layer's biases (shared memory, 16-byte aligned).
+__device__ __forceinline__ void hidden_columns(const float (&v)[32], const float *bias, unsigned char *A, int t, int c0) {
+  __align__(16) __nv_bfloat162 yb[16];
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const float4 bb = *reinterpret_cast<const float4 *>(bias + c0 + 4 * q);
+    yb[2 * q] = silu2(make_float2(v[4 * q], v[4 * q + 1]), make_float2(bb.x, bb.y));
+    yb[2 * q + 1] = silu2(make_float2(v[4 * q + 2], v[4 * q + 3]), make_float2(bb.z, bb.w));
+  }
+  // four 16-byte rows of core matrices
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    *reinterpret_cast<uint4 *>(A + kmajor_offset(t, c0 + 8 * k, kMlpHidden)) = *reinterpret_cast<const uint4 *>(yb + 4 * k);
+}
+
+// Hidden-layer epilogue of the calling thread's whole row t, 32 columns per TMEM load.
+__device__ __forceinline__ void hidden_epilogue(uint32_t trow, const float *bias, unsigned char *A, int t) {
 #pragma unroll 1
   for (int c0 = 0; c0 < kMlpHidden; c0 += 32) {
     float v[32];
     umma::tmem_ld32(trow + c0, v);
-    __align__(16) __nv_bfloat16 yb[32];
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      const float4 bb = *reinterpret_cast<const float4 *>(bias + c0 + 4 * q);
-      const float z[4] = {v[4 * q] + bb.x, v[4 * q + 1] + bb.y, v[4 * q + 2] + bb.z, v[4 * q + 3] + bb.w};
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        yb[4 * q + c] = __float2bfloat16(silu(z[c]));
-        if (z_out)
-          z_out[c0 + 4 * q + c] = z[c];
-      }
-    }
-    // four 16-byte rows of core matrices
-#pragma unroll
-    for (int k = 0; k < 4; ++k)
-      *reinterpret_cast<uint4 *>(A + kmajor_offset(t, c0 + 8 * k, kMlpHidden)) =
-          *reinterpret_cast<const uint4 *>(yb + 8 * k);
-    if (y_out)
-#pragma unroll
-      for (int k = 0; k < 4; ++k)
-        *reinterpret_cast<uint4 *>(y_out + c0 + 8 * k) = *reinterpret_cast<const uint4 *>(yb + 8 * k);
+    hidden_columns(v, bias, A, t, c0);
   }
 }
 

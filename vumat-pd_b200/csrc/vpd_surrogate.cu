@@ -147,44 +147,22 @@ int surrogate_samples_dev(const JcParams &jc, uint64_t seed, int64_t count, floa
 }
 
 // ------------------------------------------------------------------ training
-__global__ void k_gather_rows(const float *X, const float *Y, int64_t rows, uint64_t mul, uint64_t add,
-                              int64_t first, int64_t B, float *Xb, float *Yb) {
-  const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= B * 16)
-    return;
-  const int64_t r = e >> 4, c = e & 15;
-  const int64_t src = (int64_t)((mul * (uint64_t)(first + r) + add) % (uint64_t)rows);  // a permutation
-  Xb[e] = X[src * 16 + c];
-  Yb[e] = Y[src * 16 + c];
-}
-
-// Weighted MSE over the 7 targets (row weight in target column 15, target 0 weighted 4):
-// gout = d loss / d out, loss += this batch's mean.
-__global__ void k_weighted_mse(const float *out, const float *target, int64_t B, float *gout, float *loss) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  float l = 0.0f;
-  if (i < B) {
-    const float w = target[i * 16 + 15];
-    const float norm = 1.0f / (float)(B * SURROGATE_TARGETS);
-#pragma unroll
-    for (int c = 0; c < 16; ++c) {
-      const float cw = c == 0 ? 4.0f : 1.0f;
-      const float d = c < SURROGATE_TARGETS ? out[i * 16 + c] - target[i * 16 + c] : 0.0f;
-      gout[i * 16 + c] = 2.0f * w * cw * d * norm;
-      l += w * cw * d * d * norm;
-    }
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1)
-    l += __shfl_xor_sync(0xffffffffu, l, o);
-  if ((threadIdx.x & 31) == 0)
-    atomicAdd(loss, l);
-}
-
 __global__ void k_to_bf16(const float *p, __nv_bfloat16 *q, int64_t n) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n)
     q[i] = __float2bfloat16(p[i]);
+}
+
+// *sum += the plastic rows among the training targets (row weight 1 in column 15).
+__global__ void k_count_plastic(const float *Y, int64_t rows, unsigned long long *sum) {
+  int64_t k = 0;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < rows; i += (int64_t)gridDim.x * blockDim.x)
+    k += Y[i * 16 + 15] != 0.0f;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+    k += __shfl_xor_sync(0xffffffffu, k, o);
+  if ((threadIdx.x & 31) == 0)
+    atomicAdd(sum, (unsigned long long)k);
 }
 
 namespace {
@@ -246,25 +224,18 @@ int train_surrogate(const vpd_surrogate_config &cfg, uint16_t *w_out, float *b_o
   VPD_CUDA(cudaEventCreate(&g.e1));
   cudaStream_t s = g.s;
   Workspace buf(s);  // given back before the stream goes
-  float *X = nullptr, *Y = nullptr, *Xb = nullptr, *Yb = nullptr, *out = nullptr, *gout = nullptr;
-  float *z1 = nullptr, *z2 = nullptr, *z3 = nullptr, *P = nullptr, *M = nullptr, *Vm = nullptr, *G = nullptr;
+  float *X = nullptr, *Y = nullptr, *P = nullptr, *M = nullptr, *Vm = nullptr, *partials = nullptr;
   float *loss = nullptr, *vout = nullptr;
-  __nv_bfloat16 *y0 = nullptr, *y1 = nullptr, *y2 = nullptr, *y3 = nullptr, *Wb = nullptr;
+  __nv_bfloat16 *Wb = nullptr;
   unsigned *err = nullptr;
+  unsigned long long *plastic = nullptr;
   int rc;
-  const int64_t VB = std::max<int64_t>(V, 1);
-  if ((rc = buf.alloc(&X, S * 16)) || (rc = buf.alloc(&Y, S * 16)) || (rc = buf.alloc(&Xb, B * 16)) ||
-      (rc = buf.alloc(&Yb, B * 16)) || (rc = buf.alloc(&out, B * 16)) || (rc = buf.alloc(&gout, B * 16)) ||
-      (rc = buf.alloc(&z1, B * 128)) || (rc = buf.alloc(&z2, B * 128)) || (rc = buf.alloc(&z3, B * 128)) ||
-      (rc = buf.alloc(&y0, B * 16)) || (rc = buf.alloc(&y1, B * 128)) || (rc = buf.alloc(&y2, B * 128)) ||
-      (rc = buf.alloc(&y3, B * 128)) || (rc = buf.alloc(&P, kMlpParams)) || (rc = buf.alloc(&M, kMlpParams)) ||
-      (rc = buf.alloc(&Vm, kMlpParams)) || (rc = buf.alloc(&G, kMlpParams)) || (rc = buf.alloc(&Wb, kMlpWeights)) ||
+  const int64_t VB = std::max<int64_t>(V, 1), blocks = mlp_gradient_blocks(B);
+  if ((rc = buf.alloc(&X, S * 16)) || (rc = buf.alloc(&Y, S * 16)) || (rc = buf.alloc(&P, kMlpParams)) ||
+      (rc = buf.alloc(&M, kMlpParams)) || (rc = buf.alloc(&Vm, kMlpParams)) || (rc = buf.alloc(&Wb, kMlpWeights)) ||
+      (rc = buf.alloc(&partials, (size_t)blocks * kMlpParams)) ||
       (rc = buf.alloc(&loss, VPD_SURROGATE_MAX_EPOCHS + 1)) || (rc = buf.alloc(&vout, VB * 16)) ||
-      (rc = buf.alloc(&err, 1)))
-    return rc;
-  MlpBackwardScratch bscr{};
-  if ((rc = buf.alloc(&bscr.wt, kMlpWeights)) ||
-      (rc = buf.alloc(&bscr.partials, (size_t)mlp_backward_blocks(B) * kMlpParams)))
+      (rc = buf.alloc(&err, 1)) || (rc = buf.alloc(&plastic, 1)))
     return rc;
   if ((rc = surrogate_samples_dev(jc, cfg.seed, S, X, Y, nullptr, s)))
     return rc;
@@ -290,39 +261,34 @@ int train_surrogate(const vpd_surrogate_config &cfg, uint16_t *w_out, float *b_o
   VPD_CUDA(cudaMemcpyAsync(P, p0.data(), sizeof(float) * kMlpParams, cudaMemcpyHostToDevice, s));
   VPD_CUDA(cudaMemsetAsync(M, 0, sizeof(float) * kMlpParams, s));
   VPD_CUDA(cudaMemsetAsync(Vm, 0, sizeof(float) * kMlpParams, s));
-  VPD_CUDA(cudaMemsetAsync(G, 0, sizeof(float) * kMlpParams, s));
+  VPD_CUDA(cudaMemsetAsync(plastic, 0, sizeof(unsigned long long), s));
+  k_count_plastic<<<148, 256, 0, s>>>(Y, S, plastic);
+  VPD_CUDA(cudaGetLastError());
   VPD_CUDA(cudaMemsetAsync(loss, 0, sizeof(float) * (VPD_SURROGATE_MAX_EPOCHS + 1), s));
   VPD_CUDA(cudaMemsetAsync(err, 0, sizeof(unsigned), s));
   k_to_bf16<<<(unsigned)((kMlpWeights + 255) / 256), 256, 0, s>>>(P, Wb, kMlpWeights);
   VPD_CUDA(cudaGetLastError());
 
   const MlpWeights w = mlp_weights(Wb, P + kMlpWeights);
-  const MlpActs acts{y0, z1, z2, z3, y1, y2, y3};
   const int64_t steps = T / B;
   int adam_step = 0;
+  MlpBatch batch{};
+  batch.x = X, batch.target = Y, batch.rows = T;
   VPD_CUDA(cudaEventRecord(g.e0, s));
   for (int e = 0; e < cfg.epochs; ++e) {
-    const uint64_t mul = epoch_multiplier((uint64_t)T, e), add = (uint64_t)e * 7919u % (uint64_t)T;
+    batch.mul = epoch_multiplier((uint64_t)T, e), batch.add = (uint64_t)e * 7919u % (uint64_t)T;  // a permutation
+    batch.loss = loss + e;
     for (int64_t k = 0; k < steps; ++k) {
-      k_gather_rows<<<(unsigned)((B * 16 + 255) / 256), 256, 0, s>>>(X, Y, T, mul, add, k * B, B, Xb, Yb);
-      VPD_CUDA(cudaGetLastError());
-      if ((rc = mlp_forward(w, Xb, B, out, acts, err, s)))
-        return rc;
-      k_weighted_mse<<<(unsigned)((B + 255) / 256), 256, 0, s>>>(out, Yb, B, gout, loss + e);
-      VPD_CUDA(cudaGetLastError());
-      if ((rc = mlp_backward(w, acts, gout, B, G, bscr, err, s)))
-        return rc;
-      ++adam_step;
-      if ((rc = mlp_adam(P, M, Vm, G, Wb, kMlpWeights, (float)cfg.learning_rate, adam_step, s)) ||
-          (rc = mlp_adam(P + kMlpWeights, M + kMlpWeights, Vm + kMlpWeights, G + kMlpWeights, nullptr,
-                         kMlpParams - kMlpWeights, (float)cfg.learning_rate, adam_step, s)))
+      batch.first = k * B;
+      if ((rc = mlp_gradient_partials(w, batch, B, partials, err, s)) ||
+          (rc = mlp_adam(partials, blocks, P, M, Vm, Wb, (float)cfg.learning_rate, ++adam_step, s)))
         return rc;
     }
   }
   VPD_CUDA(cudaEventRecord(g.e1, s));
   // held-out rows: forward pass and the weighted loss
   if (V > 0) {
-    if ((rc = mlp_forward(w, X + T * 16, V, vout, MlpActs{}, err, s)))
+    if ((rc = mlp_forward(w, X + T * 16, V, vout, err, s)))
       return rc;
   }
   std::vector<float> losses(VPD_SURROGATE_MAX_EPOCHS + 1), hv((size_t)V * 16), hy((size_t)V * 16);
@@ -337,10 +303,8 @@ int train_surrogate(const vpd_surrogate_config &cfg, uint16_t *w_out, float *b_o
   VPD_CUDA(cudaMemcpyAsync(hw.data(), Wb, sizeof(uint16_t) * kMlpWeights, cudaMemcpyDeviceToHost, s));
   VPD_CUDA(cudaMemcpyAsync(b_out, P + kMlpWeights, sizeof(float) * (kMlpParams - kMlpWeights),
                            cudaMemcpyDeviceToHost, s));
-  // plastic fraction over all samples (target column 15)
-  std::vector<float> all_w((size_t)S);
-  VPD_CUDA(cudaMemcpy2DAsync(all_w.data(), sizeof(float), Y + 15, 16 * sizeof(float), sizeof(float), (size_t)S,
-                             cudaMemcpyDeviceToHost, s));
+  unsigned long long nplastic = 0;
+  VPD_CUDA(cudaMemcpyAsync(&nplastic, plastic, sizeof nplastic, cudaMemcpyDeviceToHost, s));
   VPD_CUDA(cudaStreamSynchronize(s));
   if (herr)
     return set_error(VPD_ERR_CUDA, "vpd_train_surrogate: tensor-core wait timed out");
@@ -368,10 +332,7 @@ int train_surrogate(const vpd_surrogate_config &cfg, uint16_t *w_out, float *b_o
     rep->validation_loss = V ? vl / ((double)V * SURROGATE_TARGETS) : 0.0;
     rep->ratio_rmse = np ? std::sqrt(r2 / np) : 0.0;
     rep->stress_rmse = np ? std::sqrt(s2 / (np * 6.0)) : 0.0;
-    double pf = 0.0;
-    for (float x : all_w)
-      pf += x;
-    rep->plastic_fraction = S ? pf / (double)S : 0.0;
+    rep->plastic_fraction = S ? (double)nplastic / (double)S : 0.0;
     float ms = 0.0f;
     VPD_CUDA(cudaEventElapsedTime(&ms, g.e0, g.e1));
     rep->train_ms = ms;
@@ -565,13 +526,13 @@ __global__ void __launch_bounds__(kMaterialThreads, MINB)
           st_bf16(sX, t, c, kMlpIn, c < SURROGATE_FEATURES ? f[c] : 0.0f);
         gemm(sy, tmem, sX, sW1, kMlpIn, kMlpHidden);
         if (sy.ok)
-          hidden_epilogue(trow, sBias, sA, nullptr, nullptr);
+          hidden_epilogue(trow, sBias, sA, t);
         gemm(sy, tmem, sA, sW2, kMlpHidden, kMlpHidden);
         if (sy.ok)
-          hidden_epilogue(trow, sBias + kMlpHidden, sA, nullptr, nullptr);
+          hidden_epilogue(trow, sBias + kMlpHidden, sA, t);
         gemm(sy, tmem, sA, sW3, kMlpHidden, kMlpHidden);
         if (sy.ok)
-          hidden_epilogue(trow, sBias + 2 * kMlpHidden, sA, nullptr, nullptr);
+          hidden_epilogue(trow, sBias + 2 * kMlpHidden, sA, t);
         gemm(sy, tmem, sA, sW4, kMlpHidden, kMlpOut);
         if (sy.ok) {
           float v[16];

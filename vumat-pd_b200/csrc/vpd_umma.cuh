@@ -43,6 +43,21 @@ __host__ __device__ constexpr uint32_t idesc_bf16(int m, int n) {
          | ((uint32_t)(m >> 4) << 24);   // M / 16
 }
 
+// An operand in shared memory, a tile stored [rows][cols] in the core-matrix layout above (cols the
+// contiguous dimension), as the K-major operand (K = cols) or, read the other way, as the MN-major operand (K =
+// rows): a core matrix is 8 rows x 16 bytes either way, so a transposed product needs no second copy. lbo
+// and sbo as the descriptor takes them, step the bytes from one K = 16 slice to the next.
+struct Operand {
+  uint32_t addr, lbo, sbo, step, mn_major;
+};
+__device__ __forceinline__ Operand k_major(const void *tile, int cols) {
+  return {smem_u32(tile), 128u, (uint32_t)(cols / 8) * 128u, 256u, 0u};
+}
+__device__ __forceinline__ Operand mn_major(const void *tile, int cols) {
+  const uint32_t group = (uint32_t)(cols / 8) * 128u;  // eight rows
+  return {smem_u32(tile), group, 128u, 2u * group, 1u};
+}
+
 __device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc,
                                          uint32_t idesc, uint32_t accumulate) {
   asm volatile(
@@ -153,6 +168,14 @@ __device__ __forceinline__ void gemm_issue(uint32_t tmem_d, uint32_t a_addr, uin
     const uint64_t bd = smem_desc(b_addr + kk * 256u, 128u, sbo_b);
     mma_bf16(tmem_d, ad, bd, idesc, (accumulate || kk > 0) ? 1u : 0u);
   }
+}
+
+// D[128 x N] (TMEM, FP32) = A[128 x K] * B[N x K]^T, each operand in either direction; issued by one thread.
+__device__ __forceinline__ void gemm_issue(uint32_t tmem_d, const Operand &a, const Operand &b, int K, int N) {
+  const uint32_t idesc = idesc_bf16(128, N) | (a.mn_major << 15) | (b.mn_major << 16);
+  for (int kk = 0; kk < K / 16; ++kk)
+    mma_bf16(tmem_d, smem_desc(a.addr + kk * a.step, a.lbo, a.sbo), smem_desc(b.addr + kk * b.step, b.lbo, b.sbo),
+             idesc, kk > 0 ? 1u : 0u);
 }
 
 }  // namespace umma
