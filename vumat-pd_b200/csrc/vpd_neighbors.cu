@@ -10,9 +10,16 @@
 // rounded root does not exceed r (found once on the host).
 //
 // Device passes: |x| max reduction; cell coordinates and their bounding box; counting sort
-// of points into a dense cell grid; a warp per point counts its matches; an exclusive scan
-// gives row_ptr; a warp per point gathers its matches with ballot compaction into shared
-// memory and bitonic-sorts the row before writing it.
+// of points into a dense cell grid; the matches of every point counted; an exclusive scan
+// gives row_ptr; the matches written in ascending order.
+//
+// The search runs a block per cell (k_nb_cell): the points of the 27 cells around it are sorted by
+// index once for all of its points, so a row's matches come out in order by ballot compaction and no row is
+// sorted by itself. Distances are decided in FP32, in units of the cell width and relative to a point of the
+// cell, outside a margin of 2e-5 of the squared radius (ten times their error), and by the exact test within it;
+// chunks of 32 candidates whose bounding box lies beyond the radius are skipped. Where the points are too
+// sparse or too dense for that (fewer than kMinCellPoints a cell on average, or more than kMaxCandidates around
+// one), a warp per point searches the cells and bitonic-sorts its row (k_nb_count, k_nb_fill).
 #include "vpd_internal.h"
 
 #include <algorithm>
@@ -140,8 +147,8 @@ int scan_exclusive_i32(const int32_t *in, int64_t n, int64_t *out, int64_t *tmp,
 
 // ------------------------------------------------------------------ neighbour kernels
 // reduce words: [0] max |x| bits, [1] non-finite flag, [2..4] min cell, [5..7] max cell,
-// [8] max row length.
-constexpr int kReduceWords = 9;
+// [8] max row length, [9] max candidates around a cell.
+constexpr int kReduceWords = 10;
 
 __global__ void k_abs_max(const double4 *xv, int64_t n, unsigned long long *red) {
   unsigned long long m = 0;
@@ -357,6 +364,196 @@ __global__ void k_nb_fill(const double4 *xv, int64_t n, const long long *cc, Gri
     row[t] = buf[t];
 }
 
+// ------------------------------------------------------------------ search by cell
+constexpr int kMaxCandidates = 4096;  // 80 KB of shared memory
+constexpr int kMinCellPoints = 4;
+constexpr int kCellThreads = 256;
+
+// The nine runs of `sorted` that hold the points of the 27 cells around cell c (the three along the last
+// dimension are consecutive): run k of lane k < 9.
+struct CellRun {
+  int64_t begin;
+  int count;
+};
+__device__ __forceinline__ CellRun cell_run(int64_t c, const GridDev &g, const int64_t *cell_start, int k) {
+  const long long c2 = c % g.d2, c1 = (c / g.d2) % g.d1, c0 = c / (g.d2 * g.d1);
+  const long long x0 = c0 + k / 3 - 1, x1 = c1 + k % 3 - 1;
+  if (k >= 9 || x0 < 0 || x0 >= g.d0 || x1 < 0 || x1 >= g.d1)
+    return {0, 0};
+  const long long row = (x0 * g.d1 + x1) * g.d2;
+  const long long lo = c2 > 0 ? c2 - 1 : 0, hi = c2 + 1 < g.d2 ? c2 + 1 : g.d2 - 1;
+  const int64_t b = cell_start[row + lo];
+  return {b, (int)(cell_start[row + hi + 1] - b)};
+}
+
+// The most candidates of any cell that holds points.
+__global__ void k_cell_candidates(int64_t ncells, GridDev g, const int64_t *cell_start, unsigned long long *most) {
+  const int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  unsigned total = 0;
+  if (c < ncells && cell_start[c + 1] > cell_start[c])
+    for (int k = 0; k < 9; ++k)
+      total += (unsigned)cell_run(c, g, cell_start, k).count;
+  total = __reduce_max_sync(0xffffffffu, total);
+  if ((threadIdx.x & 31) == 0 && total)
+    atomicMax(most, (unsigned long long)total);
+}
+
+// Ascending bitonic sort of `width` (a power of two, at least 32) shared-memory ints by the whole block.
+__device__ __forceinline__ void block_sort(int32_t *a, int width) {
+  for (int k = 2; k <= width; k <<= 1)
+    for (int j = k >> 1; j > 0; j >>= 1) {
+      for (int t = threadIdx.x; t < width / 2; t += kCellThreads) {
+        const int lo = 2 * t - (t & (j - 1)), hi = lo + j;
+        const int32_t x = a[lo], y = a[hi];
+        if ((x > y) == ((lo & k) == 0))
+          a[lo] = y, a[hi] = x;
+      }
+      __syncthreads();
+    }
+}
+
+struct CellSearch {
+  double inv_width, dist2_max;
+  float r2lo, r2hi;  // (radius / cell width)^2 less and plus the margin
+};
+
+// One block per cell. FILL: the rows of the cell's points into col; else their lengths into len (and the largest to
+// *longest).
+template <bool FILL>
+__global__ void __launch_bounds__(kCellThreads) k_nb_cell(const double4 *xv, GridDev g, const int64_t *cell_start,
+                                                          const int32_t *sorted, CellSearch cs, int width,
+                                                          const int64_t *row_ptr, int32_t *col, int32_t *len,
+                                                          unsigned long long *longest) {
+  extern __shared__ __align__(16) unsigned char s_cell[];
+  float4 *cand = reinterpret_cast<float4 *>(s_cell);  // position relative to the cell's first point, index
+  int32_t *index = reinterpret_cast<int32_t *>(cand + width);
+  float *box = reinterpret_cast<float *>(index + width);  // per 32 candidates: lowest x, y, z, highest x, y, z
+  __shared__ int64_t s_begin[9];
+  __shared__ int s_off[10];
+  const int64_t c = blockIdx.x, first = cell_start[c], last = cell_start[c + 1];
+  if (first == last)
+    return;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (threadIdx.x < 32) {
+    const CellRun r = cell_run(c, g, cell_start, lane);
+    int off = r.count;
+#pragma unroll
+    for (int o = 1; o < 16; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, off, o);
+      if (lane >= o)
+        off += y;
+    }
+    if (lane < 9)
+      s_begin[lane] = r.begin, s_off[lane + 1] = off;
+    if (lane == 0)
+      s_off[0] = 0;
+  }
+  __syncthreads();
+  const int total = s_off[9];
+  int w2 = 32;
+  while (w2 < total)
+    w2 <<= 1;
+  for (int k = 0; k < 9; ++k)
+    for (int t = s_off[k] + threadIdx.x; t < s_off[k + 1]; t += kCellThreads)
+      index[t] = sorted[s_begin[k] + (t - s_off[k])];
+  for (int t = total + threadIdx.x; t < w2; t += kCellThreads)
+    index[t] = INT_MAX;
+  __syncthreads();
+  block_sort(index, w2);
+  const double4 ref = xv[sorted[first]];
+  for (int t = threadIdx.x; t < total; t += kCellThreads) {
+    const double4 p = xv[index[t]];
+    cand[t] = make_float4((float)((p.x - ref.x) * cs.inv_width), (float)((p.y - ref.y) * cs.inv_width),
+                          (float)((p.z - ref.z) * cs.inv_width), __int_as_float(index[t]));
+  }
+  __syncthreads();
+  const int chunks = (total + 31) / 32;
+  for (int k = warp; k < chunks; k += kCellThreads / 32) {
+    const float4 p = cand[min(32 * k + lane, total - 1)];
+    float lo[3] = {p.x, p.y, p.z}, hi[3] = {p.x, p.y, p.z};
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        lo[d] = fminf(lo[d], __shfl_xor_sync(0xffffffffu, lo[d], o));
+        hi[d] = fmaxf(hi[d], __shfl_xor_sync(0xffffffffu, hi[d], o));
+      }
+    if (lane < 6)
+      box[6 * k + lane] = lane == 0 ? lo[0] : lane == 1 ? lo[1] : lane == 2 ? lo[2] : lane == 3 ? hi[0] : lane == 4 ? hi[1] : hi[2];
+  }
+  __syncthreads();
+  const unsigned lt = (1u << lane) - 1u;
+  int most = 0;
+  for (int64_t q = first + warp; q < last; q += kCellThreads / 32) {
+    const int32_t i = sorted[q];
+    const double4 pi = xv[i];
+    const float x = (float)((pi.x - ref.x) * cs.inv_width), y = (float)((pi.y - ref.y) * cs.inv_width),
+                z = (float)((pi.z - ref.z) * cs.inv_width);
+    int32_t *row = FILL ? col + row_ptr[i] : nullptr;
+    int cnt = 0;
+    for (int k0 = 0; k0 < chunks; k0 += 32) {
+      bool near = false;
+      if (k0 + lane < chunks) {
+        const float *b = box + 6 * (k0 + lane);
+        const float dx = fmaxf(fmaxf(b[0] - x, x - b[3]), 0.0f), dy = fmaxf(fmaxf(b[1] - y, y - b[4]), 0.0f),
+                    dz = fmaxf(fmaxf(b[2] - z, z - b[5]), 0.0f);
+        near = dx * dx + dy * dy + dz * dz <= cs.r2hi;
+      }
+      for (unsigned m = __ballot_sync(0xffffffffu, near); m; m &= m - 1) {
+        const int t = 32 * (k0 + __ffs(m) - 1) + lane;
+        bool keep = false;
+        int32_t j = 0;
+        if (t < total) {
+          const float4 p = cand[t];
+          j = __float_as_int(p.w);
+          const float dx = p.x - x, dy = p.y - y, dz = p.z - z, s = dx * dx + dy * dy + dz * dz;
+          keep = s < cs.r2lo;
+          if (!keep && s <= cs.r2hi)
+            keep = within(xv[j], pi, cs.dist2_max);
+          keep = keep && j != i;
+        }
+        const unsigned hit = __ballot_sync(0xffffffffu, keep);
+        if (FILL && keep)
+          row[cnt + __popc(hit & lt)] = j;
+        cnt += __popc(hit);
+      }
+    }
+    if (!FILL) {
+      if (lane == 0)
+        len[i] = cnt;
+      most = max(most, cnt);
+    }
+  }
+  if (!FILL && lane == 0 && most > 0)
+    atomicMax(longest, (unsigned long long)most);
+}
+
+// Shared memory of k_nb_cell for `candidates` points around a cell.
+static int cell_width(int candidates) {
+  int w = 32;
+  while (w < candidates)
+    w <<= 1;
+  return w;
+}
+static size_t cell_smem(int width) {
+  return (size_t)width * (sizeof(float4) + sizeof(int32_t)) + (size_t)(width / 32) * 6 * sizeof(float);
+}
+
+template <bool FILL>
+static int launch_cells(const double4 *xv, const NeighborGrid &grid, const NeighborScratch &scr, const int64_t *row_ptr,
+                        int32_t *col, cudaStream_t s) {
+  const GridDev g{grid.lo[0], grid.lo[1], grid.lo[2], grid.dims[0], grid.dims[1], grid.dims[2]};
+  const double inv = 1.0 / grid.cell_width, r2 = grid.dist2_max * inv * inv;
+  const CellSearch cs{inv, grid.dist2_max, (float)(r2 * (1.0 - 2.0e-5)), (float)(r2 * (1.0 + 2.0e-5))};
+  const int width = cell_width(grid.candidates);
+  const size_t smem = cell_smem(width);
+  VPD_CUDA(cudaFuncSetAttribute(k_nb_cell<FILL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  k_nb_cell<FILL><<<(unsigned)grid.ncells, kCellThreads, smem, s>>>(xv, g, scr.cell_start, scr.sorted, cs, width, row_ptr,
+                                                                    col, scr.len, scr.reduce + 8);
+  VPD_CUDA(cudaGetLastError());
+  return VPD_OK;
+}
+
 // ------------------------------------------------------------------ host orchestration
 template <typename T> static int scratch(NeighborScratch &scr, T **p, int64_t count) {
   return workspace_alloc(reinterpret_cast<void **>(p), sizeof(T) * (size_t)std::max<int64_t>(count, 1), scr.stream);
@@ -402,7 +599,7 @@ int neighbor_count(const double4 *xv, int64_t n, double horizon, int64_t *row_pt
   unsigned long long init[kReduceWords] = {0, 0,
                                            (unsigned long long)LLONG_MAX, (unsigned long long)LLONG_MAX,
                                            (unsigned long long)LLONG_MAX, (unsigned long long)LLONG_MIN,
-                                           (unsigned long long)LLONG_MIN, (unsigned long long)LLONG_MIN, 0};
+                                           (unsigned long long)LLONG_MIN, (unsigned long long)LLONG_MIN, 0, 0};
   VPD_CUDA(cudaMemcpyAsync(scr.reduce, init, sizeof init, cudaMemcpyHostToDevice, s));
   k_abs_max<<<grid_for(n, 256), 256, 0, s>>>(xv, n, scr.reduce);
   unsigned long long red[kReduceWords];
@@ -454,9 +651,25 @@ int neighbor_count(const double4 *xv, int64_t n, double horizon, int64_t *row_pt
     return rc;
   VPD_CUDA(cudaMemsetAsync(scr.cell_count, 0, sizeof(int32_t) * (size_t)(grid.ncells + 1), s));
   k_cell_scatter<<<pb, 256, 0, s>>>(scr.cell_of, n, scr.cell_start, scr.cell_count, scr.sorted);
-  const unsigned wb = (unsigned)((n + kNbWarps - 1) / kNbWarps);
-  k_nb_count<<<wb, 32 * kNbWarps, 0, s>>>(xv, n, scr.cell_coords, g, scr.cell_start, scr.sorted,
-                                          grid.dist2_max, scr.len, scr.reduce);
+  // the search by cell needs a few points a cell, candidates that fit shared memory, and a cell width whose
+  // reciprocal and square are ordinary numbers
+  grid.candidates = 0;
+  if (grid.ncells * kMinCellPoints <= n && grid.cell_width > 1.0e-100 && grid.cell_width < 1.0e100) {
+    k_cell_candidates<<<(unsigned)((grid.ncells + 255) / 256), 256, 0, s>>>(grid.ncells, g, scr.cell_start,
+                                                                           scr.reduce + 9);
+    VPD_CUDA(cudaMemcpyAsync(red, scr.reduce, sizeof red, cudaMemcpyDeviceToHost, s));
+    VPD_CUDA(cudaStreamSynchronize(s));
+    if (red[9] <= (unsigned long long)kMaxCandidates)
+      grid.candidates = (int)red[9];
+  }
+  if (grid.candidates) {
+    if ((rc = launch_cells<false>(xv, grid, scr, nullptr, nullptr, s)))
+      return rc;
+  } else {
+    const unsigned wb = (unsigned)((n + kNbWarps - 1) / kNbWarps);
+    k_nb_count<<<wb, 32 * kNbWarps, 0, s>>>(xv, n, scr.cell_coords, g, scr.cell_start, scr.sorted,
+                                            grid.dist2_max, scr.len, scr.reduce);
+  }
   // reuse the cell scan scratch when large enough, else the row scan needs its own
   int64_t *tmp = scr.scan_tmp;
   int64_t *own = nullptr;
@@ -479,6 +692,13 @@ int neighbor_count(const double4 *xv, int64_t n, double horizon, int64_t *row_pt
 
 int neighbor_fill(const double4 *xv, int64_t n, const int64_t *row_ptr, int32_t *col,
                   const NeighborGrid &grid, const NeighborScratch &scr, cudaStream_t s) {
+  if (grid.candidates) {  // the rows have the counted lengths: nothing to report
+    const int rc = launch_cells<true>(xv, grid, scr, row_ptr, col, s);
+    if (rc)
+      return rc;
+    VPD_CUDA(cudaStreamSynchronize(s));
+    return VPD_OK;
+  }
   int cap = 32;
   while (cap < grid.max_len)
     cap <<= 1;
