@@ -20,7 +20,9 @@
 // chunks of 32 candidates whose bounding box lies beyond the radius are skipped. Where the points are too
 // sparse or too dense for that (fewer than kMinCellPoints a cell on average, or more than kMaxCandidates around
 // one), a warp per point searches the cells and bitonic-sorts its row (k_nb_count, k_nb_fill).
-#include "vpd_internal.h"
+// 250,000 jittered points, horizon 4.015 h, on a B200: count 275 us, fill 395 us (1390 and 2565 per point); both
+// issue-bound (73 %), about a third of it sorting and placing the candidates of the 5,096 cells.
+#include "vpd_bond.cuh"  // bcast2
 
 #include <algorithm>
 #include <cfloat>
@@ -146,56 +148,38 @@ int scan_exclusive_i32(const int32_t *in, int64_t n, int64_t *out, int64_t *tmp,
 }
 
 // ------------------------------------------------------------------ neighbour kernels
-// reduce words: [0] max |x| bits, [1] non-finite flag, [2..4] min cell, [5..7] max cell,
-// [8] max row length, [9] max candidates around a cell.
-constexpr int kReduceWords = 10;
+// reduce words: [0] max row length, [1] flags (1: non-finite coordinate, 2: a row beyond its buffer), [2..4] min
+// coordinate, [5..7] max coordinate (order_key), [8] max candidates around a cell.
+constexpr int kReduceWords = 9;
 
-__global__ void k_abs_max(const double4 *xv, int64_t n, unsigned long long *red) {
-  unsigned long long m = 0;
-  unsigned int bad = 0;
+// Doubles as integers of the same order (a finite number and its key determine each other).
+__host__ __device__ __forceinline__ long long order_key(long long bits) {
+  return bits < 0 ? bits ^ 0x7fffffffffffffffll : bits;
+}
+static double key_value(unsigned long long key) {
+  const long long bits = order_key((long long)key);
+  double v;
+  memcpy(&v, &bits, sizeof v);
+  return v;
+}
+
+__global__ void __launch_bounds__(256) k_bounds(const double4 *xv, int64_t n, unsigned long long *red) {
+  long long lo[3] = {LLONG_MAX, LLONG_MAX, LLONG_MAX}, hi[3] = {LLONG_MIN, LLONG_MIN, LLONG_MIN};
+  bool bad = false;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x) {
     const double4 p = xv[i];
     const double c[3] = {p.x, p.y, p.z};
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-      if (!isfinite(c[d]))
-        bad = 1;
-      const unsigned long long b = (unsigned long long)__double_as_longlong(fabs(c[d]));
-      m = b > m ? b : m;
+      bad = bad || !isfinite(c[d]);
+      const long long k = order_key(__double_as_longlong(c[d]));
+      lo[d] = k < lo[d] ? k : lo[d];
+      hi[d] = k > hi[d] ? k : hi[d];
     }
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const unsigned long long y = __shfl_xor_sync(0xffffffffu, m, o);
-    m = y > m ? y : m;
-    bad |= __shfl_xor_sync(0xffffffffu, bad, o);
-  }
-  if ((threadIdx.x & 31) == 0) {
-    atomicMax(&red[0], m);
-    if (bad)
-      atomicOr(&red[1], 1ull);
-  }
-}
-
-__device__ __forceinline__ long long cell_coord(double x, double cw) {
-  return (long long)floor(__ddiv_rn(x, cw));
-}
-
-__global__ void k_cell_coords(const double4 *xv, int64_t n, double cw, long long *cc,
-                              long long *red) {
-  long long lo[3] = {LLONG_MAX, LLONG_MAX, LLONG_MAX}, hi[3] = {LLONG_MIN, LLONG_MIN, LLONG_MIN};
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    const double4 p = xv[i];
-    const long long c[3] = {cell_coord(p.x, cw), cell_coord(p.y, cw), cell_coord(p.z, cw)};
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      cc[3 * i + d] = c[d];
-      lo[d] = c[d] < lo[d] ? c[d] : lo[d];
-      hi[d] = c[d] > hi[d] ? c[d] : hi[d];
-    }
-  }
+  __shared__ long long s_lo[8][3], s_hi[8][3];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
 #pragma unroll
@@ -205,24 +189,39 @@ __global__ void k_cell_coords(const double4 *xv, int64_t n, double cw, long long
       lo[d] = a < lo[d] ? a : lo[d];
       hi[d] = b > hi[d] ? b : hi[d];
     }
-    if ((threadIdx.x & 31) == 0) {
-      atomicMin(&red[2 + d], lo[d]);
-      atomicMax(&red[5 + d], hi[d]);
-    }
+    if (lane == 0)
+      s_lo[warp][d] = lo[d], s_hi[warp][d] = hi[d];
   }
+  const bool any = __syncthreads_or(bad);
+  if (threadIdx.x < 3) {
+    const int d = threadIdx.x;
+    long long a = s_lo[0][d], b = s_hi[0][d];
+    for (int w = 1; w < 8; ++w)
+      a = s_lo[w][d] < a ? s_lo[w][d] : a, b = s_hi[w][d] > b ? s_hi[w][d] : b;
+    atomicMin((long long *)red + 2 + d, a);
+    atomicMax((long long *)red + 5 + d, b);
+  }
+  if (any && threadIdx.x == 0)
+    atomicOr(&red[1], 1ull);
+}
+
+__device__ __forceinline__ long long cell_coord(double x, double cw) {
+  return (long long)floor(__ddiv_rn(x, cw));
 }
 
 struct GridDev {
   long long lo0, lo1, lo2, d0, d1, d2;
 };
 
-__global__ void k_cell_assign(const long long *cc, int64_t n, GridDev g, int32_t *cell_of,
+__global__ void k_cell_assign(const double4 *xv, int64_t n, double cw, GridDev g, long long *cc, int32_t *cell_of,
                               int32_t *count) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= n)
     return;
-  const long long c =
-      ((cc[3 * i] - g.lo0) * g.d1 + (cc[3 * i + 1] - g.lo1)) * g.d2 + (cc[3 * i + 2] - g.lo2);
+  const double4 p = xv[i];
+  const long long x = cell_coord(p.x, cw), y = cell_coord(p.y, cw), z = cell_coord(p.z, cw);
+  cc[3 * i] = x, cc[3 * i + 1] = y, cc[3 * i + 2] = z;
+  const long long c = ((x - g.lo0) * g.d1 + (y - g.lo1)) * g.d2 + (z - g.lo2);
   cell_of[i] = (int32_t)c;
   atomicAdd(&count[c], 1);
 }
@@ -241,6 +240,10 @@ __device__ __forceinline__ bool within(const double4 &pj, const double4 &pi, dou
   const double a0 = __dsub_rn(pj.x, pi.x), a1 = __dsub_rn(pj.y, pi.y), a2 = __dsub_rn(pj.z, pi.z);
   const double s = __dadd_rn(__dadd_rn(__dmul_rn(a0, a0), __dmul_rn(a1, a1)), __dmul_rn(a2, a2));
   return s <= dist2_max;
+}
+
+static __device__ __noinline__ bool within_exact(const double4 *xv, int32_t j, int32_t i, double dist2_max) {
+  return within(xv[j], xv[i], dist2_max);
 }
 
 constexpr int kNbWarps = 8;
@@ -283,7 +286,7 @@ __global__ void k_nb_count(const double4 *xv, int64_t n, const long long *cc, Gr
     cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
   if (lane == 0) {
     len[i] = cnt;
-    atomicMax(&red[8], (unsigned long long)cnt);
+    atomicMax(&red[0], (unsigned long long)cnt);
   }
 }
 
@@ -365,7 +368,7 @@ __global__ void k_nb_fill(const double4 *xv, int64_t n, const long long *cc, Gri
 }
 
 // ------------------------------------------------------------------ search by cell
-constexpr int kMaxCandidates = 4096;  // 80 KB of shared memory
+constexpr int kMaxCandidates = 4096;  // 99 KB of shared memory
 constexpr int kMinCellPoints = 4;
 constexpr int kCellThreads = 256;
 
@@ -412,6 +415,55 @@ __device__ __forceinline__ void block_sort(int32_t *a, int width) {
     }
 }
 
+// Sorts the `total` distinct ints of a (lowest `lo`) by setting their bits in `bits` (words 32-bit words, range of the
+// values at most 32 words) and listing the set bits: a fraction of the comparisons' work where the indices around a
+// cell lie close together, as those of a lattice do.
+__device__ __forceinline__ void block_sort_bits(int32_t *a, int total, int32_t lo, uint32_t *bits, int words) {
+  __shared__ int s_warp[kCellThreads / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int w = threadIdx.x; w < words; w += kCellThreads)
+    bits[w] = 0u;
+  __syncthreads();
+  for (int t = threadIdx.x; t < total; t += kCellThreads) {
+    const uint32_t b = (uint32_t)(a[t] - lo);
+    atomicOr(bits + (b >> 5), 1u << (b & 31));
+  }
+  __syncthreads();
+  const int per = (words + kCellThreads - 1) / kCellThreads;
+  const int w0 = min(words, (int)threadIdx.x * per), w1 = min(words, w0 + per);
+  int mine = 0;
+  for (int w = w0; w < w1; ++w)
+    mine += __popc(bits[w]);
+  int incl = mine;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o)
+      incl += y;
+  }
+  if (lane == 31)
+    s_warp[warp] = incl;
+  __syncthreads();
+  int pos = incl - mine;
+  for (int k = 0; k < warp; ++k)
+    pos += s_warp[k];
+  for (int w = w0; w < w1; ++w)
+    for (uint32_t m = bits[w]; m; m &= m - 1)
+      a[pos++] = lo + 32 * w + (__ffs(m) - 1);
+  __syncthreads();
+}
+
+__device__ __forceinline__ float warp_min(float v) {
+  float r;
+  asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+  return r;
+}
+__device__ __forceinline__ float warp_max(float v) {
+  float r;
+  asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+  return r;
+}
+
 struct CellSearch {
   double inv_width, dist2_max;
   float r2lo, r2hi;  // (radius / cell width)^2 less and plus the margin
@@ -427,9 +479,10 @@ __global__ void __launch_bounds__(kCellThreads) k_nb_cell(const double4 *xv, Gri
   extern __shared__ __align__(16) unsigned char s_cell[];
   float4 *cand = reinterpret_cast<float4 *>(s_cell);  // position relative to the cell's first point, index
   int32_t *index = reinterpret_cast<int32_t *>(cand + width);
-  float *box = reinterpret_cast<float *>(index + width);  // per 32 candidates: lowest x, y, z, highest x, y, z
+  int32_t *own = index + width;                             // the cell's points, in ascending order
+  float *box = reinterpret_cast<float *>(own + width);      // per 32 candidates: lowest x, y, z, highest x, y, z
   __shared__ int64_t s_begin[9];
-  __shared__ int s_off[10];
+  __shared__ int s_off[10], s_lo, s_hi;
   const int64_t c = blockIdx.x, first = cell_start[c], last = cell_start[c + 1];
   if (first == last)
     return;
@@ -458,9 +511,33 @@ __global__ void __launch_bounds__(kCellThreads) k_nb_cell(const double4 *xv, Gri
       index[t] = sorted[s_begin[k] + (t - s_off[k])];
   for (int t = total + threadIdx.x; t < w2; t += kCellThreads)
     index[t] = INT_MAX;
+  int o2 = 32;
+  while (o2 < (int)(last - first))
+    o2 <<= 1;
+  for (int t = threadIdx.x; t < o2; t += kCellThreads)
+    own[t] = t < last - first ? sorted[first + t] : INT_MAX;
+  if (threadIdx.x == 0)
+    s_lo = INT_MAX, s_hi = 0;
   __syncthreads();
-  block_sort(index, w2);
+  int lo = INT_MAX, hi = 0;
+  for (int t = threadIdx.x; t < total; t += kCellThreads)
+    lo = min(lo, index[t]), hi = max(hi, index[t]);
+  lo = __reduce_min_sync(0xffffffffu, lo), hi = __reduce_max_sync(0xffffffffu, hi);
+  if (lane == 0)
+    atomicMin(&s_lo, lo), atomicMax(&s_hi, hi);
+  __syncthreads();
+  const int words = (s_hi - s_lo) / 32 + 1;
+  const int points = (int)(last - first);
+  if (words <= 4 * width) {  // the candidates' positions are not there yet: 16 bytes each
+    block_sort_bits(index, total, s_lo, reinterpret_cast<uint32_t *>(cand), words);
+    block_sort_bits(own, points, s_lo, reinterpret_cast<uint32_t *>(cand), words);
+  } else {
+    block_sort(index, w2);
+    block_sort(own, o2);
+  }
   const double4 ref = xv[sorted[first]];
+  for (int t = total + threadIdx.x; t < min(width, (total + 31) & ~31); t += kCellThreads)
+    cand[t] = make_float4(1.0e18f, 1.0e18f, 1.0e18f, __int_as_float(-1));
   for (int t = threadIdx.x; t < total; t += kCellThreads) {
     const double4 p = xv[index[t]];
     cand[t] = make_float4((float)((p.x - ref.x) * cs.inv_width), (float)((p.y - ref.y) * cs.inv_width),
@@ -470,59 +547,77 @@ __global__ void __launch_bounds__(kCellThreads) k_nb_cell(const double4 *xv, Gri
   const int chunks = (total + 31) / 32;
   for (int k = warp; k < chunks; k += kCellThreads / 32) {
     const float4 p = cand[min(32 * k + lane, total - 1)];
-    float lo[3] = {p.x, p.y, p.z}, hi[3] = {p.x, p.y, p.z};
-#pragma unroll
-    for (int d = 0; d < 3; ++d)
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        lo[d] = fminf(lo[d], __shfl_xor_sync(0xffffffffu, lo[d], o));
-        hi[d] = fmaxf(hi[d], __shfl_xor_sync(0xffffffffu, hi[d], o));
-      }
+    const float lo[3] = {warp_min(p.x), warp_min(p.y), warp_min(p.z)};
+    const float hi[3] = {warp_max(p.x), warp_max(p.y), warp_max(p.z)};
     if (lane < 6)
       box[6 * k + lane] = lane == 0 ? lo[0] : lane == 1 ? lo[1] : lane == 2 ? lo[2] : lane == 3 ? hi[0] : lane == 4 ? hi[1] : hi[2];
   }
   __syncthreads();
+  // two points of the cell at a time, consecutive in index, over the chunks near either: one read of a candidate
+  // and packed FP32 arithmetic for both
   const unsigned lt = (1u << lane) - 1u;
   int most = 0;
-  for (int64_t q = first + warp; q < last; q += kCellThreads / 32) {
-    const int32_t i = sorted[q];
-    const double4 pi = xv[i];
-    const float x = (float)((pi.x - ref.x) * cs.inv_width), y = (float)((pi.y - ref.y) * cs.inv_width),
-                z = (float)((pi.z - ref.z) * cs.inv_width);
-    int32_t *row = FILL ? col + row_ptr[i] : nullptr;
-    int cnt = 0;
+  for (int q = 2 * warp; q < points; q += 2 * (kCellThreads / 32)) {
+    int32_t i[2];
+    float x[2], y[2], z[2];
+    int32_t *row[2];
+    int cnt[2] = {0, 0};
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      i[h] = own[min(q + h, points - 1)];
+      const double4 pi = xv[i[h]];
+      x[h] = (float)((pi.x - ref.x) * cs.inv_width), y[h] = (float)((pi.y - ref.y) * cs.inv_width);
+      z[h] = (float)((pi.z - ref.z) * cs.inv_width);
+      row[h] = FILL ? col + row_ptr[i[h]] : nullptr;
+    }
+    const float2 nx = make_float2(-x[0], -x[1]), ny = make_float2(-y[0], -y[1]), nz = make_float2(-z[0], -z[1]);
     for (int k0 = 0; k0 < chunks; k0 += 32) {
       bool near = false;
       if (k0 + lane < chunks) {
         const float *b = box + 6 * (k0 + lane);
-        const float dx = fmaxf(fmaxf(b[0] - x, x - b[3]), 0.0f), dy = fmaxf(fmaxf(b[1] - y, y - b[4]), 0.0f),
-                    dz = fmaxf(fmaxf(b[2] - z, z - b[5]), 0.0f);
-        near = dx * dx + dy * dy + dz * dz <= cs.r2hi;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const float dx = fmaxf(fmaxf(b[0] - x[h], x[h] - b[3]), 0.0f), dy = fmaxf(fmaxf(b[1] - y[h], y[h] - b[4]), 0.0f),
+                      dz = fmaxf(fmaxf(b[2] - z[h], z[h] - b[5]), 0.0f);
+          near = near || dx * dx + dy * dy + dz * dz <= cs.r2hi;
+        }
       }
       for (unsigned m = __ballot_sync(0xffffffffu, near); m; m &= m - 1) {
         const int t = 32 * (k0 + __ffs(m) - 1) + lane;
-        bool keep = false;
-        int32_t j = 0;
-        if (t < total) {
-          const float4 p = cand[t];
-          j = __float_as_int(p.w);
-          const float dx = p.x - x, dy = p.y - y, dz = p.z - z, s = dx * dx + dy * dy + dz * dz;
-          keep = s < cs.r2lo;
-          if (!keep && s <= cs.r2hi)
-            keep = within(xv[j], pi, cs.dist2_max);
-          keep = keep && j != i;
+        const float4 p = cand[t];  // (past the last candidate: one far away)
+        const int32_t j = __float_as_int(p.w);
+        const float2 dx = __fadd2_rn(bcast2(p.x), nx), dy = __fadd2_rn(bcast2(p.y), ny), dz = __fadd2_rn(bcast2(p.z), nz);
+        const float2 s = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __fmul2_rn(dx, dx)));
+        bool keep[2] = {s.x < cs.r2lo, s.y < cs.r2lo};
+        const bool near0 = !keep[0] && s.x <= cs.r2hi, near1 = !keep[1] && s.y <= cs.r2hi;
+        if (__any_sync(0xffffffffu, near0 || near1)) {  // rare: out of line, by a uniform branch
+          if (near0)
+            keep[0] = within_exact(xv, j, i[0], cs.dist2_max);
+          if (near1)
+            keep[1] = within_exact(xv, j, i[1], cs.dist2_max);
         }
-        const unsigned hit = __ballot_sync(0xffffffffu, keep);
-        if (FILL && keep)
-          row[cnt + __popc(hit & lt)] = j;
-        cnt += __popc(hit);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const bool k = keep[h] && j != i[h];
+          if (FILL) {
+            const unsigned hit = __ballot_sync(0xffffffffu, k);
+            if (k && q + h < points)
+              row[h][cnt[h] + __popc(hit & lt)] = j;
+            cnt[h] += __popc(hit);
+          } else {
+            cnt[h] += k;
+          }
+        }
       }
     }
-    if (!FILL) {
-      if (lane == 0)
-        len[i] = cnt;
-      most = max(most, cnt);
-    }
+    if (!FILL)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int total_h = __reduce_add_sync(0xffffffffu, cnt[h]);
+        if (lane == 0)
+          len[i[h]] = total_h;
+        most = max(most, total_h);
+      }
   }
   if (!FILL && lane == 0 && most > 0)
     atomicMax(longest, (unsigned long long)most);
@@ -536,7 +631,7 @@ static int cell_width(int candidates) {
   return w;
 }
 static size_t cell_smem(int width) {
-  return (size_t)width * (sizeof(float4) + sizeof(int32_t)) + (size_t)(width / 32) * 6 * sizeof(float);
+  return (size_t)width * (sizeof(float4) + 2 * sizeof(int32_t)) + (size_t)(width / 32) * 6 * sizeof(float);
 }
 
 template <bool FILL>
@@ -549,7 +644,7 @@ static int launch_cells(const double4 *xv, const NeighborGrid &grid, const Neigh
   const size_t smem = cell_smem(width);
   VPD_CUDA(cudaFuncSetAttribute(k_nb_cell<FILL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   k_nb_cell<FILL><<<(unsigned)grid.ncells, kCellThreads, smem, s>>>(xv, g, scr.cell_start, scr.sorted, cs, width, row_ptr,
-                                                                    col, scr.len, scr.reduce + 8);
+                                                                    col, scr.len, scr.reduce);
   VPD_CUDA(cudaGetLastError());
   return VPD_OK;
 }
@@ -599,16 +694,19 @@ int neighbor_count(const double4 *xv, int64_t n, double horizon, int64_t *row_pt
   unsigned long long init[kReduceWords] = {0, 0,
                                            (unsigned long long)LLONG_MAX, (unsigned long long)LLONG_MAX,
                                            (unsigned long long)LLONG_MAX, (unsigned long long)LLONG_MIN,
-                                           (unsigned long long)LLONG_MIN, (unsigned long long)LLONG_MIN, 0, 0};
+                                           (unsigned long long)LLONG_MIN, (unsigned long long)LLONG_MIN, 0};
   VPD_CUDA(cudaMemcpyAsync(scr.reduce, init, sizeof init, cudaMemcpyHostToDevice, s));
-  k_abs_max<<<grid_for(n, 256), 256, 0, s>>>(xv, n, scr.reduce);
+  k_bounds<<<grid_for(n, 256), 256, 0, s>>>(xv, n, scr.reduce);
   unsigned long long red[kReduceWords];
   VPD_CUDA(cudaMemcpyAsync(red, scr.reduce, sizeof red, cudaMemcpyDeviceToHost, s));
   VPD_CUDA(cudaStreamSynchronize(s));
   if (red[1])
     return set_error(VPD_ERR_NONFINITE, "Nonfinite PD coordinate.");
-  double maxabs;
-  memcpy(&maxabs, &red[0], sizeof maxabs);
+  double low[3], high[3], maxabs = 0.0;
+  for (int d = 0; d < 3; ++d) {
+    low[d] = key_value(red[2 + d]), high[d] = key_value(red[5 + d]);
+    maxabs = std::max(maxabs, std::max(std::fabs(low[d]), std::fabs(high[d])));
+  }
   const double scale = std::max(horizon, maxabs);
   grid.tolerance = 64.0 * DBL_EPSILON * scale;
   grid.radius = horizon + grid.tolerance;
@@ -620,17 +718,11 @@ int neighbor_count(const double4 *xv, int64_t n, double horizon, int64_t *row_pt
     s2 = std::nextafter(s2, 0.0);
   grid.dist2_max = s2;
 
-  k_cell_coords<<<grid_for(n, 256), 256, 0, s>>>(xv, n, grid.cell_width, scr.cell_coords,
-                                                 (long long *)scr.reduce);
-  VPD_CUDA(cudaMemcpyAsync(red, scr.reduce, sizeof red, cudaMemcpyDeviceToHost, s));
-  VPD_CUDA(cudaStreamSynchronize(s));
-  long long lo[3], hi[3];
-  memcpy(lo, &red[2], sizeof lo);
-  memcpy(hi, &red[5], sizeof hi);
+  // the cells of the extreme coordinates bound all cells (cell_coord does not decrease with x)
   double cells = 1.0;
   for (int d = 0; d < 3; ++d) {
-    grid.lo[d] = lo[d];
-    grid.dims[d] = hi[d] - lo[d] + 1;
+    grid.lo[d] = (long long)std::floor(low[d] / grid.cell_width);
+    grid.dims[d] = (long long)std::floor(high[d] / grid.cell_width) - grid.lo[d] + 1;
     cells *= (double)grid.dims[d];
   }
   if (cells > (double)kMaxCells)
@@ -645,7 +737,7 @@ int neighbor_count(const double4 *xv, int64_t n, double horizon, int64_t *row_pt
   const GridDev g{grid.lo[0], grid.lo[1], grid.lo[2], grid.dims[0], grid.dims[1], grid.dims[2]};
   VPD_CUDA(cudaMemsetAsync(scr.cell_count, 0, sizeof(int32_t) * (size_t)(grid.ncells + 1), s));
   const unsigned pb = (unsigned)((n + 255) / 256);
-  k_cell_assign<<<pb, 256, 0, s>>>(scr.cell_coords, n, g, scr.cell_of, scr.cell_count);
+  k_cell_assign<<<pb, 256, 0, s>>>(xv, n, grid.cell_width, g, scr.cell_coords, scr.cell_of, scr.cell_count);
   int rc = scan_exclusive_i32(scr.cell_count, grid.ncells, scr.cell_start, scr.scan_tmp, s);
   if (rc)
     return rc;
@@ -656,11 +748,11 @@ int neighbor_count(const double4 *xv, int64_t n, double horizon, int64_t *row_pt
   grid.candidates = 0;
   if (grid.ncells * kMinCellPoints <= n && grid.cell_width > 1.0e-100 && grid.cell_width < 1.0e100) {
     k_cell_candidates<<<(unsigned)((grid.ncells + 255) / 256), 256, 0, s>>>(grid.ncells, g, scr.cell_start,
-                                                                           scr.reduce + 9);
+                                                                           scr.reduce + 8);
     VPD_CUDA(cudaMemcpyAsync(red, scr.reduce, sizeof red, cudaMemcpyDeviceToHost, s));
     VPD_CUDA(cudaStreamSynchronize(s));
-    if (red[9] <= (unsigned long long)kMaxCandidates)
-      grid.candidates = (int)red[9];
+    if (red[8] <= (unsigned long long)kMaxCandidates)
+      grid.candidates = (int)red[8];
   }
   if (grid.candidates) {
     if ((rc = launch_cells<false>(xv, grid, scr, nullptr, nullptr, s)))
@@ -684,7 +776,7 @@ int neighbor_count(const double4 *xv, int64_t n, double horizon, int64_t *row_pt
   workspace_free(own, s);
   if (rc)
     return rc;
-  grid.max_len = (int)red[8];
+  grid.max_len = (int)red[0];
   if (grid.max_len > kMaxRow)
     return set_error(VPD_ERR_CAPACITY, "a point has more than 8192 neighbours");
   return VPD_OK;
