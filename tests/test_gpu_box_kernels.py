@@ -30,3 +30,23 @@ def test_box_kernels_match_slot_kernels_bitwise(monkeypatch, dims, ratio, damage
     for kind in ("box", "tiles", ""):
         for f, want in out["slot"].items():
             assert np.array_equal(out[kind][f], want), (kind, f)
+
+
+# the tile shapes of larger lattices: one point per thread in both kernels (20k points), two and three in small blocks
+# (98k), three in the deformation too, one wave of it (155k), two again (210k)
+@pytest.mark.parametrize("dims", [(33, 25, 24), (61, 41, 40), (80, 45, 43), (103, 46, 45)])
+@pytest.mark.parametrize("damage", [0, 1])
+def test_tile_shapes_match_slot_kernels_bitwise(monkeypatch, dims, damage):
+    nx, ny, nz = dims
+    case = tensile_bar(3, nx=nx, ny=ny, nz=nz, horizon=0.3015, damage_mode=damage, damage_initiation=0.002,
+                       precision=PRECISION_FP64)
+    out = {}
+    for kind in ("slot", "tiles"):
+        monkeypatch.setenv("VPD_BOND_KERNEL", kind)
+        with vpd.Simulation(case) as sim:
+            rows = sim.step(60)
+            out[kind] = {f: sim.field(f) for f in FIELDS} | {"rows": rows}
+    for f, want in out["slot"].items():
+        assert np.array_equal(out["tiles"][f], want), f
+    if damage:
+        assert out["slot"]["damage_index"].max() > 0

@@ -161,6 +161,11 @@ template <int kTileP> static unsigned tiled_grid(const StepParams &p) {
   return (unsigned)((threads + kBondThreads - 1) / kBondThreads);
 }
 
+template <int kTileP, int kThreads> static unsigned tiled_blocks(const StepParams &p) {
+  const int64_t threads = (int64_t)p.lat_nx * ((p.lat_ny + kTileP - 1) / kTileP) * p.lat_nz;
+  return (unsigned)((threads + kThreads - 1) / kThreads);
+}
+
 // 32-bit window indices need every index within a stencil reach of the lattice below 2^31
 static inline bool index32(const StepParams &p) { return p.n < (int64_t(1) << 30); }
 

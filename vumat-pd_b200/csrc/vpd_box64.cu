@@ -16,8 +16,9 @@
 // extent along z modulo 8, so that the consecutive points of a warp fall into different banks. Their
 // length is a template parameter (at least the region's), so that one address serves every array.
 //
-// Measured on a B200, per increment with the material and integration kernels (28 us): 40x10x10 bar at
-// horizon 3.015 h 92 to 43 us, the archived 101x21x5 lattice at 3 h 113 to 57 us. Both kernels are
+// Measured on a B200, per increment with the material and integration kernels (28 us), against two points per
+// thread in 256-thread blocks: 40x10x10 bar at horizon 3.015 h 92 to 43 us, the archived 101x21x5 lattice at 3 h
+// 113 to 57 us. Both kernels are
 // still bound by latency: about 3 us to stage the region and 4 us for the 122 slots at one warp
 // per scheduler.
 //
@@ -275,7 +276,7 @@ constexpr int kBoxMaxRecords = 2304;
 // (more points per staged region where several blocks would queue per SM anyway).
 int setup_box64(StepParams &p) {
   p.box = BoxTiles{};
-  const int points = p.n <= 148 * 32 ? 32 : (p.n <= 148 * 64 ? 64 : 128);
+  const int points = p.n <= 148 * 32 ? 32 : (p.n <= 148 * 48 ? 64 : 128);
   double best = 0.0;
   for (int tx = 1; tx <= points; ++tx)
     for (int ty = 1; tx * ty <= points; ++ty)

@@ -186,12 +186,12 @@ int launch_force_tiled(const StepParams &p, cudaStream_t s);
 int launch_deformation_tiled64(const StepParams &p, cudaStream_t s);
 int launch_force_tiled64(const StepParams &p, cudaStream_t s);
 // FP64 bond kernels of small lattices (vpd_box64.cu): setup fills p.box (threads stays 0 when no
-// box's neighbourhood fits shared memory). Default up to kBoxPoints points: beyond, the tiled kernels
-// have enough blocks. Per increment in microseconds, tiled against boxes, at horizons 3.015 h | 4.015 h:
-// 4,000 points 92/43 | 158/62, 10,605 112/57 | 204/91, 20,400 99/95 | 174/154 (168 with 128-point boxes),
-// 27,000 99/98 | 166/167, 54,000 100/138 | 171/241. With bond damage the boxes' stretch tests cost less
-// than the tiles': 4,000 points 117/49 | 208/70, 27,000 128/107 | 223/189, 54,000 126/156 | 224/275.
-constexpr int64_t kBoxPoints = 20000, kBoxPointsDamage = 32000;
+// box's neighbourhood fits shared memory). Default up to kBoxPoints points: beyond, single points per
+// thread (vpd_tiled64.cu) fill the GPU as well. Per increment in microseconds, boxes | tiles, at horizons
+// 3.015 h and 4.015 h: 1,600 points 40 | 57 and 58 | 86, 4,000 43 | 59 and 62 | 89, 10,605 58 | 59 and 91 | 90,
+// 20,400 95 | 63 and 168 | 100. With bond damage the boxes' stretch tests cost less than the tiles':
+// 10,605 63 | 73 and 101 | 119, 16,800 67 | 74 and 106 | 122, 20,400 102 | 77 and 188 | 129.
+constexpr int64_t kBoxPoints = 11000, kBoxPointsDamage = 17500;
 int setup_box64(StepParams &p);
 int launch_deformation_box64(const StepParams &p, cudaStream_t s);
 int launch_force_box64(const StepParams &p, cudaStream_t s);
