@@ -1,10 +1,10 @@
-"""The FP64 bond kernels of small lattices (vpd_box64.cu) against the per-slot kernels, bit for bit:
+"""The bond kernels' shapes by lattice size against one another, bit for bit. FP64 against the per-slot kernels:
 both sum every point's bonds in slot order with the same operations."""
 import numpy as np
 import pytest
 
 import vpd
-from vpd.case import PRECISION_FP64, tensile_bar
+from vpd.case import PRECISION_FP64, PRECISION_MIXED, tensile_bar
 
 pytestmark = pytest.mark.gpu
 
@@ -50,3 +50,23 @@ def test_tile_shapes_match_slot_kernels_bitwise(monkeypatch, dims, damage):
         assert np.array_equal(out["tiles"][f], want), f
     if damage:
         assert out["slot"]["damage_index"].max() > 0
+
+
+# a warp per stencil plane (seven, nine and eleven planes; a lattice thinner than the stencil; ragged columns) and a
+# thread per tile against each other in mixed precision: the plane partials are folded in the same order
+@pytest.mark.parametrize("dims,ratio", [((8, 3, 5), 4.0), ((13, 5, 7), 3.015), ((24, 21, 17), 4.015), ((19, 12, 13), 5.015),
+                                        ((41, 10, 11), 3.0)])
+@pytest.mark.parametrize("damage", [0, 1])
+def test_plane_split_mixed_kernels_match_bitwise(monkeypatch, dims, ratio, damage):
+    nx, ny, nz = dims
+    case = tensile_bar(3, nx=nx, ny=ny, nz=nz, horizon=ratio * 0.1, damage_mode=damage, damage_initiation=0.004,
+                       precision=PRECISION_MIXED)
+    out = {}
+    for kind in ("pair", "planes", ""):
+        monkeypatch.setenv("VPD_BOND_KERNEL", kind)
+        with vpd.Simulation(case) as sim:
+            rows = sim.step(150)
+            out[kind] = {f: sim.field(f) for f in FIELDS} | {"rows": rows}
+    for kind in ("planes", ""):
+        for f, want in out["pair"].items():
+            assert np.array_equal(out[kind][f], want), (kind, f)

@@ -478,14 +478,22 @@ int create_impl(vpd_handle *h, const vpd_case *c, const double *positions, const
   p.st = h->st;
   p.lat_nx = c->nx, p.lat_ny = c->ny, p.lat_nz = c->nz, p.lat_h = c->spacing;
   {
-    // VPD_BOND_KERNEL=slot selects the per-slot bond kernels (both precisions), scalar the
-    // two-point tiled mixed kernels in scalar FP32, tiled2 the two-point FP64 force kernel,
-    // staged the TMA-staged FP64 force kernel, tiles the tiled FP64 kernels at any size, box the
-    // small-lattice FP64 kernels at any size (default: boxes on small lattices, kBoxPoints, else tiled;
-    // packed pairs when mixed)
+    // VPD_BOND_KERNEL=slot selects the per-slot bond kernels (both precisions). Mixed: scalar the two-point
+    // tiled kernels in scalar FP32, planes or pair the packed pairs with or without a warp per stencil
+    // plane at any size (default: by size). FP64: tiled2 the two-point force kernel, staged the TMA-staged one,
+    // tiles or box the tiled kernels or the small-lattice boxes at any size (default: boxes on small
+    // lattices, else tiled).
     const char *bk = getenv("VPD_BOND_KERNEL");
     const std::string kind = bk ? bk : "";
-    p.tiled = kind == "slot" ? 0 : kind == "scalar" ? 1 : kind == "tiled2" ? 3 : kind == "staged" ? 6 : kind == "tiles" ? 4 : kind == "box" ? 7 : 2;
+    p.tiled = kind == "slot"     ? 0
+              : kind == "scalar" ? 1
+              : kind == "tiled2" ? 3
+              : kind == "tiles"  ? 4
+              : kind == "planes" ? 5
+              : kind == "staged" ? 6
+              : kind == "box"    ? 7
+              : kind == "pair"   ? 8
+                                 : 2;
     // VPD_RETURN_MAP=bisection: the material kernel evaluates every bisection iteration (the
     // default decides most of them from two anchor evaluations; the results are the same)
     const char *rm = getenv("VPD_RETURN_MAP");

@@ -156,11 +156,6 @@ __device__ __forceinline__ void commit_breaks(const StepParams &p, int64_t i, in
   }
 }
 
-template <int kTileP> static unsigned tiled_grid(const StepParams &p) {
-  const int64_t threads = (int64_t)p.lat_nx * ((p.lat_ny + kTileP - 1) / kTileP) * p.lat_nz;
-  return (unsigned)((threads + kBondThreads - 1) / kBondThreads);
-}
-
 template <int kTileP, int kThreads> static unsigned tiled_blocks(const StepParams &p) {
   const int64_t threads = (int64_t)p.lat_nx * ((p.lat_ny + kTileP - 1) / kTileP) * p.lat_nz;
   return (unsigned)((threads + kThreads - 1) / kThreads);

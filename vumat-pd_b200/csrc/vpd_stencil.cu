@@ -206,6 +206,15 @@ int build_stencil(const int64_t *row_ptr, const int32_t *col, int64_t n, int ny,
   st.slots = S;
   st.nw = nw;
   st.ngroups = (int)groups.size();
+  for (int g = 0; g < st.ngroups; ++g)
+    if (g == 0 || groups[g].x != groups[g - 1].x) {
+      if (st.nplanes == kMaxPlanes) {
+        st.nplanes = 0;
+        break;
+      }
+      st.plane[st.nplanes++] = g;
+    }
+  st.plane[st.nplanes] = st.ngroups;
   // a two-point tile's window reaches y in [-ry, ny + ry], x and z within the extent
   st.halo = (int64_t)ex.rx * ny * nz + (int64_t)(ex.ry + 2) * nz + ex.rz + 1;
   st.rx = ex.rx, st.ry = ex.ry, st.rz = ex.rz;

@@ -33,6 +33,8 @@ constexpr int kMaxStencilWords = 32; // at most 1024 lattice offsets per stencil
 constexpr int kMaxGroupSlots = 29;
 constexpr size_t kStagedMaxBytes = 110 * 1024;  // its box, so that two blocks fit an SM
 
+constexpr int kMaxPlanes = 16;  // planes of a stencil that the plane-split mixed kernels take, one warp each
+
 // Tiles of the TMA-staged FP64 force kernel (vpd_staged64.cu); bytes == 0: not in use.
 struct StagedTiles {
   int p = 2;                           // points per thread along y (2 or 4)
@@ -64,6 +66,8 @@ struct StencilLayout {
   float4 *e0 = nullptr;        // [32 nw] lattice offset of each slot times h (mixed precision)
   int64_t halo = 0;            // points a tile's window can reach beyond either end of the lattice
   int rx = 0, ry = 0, rz = 0;  // the largest |offset| along x, y, z
+  int nplanes = 0;             // stencil planes (runs of groups with one x offset), 0: more than kMaxPlanes
+  int plane[kMaxPlanes + 1] = {};  // their first groups, then ngroups
 };
 
 struct StepParams {
@@ -78,9 +82,9 @@ struct StepParams {
   StencilLayout st;           // lattice-stencil layout; used instead of the ELL when st.nw > 0
   int lat_nx, lat_ny, lat_nz; // the lattice (points in index order (x ny + y) nz + z)
   double lat_h;               // lattice spacing
-  int tiled;                  // bond kernels: 0 per slot; mixed 1 tiled scalar, else packed pairs; FP64
-                              // tiled with the 4-point force, 3 with the 2-point force, 6 with the
-                              // TMA-staged force, 4 never the small-lattice boxes, 7 always
+  int tiled;                  // bond kernels (VPD_BOND_KERNEL): 0 per slot, 2 by precision and size; mixed 1 tiled
+                              // scalar, 5 / 8 packed pairs with / without a warp per plane; FP64 3 with the
+                              // 2-point force, 4 tiles, 6 with the TMA-staged force, 7 boxes
   int literal_bisection;      // 1: k_material runs the VUMAT's bisection literally (every iteration
                               // evaluated), 0: jc_return_map (same results)
   // kinematic state

@@ -23,6 +23,8 @@
 // kernel: for every bond not clearly intact), pairs broken once by the lower-index point.
 #include "vpd_bond.cuh"
 
+#include <type_traits>
+
 namespace vpd {
 
 template <bool B> struct BoolConstant {
@@ -446,8 +448,8 @@ __device__ __forceinline__ void deform_pair_window(const StepParams &p, int cnt,
   }
 }
 
-template <bool DAMAGE, bool UNROLL>
-__global__ void __launch_bounds__(kBondThreads, 2) k_deformation_pair(const __grid_constant__ StepParams p) {
+template <bool DAMAGE, bool UNROLL, int TPB, int MINB>
+__global__ void __launch_bounds__(TPB, MINB) k_deformation_pair(const __grid_constant__ StepParams p) {
   const int64_t n = p.n;
   const int ny = p.lat_ny, nz = p.lat_nz;
   const float h = (float)p.lat_h;
@@ -557,12 +559,151 @@ __global__ void __launch_bounds__(kBondThreads, 2) k_deformation_pair(const __gr
   }
 }
 
+// The thread's two points (lanes of the pairs) and their lattice column.
+struct PairTile {
+  int x, yb, z;
+  int64_t ip[2];
+  bool vp[2];
+};
+__device__ __forceinline__ PairTile pair_tile(const StepParams &p, int64_t tau) {
+  PairTile t;
+  const bool inb = tile_coords<2>(p, tau, t.x, t.yb, t.z);
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    const int y = t.yb * 2 + q;
+    t.vp[q] = inb && y < p.lat_ny;
+    t.ip[q] = t.vp[q] ? ((int64_t)t.x * p.lat_ny + y) * p.lat_nz + t.z : 0;
+  }
+  return t;
+}
+__device__ __forceinline__ DeformPair deform_pair(const StepParams &p, const PairTile &t, float h) {
+  float4 pa[2], pb[2];
+#pragma unroll
+  for (int q = 0; q < 2; ++q)
+    pa[q] = ldgf4(p.jit + t.ip[q]), pb[q] = ldgf4(p.uf + t.ip[q]);
+  DeformPair pt;
+  pt.jx = make_float2(pa[0].x, pa[1].x), pt.jy = make_float2(pa[0].y, pa[1].y + h);
+  pt.jz = make_float2(pa[0].z, pa[1].z);
+  pt.ux = make_float2(pb[0].x, pb[1].x), pt.uy = make_float2(pb[0].y, pb[1].y);
+  pt.uz = make_float2(pb[0].z, pb[1].z);
+  return pt;
+}
+
+// The windows of one plane's groups [g0, g1) summed into `part`: the loop of k_deformation_pair without its folds. (Not
+// shared with it: called from there, the kernel with damage came out 5 % slower, 615 against 590 us at 1M points.)
+template <bool DAMAGE, bool UNROLL>
+__device__ __forceinline__ void deform_pair_groups(const StepParams &p, int g0, int g1, const PairTile &tile, float h,
+                                                   const DeformPair &pt, float2 (&part)[9]) {
+  const int64_t n = p.n;
+  const int ny = p.lat_ny, nz = p.lat_nz, x = tile.x, yb = tile.yb, z = tile.z;
+  const int64_t(&ip)[2] = tile.ip;
+  const bool(&vp)[2] = tile.vp;
+  int word = -1;  // the mask word held in mw (groups come in slot order: several per word)
+  // mw: the mask words; bw: the broken-bond words, read with them (only this thread sets the
+  // bits of its points' forward slots, the only ones tested, and each slot is in one group)
+  uint32_t mw[2] = {0u, 0u}, bw[2] = {0u, 0u};
+  for (int g = g0; g < g1; ++g) {
+    const int4 gr = __ldg(p.st.groups + g);  // dx, dz, lowest dy, (slots << 16) | first slot
+    const int cnt = gr.w >> 16, pos = gr.w & 0xffff, wd = pos >> 5, sh = pos & 31;
+    const uint32_t cm = cnt >= 32 ? ~0u : ((1u << cnt) - 1u);
+    if (wd != word) {  // uniform: the group table is the same for every thread
+      word = wd;
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        mw[q] = vp[q] ? __ldg(p.st.mask + (int64_t)wd * n + ip[q]) : 0u;
+        if (DAMAGE)
+          bw[q] = vp[q] ? p.st.broken[(int64_t)wd * n + ip[q]] : 0u;
+      }
+    }
+    uint32_t bits[2], live[2];
+    const uint32_t fw = DAMAGE ? group_bits(__ldg(p.st.forward + wd), sh, cm) : 0u;
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const uint32_t m = group_bits(mw[q], sh, cm);
+      bits[q] = m << q;  // bit t: the neighbour at window position t (slot pos + t - q)
+      live[q] = DAMAGE ? (m & fw & ~group_bits(bw[q], sh, cm)) << q : 0u;
+    }
+    if (__all_sync(0xffffffffu, (bits[0] | bits[1]) == 0u))
+      continue;
+    const float gx = (float)gr.x * h, gz = (float)gr.y * h, by0 = (float)gr.z * h;
+    const GroupOffsets o{sub2(bcast2(gx), pt.jx), sub2(bcast2(by0), pt.jy), sub2(bcast2(gz), pt.jz)};
+    const int64_t jb = ((int64_t)(x + gr.x) * ny + (yb * 2 + gr.z)) * nz + (z + gr.y);
+    uint32_t fresh[2] = {0u, 0u}, near[2] = {0u, 0u};
+    // windows with stretch tests only where some lane of the warp has a live bond in the group
+    // (with damage: the forward groups, less their broken bonds)
+    const bool tests = DAMAGE && __any_sync(0xffffffffu, (live[0] | live[1]) != 0u);
+    auto windows = [&](auto tested) {
+      constexpr bool D = decltype(tested)::value;
+      if (UNROLL) {
+        static_assert(kUnrolledSlots == 12, "the cases below list the unrolled slot counts");
+        const int jb32 = (int)jb, nz32 = nz, n32 = (int)n;
+#define VPD_DEFORM_CASE(C)                                                                                   \
+  case C:                                                                                                    \
+    deform_pair_window<C, D, int>(p, cnt, jb32, nz32, n32, o, h, pt, bits, live, part, fresh, near);         \
+    break;
+        switch (cnt) {
+          VPD_DEFORM_CASE(1) VPD_DEFORM_CASE(2) VPD_DEFORM_CASE(3) VPD_DEFORM_CASE(4)
+          VPD_DEFORM_CASE(5) VPD_DEFORM_CASE(6) VPD_DEFORM_CASE(7) VPD_DEFORM_CASE(8)
+          VPD_DEFORM_CASE(9) VPD_DEFORM_CASE(10) VPD_DEFORM_CASE(11) VPD_DEFORM_CASE(12)
+        default:
+          deform_pair_window<0, D, int>(p, cnt, jb32, nz32, n32, o, h, pt, bits, live, part, fresh, near);
+        }
+#undef VPD_DEFORM_CASE
+      } else {
+        deform_pair_window<0, D, int64_t>(p, cnt, jb, (int64_t)nz, n, o, h, pt, bits, live, part, fresh, near);
+      }
+    };
+    if (tests)
+      windows(BoolConstant<DAMAGE>{});
+    else
+      windows(BoolConstant<false>{});
+    if (DAMAGE)
+#pragma unroll
+      for (int q = 0; q < 2; ++q)
+        commit_breaks(p, ip[q], pos, wd, sh, fresh[q] >> q, near[q] >> q);
+  }
+}
+
+// The same sums with the stencil's planes dealt out to the warps of a block, for lattices that do not fill the GPU
+// with a thread per two points: warp w sums plane w of the block's 32 tiles, and the planes' partials are
+// folded in plane order from shared memory, so the bits are k_deformation_pair's. The stencil of a horizon of
+// three or four spacings has seven or nine planes, that many times the warps (4,000 points: 46 to 16 us a kernel).
+template <bool DAMAGE, bool UNROLL, int THREADS, int MINB>
+__global__ void __launch_bounds__(THREADS, MINB) k_deformation_planes(const __grid_constant__ StepParams p) {
+  extern __shared__ float2 s_part[];  // [nplanes][9][32]
+  const int64_t n = p.n;
+  const float h = (float)p.lat_h;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, planes = p.st.nplanes;
+  const PairTile tile = pair_tile(p, (int64_t)blockIdx.x * 32 + lane);
+  const DeformPair pt = deform_pair(p, tile, h);
+  float2 part[9];
+#pragma unroll
+  for (int c = 0; c < 9; ++c)
+    part[c] = make_float2(0.0f, 0.0f);
+  deform_pair_groups<DAMAGE, UNROLL>(p, p.st.plane[warp], p.st.plane[warp + 1], tile, h, pt, part);
+#pragma unroll
+  for (int c = 0; c < 9; ++c)
+    s_part[(warp * 9 + c) * 32 + lane] = part[c];
+  __syncthreads();
+  for (int c = warp; c < 9; c += planes) {
+    float2 G = make_float2(0.0f, 0.0f), Gc = G;
+    for (int w = 0; w < planes; ++w)
+      kahan_add2(G, Gc, s_part[(w * 9 + c) * 32 + lane]);
+    const float2 g = sub2(G, Gc);
+    if (tile.vp[0])
+      p.Gf[c * n + tile.ip[0]] = g.x;
+    if (tile.vp[1])
+      p.Gf[c * n + tile.ip[1]] = g.y;
+  }
+}
+
 // The packed force kernel pairs the rows of a neighbour's force map, not the thread's points:
 // a neighbour's records load as the pairs (VM_0c, VM_1c) and (R_0, R_1) (fmap_record), so rows 0
 // and 1 of a bond term are three paired multiply-adds with the point's reference offset on both
 // lanes, and row 2 is three scalar ones; no neighbour value is copied to both lanes of a pair.
 // Point q's offsets from the group's window position 0, o - J_q, on both lanes of a pair
 // (ey at window position t adds t h):
+constexpr int kForcePairThreads = 192;
 struct ForceOffsets {
   float2 ex[2], ey[2], ez[2];
 };
@@ -611,53 +752,24 @@ __device__ __forceinline__ void force_pair_window(const StepParams &p, int cnt, 
   }
 }
 
-// f = sum (V_j M_j) xi over intact bonds + M_i s_i with s_i = vxi_i - sum_{broken j} V_j xi.
-// Two blocks per SM (128 registers, no spills): 0.375 against 0.393 ms at three blocks (80
-// registers and spills) on the 1M-point bar in plastic flow.
-template <bool DAMAGE, bool UNROLL>
-__global__ void __launch_bounds__(kBondThreads, 2) k_force_pair(const __grid_constant__ StepParams p) {
+// The windows of the groups [g0, g1) summed into part01, part2; new_plane(x offset) before each group. any_broken:
+// some of the groups' bonds are broken.
+template <bool DAMAGE, bool UNROLL, typename NewPlane>
+__device__ __forceinline__ void force_pair_groups(const StepParams &p, int g0, int g1, const PairTile &tile, float h,
+                                                  const float (&jx)[2], const float (&jy)[2], const float (&jz)[2],
+                                                  float2 (&part01)[2], float (&part2)[2], bool &any_broken,
+                                                  NewPlane new_plane) {
   const int64_t n = p.n;
-  const int ny = p.lat_ny, nz = p.lat_nz;
-  const float h = (float)p.lat_h;
-  int x, yb, z;
-  const bool inb = tile_coords<2>(p, (int64_t)blockIdx.x * blockDim.x + threadIdx.x, x, yb, z);
-  const float4 *P0 = p.fmapf, *P1 = p.fmapf + n, *P2 = p.fmapf + 2 * n;
-  int64_t ip[2];
-  bool vp[2];
-  float jx[2], jy[2], jz[2];  // jy includes q h (y relative to the thread's first point)
-#pragma unroll
-  for (int q = 0; q < 2; ++q) {
-    const int y = yb * 2 + q;
-    vp[q] = inb && y < ny;
-    ip[q] = vp[q] ? ((int64_t)x * ny + y) * nz + z : 0;
-    const float4 a = ldgf4(p.jit + ip[q]);
-    jx[q] = a.x, jy[q] = a.y + (float)q * h, jz[q] = a.z;
-  }
-  // the windows of one stencil plane sum into part01/part2, folded into fs01/fs2 with Kahan
-  // compensation (fc01/fc2)
-  float2 fs01[2], fc01[2], part01[2];
-  float fs2[2], fc2[2], part2[2];
-  bool any_broken = false;  // broken bonds' corrections are rare: gathered after the sum
-#pragma unroll
-  for (int q = 0; q < 2; ++q) {
-    fs01[q] = fc01[q] = part01[q] = make_float2(0.0f, 0.0f);
-    fs2[q] = fc2[q] = part2[q] = 0.0f;
-  }
+  const int ny = p.lat_ny, nz = p.lat_nz, x = tile.x, yb = tile.yb, z = tile.z;
+  const int64_t(&ip)[2] = tile.ip;
+  const bool(&vp)[2] = tile.vp;
   int word = -1;  // the mask (and broken-bond) words held in mw (bw): several groups per word
-  int plane = INT_MIN;
   uint32_t mw[2] = {0u, 0u}, bw[2] = {0u, 0u};
-  for (int g = 0; g < p.st.ngroups; ++g) {
+  for (int g = g0; g < g1; ++g) {
     const int4 gr = __ldg(p.st.groups + g);
     const int cnt = gr.w >> 16, pos = gr.w & 0xffff, wd = pos >> 5, sh = pos & 31;
     const uint32_t cm = cnt >= 32 ? ~0u : ((1u << cnt) - 1u);
-    if (gr.x != plane) {  // uniform: a new plane
-      plane = gr.x;
-#pragma unroll
-      for (int q = 0; q < 2; ++q) {
-        kahan_add2(fs01[q], fc01[q], part01[q]), kahan_add(fs2[q], fc2[q], part2[q]);
-        part01[q] = make_float2(0.0f, 0.0f), part2[q] = 0.0f;
-      }
-    }
+    new_plane(gr.x);
     if (wd != word) {  // uniform: the group table is the same for every thread
       word = wd;
 #pragma unroll
@@ -705,53 +817,172 @@ __global__ void __launch_bounds__(kBondThreads, 2) k_force_pair(const __grid_con
       force_pair_window<0, int64_t>(p, cnt, jb, (int64_t)nz, n, h, o, bits, part01, part2);
     }
   }
+}
+
+// The thread's points' jitters (jy includes q h: y relative to the thread's first point).
+__device__ __forceinline__ void force_pair_points(const StepParams &p, const PairTile &t, float h, float (&jx)[2],
+                                                  float (&jy)[2], float (&jz)[2]) {
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    const float4 a = ldgf4(p.jit + t.ip[q]);
+    jx[q] = a.x, jy[q] = a.y + (float)q * h, jz[q] = a.z;
+  }
+}
+
+// Point i's force from its bond sum (rows 0, 1 and row 2) and M_i s_i, written out.
+__device__ __forceinline__ void force_pair_finish(const StepParams &p, int64_t i, float2 f01, float f2_,
+                                                  bool any_broken) {
+  const int64_t n = p.n;
+  const float4 *P0 = p.fmapf, *P1 = p.fmapf + n, *P2 = p.fmapf + 2 * n;
+  // s_i less the broken bonds' V_j xi, summed in slot order
+  double c0 = 0.0, c1 = 0.0, c2 = 0.0;
+  if (any_broken) {
+    const float4 ji = p.jit[i];
+    for (int w = 0; w < p.st.nw; ++w)
+      for (uint32_t f = p.st.mask[(int64_t)w * n + i] & p.st.broken[(int64_t)w * n + i]; f; f &= f - 1) {
+        const int sl = 32 * w + __ffs(f) - 1;
+        const float4 jj = p.jit[i + p.st.delta[sl]], o = p.st.e0[sl];
+        c0 += (double)(jj.w * (o.x + (jj.x - ji.x)));
+        c1 += (double)(jj.w * (o.y + (jj.y - ji.y)));
+        c2 += (double)(jj.w * (o.z + (jj.z - ji.z)));
+      }
+  }
+  float VM[9];
+  fmap_rows(P0[i], P1[i], P2[i], VM);
+  const double4 s = p.vxi[i];
+  const double s0 = s.x - c0, s1 = s.y - c1, s2 = s.z - c2;
+  const double rv = 1.0 / (double)p.jit[i].w;
+  const double f0 = (double)f01.x + (VM[0] * s0 + VM[1] * s1 + VM[2] * s2) * rv;
+  const double f1 = (double)f01.y + (VM[3] * s0 + VM[4] * s1 + VM[5] * s2) * rv;
+  const double f2 = (double)f2_ + (VM[6] * s0 + VM[7] * s1 + VM[8] * s2) * rv;
+  p.force[i] = make_double4(f0, f1, f2, 0.0);
+}
+
+// f = sum (V_j M_j) xi over intact bonds + M_i s_i with s_i = vxi_i - sum_{broken j} V_j xi.
+// Three blocks of 192 threads per SM (up to 112 registers, no spills): on the 1M-point bar 0.373 ms, as two blocks of
+// 256, against 0.393 at three blocks of those (80 registers and spills); 154,000 points fit one wave of it
+// (75 against 98 us).
+template <bool DAMAGE, bool UNROLL>
+__global__ void __launch_bounds__(kForcePairThreads, 3) k_force_pair(const __grid_constant__ StepParams p) {
+  const float h = (float)p.lat_h;
+  const PairTile tile = pair_tile(p, (int64_t)blockIdx.x * blockDim.x + threadIdx.x);
+  float jx[2], jy[2], jz[2];
+  force_pair_points(p, tile, h, jx, jy, jz);
+  // the windows of one stencil plane sum into part01/part2, folded into fs01/fs2 with Kahan
+  // compensation (fc01/fc2)
+  float2 fs01[2], fc01[2], part01[2];
+  float fs2[2], fc2[2], part2[2];
+  bool any_broken = false;  // broken bonds' corrections are rare: gathered after the sum
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    fs01[q] = fc01[q] = part01[q] = make_float2(0.0f, 0.0f);
+    fs2[q] = fc2[q] = part2[q] = 0.0f;
+  }
+  int plane = INT_MIN;
+  force_pair_groups<DAMAGE, UNROLL>(p, 0, p.st.ngroups, tile, h, jx, jy, jz, part01, part2, any_broken, [&](int gx) {
+    if (gx != plane) {  // uniform: a new plane
+      plane = gx;
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        kahan_add2(fs01[q], fc01[q], part01[q]), kahan_add(fs2[q], fc2[q], part2[q]);
+        part01[q] = make_float2(0.0f, 0.0f), part2[q] = 0.0f;
+      }
+    }
+  });
 #pragma unroll
   for (int q = 0; q < 2; ++q) {
     kahan_add2(fs01[q], fc01[q], part01[q]), kahan_add(fs2[q], fc2[q], part2[q]);
-    if (!vp[q])
-      continue;
-    const int64_t i = ip[q];
-    // s_i less the broken bonds' V_j xi, summed in slot order
-    double c0 = 0.0, c1 = 0.0, c2 = 0.0;
-    if (DAMAGE && any_broken) {
-      const float4 ji = p.jit[i];
-      for (int w = 0; w < p.st.nw; ++w)
-        for (uint32_t f = p.st.mask[(int64_t)w * n + i] & p.st.broken[(int64_t)w * n + i]; f; f &= f - 1) {
-          const int sl = 32 * w + __ffs(f) - 1;
-          const float4 jj = p.jit[i + p.st.delta[sl]], o = p.st.e0[sl];
-          c0 += (double)(jj.w * (o.x + (jj.x - ji.x)));
-          c1 += (double)(jj.w * (o.y + (jj.y - ji.y)));
-          c2 += (double)(jj.w * (o.z + (jj.z - ji.z)));
-        }
+    if (tile.vp[q])
+      force_pair_finish(p, tile.ip[q], fs01[q], fs2[q], DAMAGE && any_broken);
+  }
+}
+
+// The same with a warp per stencil plane (k_deformation_planes).
+template <bool DAMAGE, bool UNROLL, int THREADS, int MINB>
+__global__ void __launch_bounds__(THREADS, MINB) k_force_planes(const __grid_constant__ StepParams p) {
+  extern __shared__ float2 s_part[];  // [nplanes][2][32] rows 0, 1 by point; then [nplanes][32] row 2 of both points
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, planes = p.st.nplanes;
+  float2 *s_part2 = s_part + planes * 64;
+  __shared__ int s_broken[32];
+  const float h = (float)p.lat_h;
+  const PairTile tile = pair_tile(p, (int64_t)blockIdx.x * 32 + lane);
+  float jx[2], jy[2], jz[2];
+  force_pair_points(p, tile, h, jx, jy, jz);
+  if (threadIdx.x < 32)
+    s_broken[lane] = 0;
+  float2 part01[2] = {make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f)};
+  float part2[2] = {0.0f, 0.0f};
+  bool any_broken = false;
+  force_pair_groups<DAMAGE, UNROLL>(p, p.st.plane[warp], p.st.plane[warp + 1], tile, h, jx, jy, jz, part01, part2,
+                                    any_broken, [](int) {});
+  s_part[(warp * 2) * 32 + lane] = part01[0], s_part[(warp * 2 + 1) * 32 + lane] = part01[1];
+  s_part2[warp * 32 + lane] = make_float2(part2[0], part2[1]);
+  __syncthreads();
+  if (DAMAGE) {
+    if (any_broken)
+      s_broken[lane] = 1;
+    __syncthreads();
+  }
+  for (int q = warp; q < 2; q += planes) {  // warp q: point q of every tile
+    float2 fs01 = make_float2(0.0f, 0.0f), fc01 = fs01;
+    float fs2 = 0.0f, fc2 = 0.0f;
+    for (int w = 0; w < planes; ++w) {
+      const float2 r2 = s_part2[w * 32 + lane];
+      kahan_add2(fs01, fc01, s_part[(w * 2 + q) * 32 + lane]), kahan_add(fs2, fc2, q ? r2.y : r2.x);
     }
-    float VM[9];
-    fmap_rows(P0[i], P1[i], P2[i], VM);
-    const double4 s = p.vxi[i];
-    const double s0 = s.x - c0, s1 = s.y - c1, s2 = s.z - c2;
-    const double rv = 1.0 / (double)p.jit[i].w;
-    const double f0 = (double)fs01[q].x + (VM[0] * s0 + VM[1] * s1 + VM[2] * s2) * rv;
-    const double f1 = (double)fs01[q].y + (VM[3] * s0 + VM[4] * s1 + VM[5] * s2) * rv;
-    const double f2 = (double)fs2[q] + (VM[6] * s0 + VM[7] * s1 + VM[8] * s2) * rv;
-    p.force[i] = make_double4(f0, f1, f2, 0.0);
+    if (tile.vp[q])
+      force_pair_finish(p, tile.ip[q], fs01, fs2, DAMAGE && s_broken[lane]);
   }
 }
 
 // ------------------------------------------------------------------ launchers
+// Whether the packed kernels run with a warp per stencil plane (p.tiled: 5 always, 8 never). Per increment in
+// microseconds, a thread per tile | a warp per plane, horizon 4.015 h: 1,600 points 96 | 37, 4,000 99 | 38, 10,605
+// 118 | 48, 20,400 101 | 62, 54,000 106 | 91, 79,360 145 | 139, 108,900 168 | 189; at 3.015 h: 4,000 63 | 34, 54,000
+// 70 | 67, 79,360 95 | 102; with damage at 4.015 h: 4,000 128 | 44, 54,000 138 | 123, 79,360 176 | 189.
+constexpr int64_t kPlanesPoints = 60000;
+static bool by_planes(const StepParams &p) {
+  return p.st.nplanes > 1 && (p.tiled == 5 || (p.tiled != 8 && p.n <= kPlanesPoints));
+}
+
+// launch(std::integral_constant<int, THREADS>, <int, MINB>) with the bounds that fit a block of nplanes warps: two blocks
+// per SM up to nine planes (the stencils of horizons to just over four spacings)
+template <typename F> static void with_plane_threads(const StepParams &p, F &&launch) {
+  using std::integral_constant;
+  if (p.st.nplanes <= 7)
+    launch(integral_constant<int, 224>{}, integral_constant<int, 2>{});
+  else if (p.st.nplanes <= 9)
+    launch(integral_constant<int, 288>{}, integral_constant<int, 2>{});
+  else
+    launch(integral_constant<int, 32 * kMaxPlanes>{}, integral_constant<int, 1>{});
+}
+
 // With damage the scalar deformation kernel keeps the runtime window loop (unrolled, its
 // stretch tests made it slower: 0.28 against 0.25 ms on the 250k-point bar); the packed-pair
 // kernel unrolls its windows with damage too (0.698 against 0.783 ms on the 1M-point bar).
+template <bool DAMAGE, bool UNROLL> static void launch_deformation_pair(const StepParams &p, cudaStream_t s) {
+  const int64_t tiles = (int64_t)p.lat_nx * ((p.lat_ny + 1) / 2) * p.lat_nz;
+  if (by_planes(p))
+    with_plane_threads(p, [&](auto threads, auto minb) {
+      k_deformation_planes<DAMAGE, UNROLL, decltype(threads)::value, decltype(minb)::value>
+          <<<tiled_blocks<2, 32>(p), 32 * p.st.nplanes, sizeof(float2) * 9 * 32 * p.st.nplanes, s>>>(p);
+    });
+  else if (tiles > 148 * 512 && tiles <= 148 * 576)  // one wave of 18 warps per SM, not of 16: 82 against 87 us
+    k_deformation_pair<DAMAGE, UNROLL, 192, 3><<<tiled_blocks<2, 192>(p), 192, 0, s>>>(p);
+  else if (DAMAGE)  // 161 against 165 us in 128-thread blocks at 500,000 points
+    k_deformation_pair<DAMAGE, UNROLL, 256, 2><<<tiled_blocks<2, 256>(p), 256, 0, s>>>(p);
+  else  // 365 against 372 us in 256-thread blocks at 1M points
+    k_deformation_pair<DAMAGE, UNROLL, 128, 4><<<tiled_blocks<2, 128>(p), 128, 0, s>>>(p);
+}
 template <bool UNROLL> static void launch_deformation(const StepParams &p, cudaStream_t s) {
-  const unsigned grid = tiled_grid<2>(p);
+  const unsigned grid = tiled_blocks<2, kBondThreads>(p);
   if (p.tiled == 1) {
     if (p.damage)
       k_deformation_tiled<true, 2, false><<<grid, kBondThreads, 0, s>>>(p);
     else
       k_deformation_tiled<false, 2, UNROLL><<<grid, kBondThreads, 0, s>>>(p);
   } else {
-    if (p.damage)
-      k_deformation_pair<true, UNROLL><<<grid, kBondThreads, 0, s>>>(p);
-    else
-      k_deformation_pair<false, UNROLL><<<grid, kBondThreads, 0, s>>>(p);
+    p.damage ? launch_deformation_pair<true, UNROLL>(p, s) : launch_deformation_pair<false, UNROLL>(p, s);
   }
 }
 
@@ -763,21 +994,28 @@ int launch_deformation_tiled(const StepParams &p, cudaStream_t s) {
   return VPD_OK;
 }
 
+template <bool DAMAGE, bool UNROLL> static void launch_force_pair(const StepParams &p, cudaStream_t s) {
+  if (by_planes(p))
+    with_plane_threads(p, [&](auto threads, auto minb) {
+      k_force_planes<DAMAGE, UNROLL, decltype(threads)::value, decltype(minb)::value>
+          <<<tiled_blocks<2, 32>(p), 32 * p.st.nplanes, sizeof(float2) * 96 * p.st.nplanes, s>>>(p);
+    });
+  else
+    k_force_pair<DAMAGE, UNROLL><<<tiled_blocks<2, kForcePairThreads>(p), kForcePairThreads, 0, s>>>(p);
+}
+
 int launch_force_tiled(const StepParams &p, cudaStream_t s) {
   const bool u = index32(p);
-  const unsigned grid = tiled_grid<2>(p);
+  const unsigned grid = tiled_blocks<2, kBondThreads>(p);
   if (p.tiled == 1) {
     if (u)
       k_force_tiled<2, true><<<grid, kBondThreads, 0, s>>>(p);
     else
       k_force_tiled<2, false><<<grid, kBondThreads, 0, s>>>(p);
+  } else if (p.damage) {
+    u ? launch_force_pair<true, true>(p, s) : launch_force_pair<true, false>(p, s);
   } else {
-    if (p.damage)
-      u ? k_force_pair<true, true><<<grid, kBondThreads, 0, s>>>(p)
-        : k_force_pair<true, false><<<grid, kBondThreads, 0, s>>>(p);
-    else
-      u ? k_force_pair<false, true><<<grid, kBondThreads, 0, s>>>(p)
-        : k_force_pair<false, false><<<grid, kBondThreads, 0, s>>>(p);
+    u ? launch_force_pair<false, true>(p, s) : launch_force_pair<false, false>(p, s);
   }
   VPD_CUDA(cudaGetLastError());
   return VPD_OK;
