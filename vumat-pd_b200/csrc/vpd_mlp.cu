@@ -18,8 +18,15 @@ constexpr int kWeightBytes = 4096 + 32768 + 32768 + 4096;
 struct StagedWeights {
   unsigned char *w1, *w2, *w3, *w4;
 };
-__device__ __forceinline__ StagedWeights stage_weights(unsigned char *s, const MlpWeights &w) {
+// Every thread calls it; complete at stage_wait() and, for tiled weights, the first phase of wbar (initialised by
+// thread 0).
+__device__ __forceinline__ StagedWeights stage_weights(unsigned char *s, const MlpWeights &w, uint64_t *wbar) {
   const StagedWeights sw{s, s + 4096, s + 4096 + 32768, s + 4096 + 65536};
+  if (w.tiled) {
+    if (threadIdx.x == 0)
+      umma::bulk_load(s, w.w1, kWeightBytes, wbar);
+    return sw;
+  }
   stage_rowmajor(sw.w1, w.w1, kMlpHidden, kMlpIn);
   stage_rowmajor(sw.w2, w.w2, kMlpHidden, kMlpHidden);
   stage_rowmajor(sw.w3, w.w3, kMlpHidden, kMlpHidden);
@@ -36,7 +43,7 @@ __device__ __forceinline__ StagedWeights stage_weights(unsigned char *s, const M
 // block per tile that staged the 72 KB of weights each time), the tanh unit about half busy; the rest is the chain's
 // waits (barriers, TMEM loads) at 16 warps.
 constexpr int kGroups = 4;
-constexpr size_t kFwdSmem = kWeightBytes + kGroups * 32768 + kGroups * 16 + 4 * kBiasFloats;
+constexpr size_t kFwdSmem = kWeightBytes + kGroups * 32768 + (kGroups + 1) * 16 + 4 * kBiasFloats;
 
 // Four consecutive floats; the callers' arrays may start at any multiple of 4 bytes (vec: at one of 16).
 __device__ __forceinline__ float4 load4(const float *p, bool vec) {
@@ -70,14 +77,17 @@ __global__ void __launch_bounds__(128 * kGroups, 1) k_mlp_forward(MlpWeights w, 
   extern __shared__ __align__(1024) unsigned char smem[];
   unsigned char *sAll = smem + kWeightBytes;
   uint64_t *mbars = reinterpret_cast<uint64_t *>(sAll + kGroups * 32768);
-  float *sBias = reinterpret_cast<float *>(sAll + kGroups * 32768 + kGroups * 16);
+  uint64_t *wbar = mbars + 2 * kGroups;
+  float *sBias = reinterpret_cast<float *>(sAll + kGroups * 32768 + (kGroups + 1) * 16);
   __shared__ uint32_t s_tmem;
   const int g = threadIdx.x >> 7, t = threadIdx.x & 127;
   if (threadIdx.x < 32)
     umma::tmem_alloc(&s_tmem, 128 * kGroups);
   if (t == 0)
     umma::mbar_init(mbars + 2 * g, 1);
-  const StagedWeights sw = stage_weights(smem, w);
+  if (threadIdx.x == 0)
+    umma::mbar_init(wbar, 1);
+  const StagedWeights sw = stage_weights(smem, w, wbar);
   stage_biases(sBias, w);
   stage_wait();
   umma::fence_proxy_async();
@@ -89,7 +99,7 @@ __global__ void __launch_bounds__(128 * kGroups, 1) k_mlp_forward(MlpWeights w, 
   const uint32_t tmem = s_tmem + 128u * g;
   const uint32_t trow = tmem + ((uint32_t)(t & ~31) << 16);  // this warp's TMEM lanes
   uint32_t phase = 0;
-  bool ok = true;
+  bool ok = !w.tiled || group_all(g, umma::mbar_wait(wbar, 0u, kWaitLimit));
   // D = A B^T by the group's first thread, awaited by the group
   auto product = [&](const unsigned char *b, int K, int N) {
     umma::fence_proxy_async();
@@ -168,8 +178,10 @@ __global__ void __launch_bounds__(128 * kGroups, 1) k_mlp_forward(MlpWeights w, 
 //   backward  dZ = dY * silu'(Z); dW = dZ^T Y_prev and dY_prev = dZ W. The products that need an operand the other
 //             way round read the forward pass's own tiles through MN-major descriptors.
 // The tile's weight and bias gradients go to the block's slice of `partials`; the slices are summed in block
-// order, so the gradient does not depend on the order the blocks run in. Batch 8192 on a B200: 27 us and 3.5 us for
-// the sum (46 + 60 + 6 us in the separate kernels); eight dependent stages at one block on 64 SMs, so latency.
+// order, so the gradient does not depend on the order the blocks run in. Batch 8192 on a B200: 21 us (20 with
+// tiled weights) and 3.3 us for the sum (46 + 60 + 6 us in the separate kernels). Eight dependent stages at one
+// block on 64 SMs, so latency: about 4 us to start and stage, 0.2 to 0.5 us a product, 0.7 us a forward epilogue, 1.6
+// to 3 us a backward one with its stores (5.5 us before they turned through shared memory).
 constexpr int kGradThreads = 512;
 // weights | Y0 (128x16) | Y1 | Y2 | Y3 | dZ (128x128) | dZ4 (128x16) | mbarrier | biases
 constexpr size_t kGradSmem = kWeightBytes + 4096 + 4 * 32768 + 4096 + 64 + 4 * kBiasFloats;
@@ -214,9 +226,10 @@ __global__ void __launch_bounds__(kGradThreads, 1) k_mlp_gradient(MlpWeights w, 
   const MlpGrads grad = mlp_grads(partials + (size_t)blockIdx.x * kMlpParams);
   if (warp == 0)
     umma::tmem_alloc(&s_tmem, 512);
+  uint64_t *wbar = mbar + 2;
   if (threadIdx.x == 0)
-    umma::mbar_init(mbar, 1);
-  const StagedWeights sw = stage_weights(smem, w);
+    umma::mbar_init(mbar, 1), umma::mbar_init(wbar, 1);
+  const StagedWeights sw = stage_weights(smem, w, wbar);
   stage_biases(sBias, w);
   // the batch row's place in the arrays it is read from
   auto source = [&](int64_t r) {
@@ -231,6 +244,15 @@ __global__ void __launch_bounds__(kGradThreads, 1) k_mlp_gradient(MlpWeights w, 
                                         __float2bfloat16(v.w)};
     *reinterpret_cast<uint2 *>(sY0 + kmajor_offset(rr, 4 * part, kMlpIn)) = *reinterpret_cast<const uint2 *>(xb);
   }
+  // the output layer's rows, a row per thread of the first group: read now, used after the forward pass
+  float4 last[4];
+  if (group == 0) {
+    const float *from = TRAIN ? batch.target + (keep ? source(row) : 0) * 16 : batch.gout + (keep ? row : 0) * kMlpOut;
+    const bool vec = aligned16(from);
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+      last[c] = load4(from + 4 * c, vec);
+  }
   stage_wait();
   umma::fence_before_sync();
   __syncthreads();
@@ -239,6 +261,11 @@ __global__ void __launch_bounds__(kGradThreads, 1) k_mlp_gradient(MlpWeights w, 
   // four accumulators of 128 columns
   const uint32_t T0 = tmem, T1 = tmem + 128, T2 = tmem + 256, T3 = tmem + 384;
   Sync sy{mbar, 0u, err, 1u, true};
+  if (w.tiled) {
+    sy.ok = __syncthreads_and(umma::mbar_wait(wbar, 0u, kWaitLimit)) != 0;
+    if (!sy.ok && threadIdx.x == 0)
+      atomicOr(err, 1u);
+  }
   // The stage's products, issued by one thread once every thread's operands are in place, awaited by all.
   auto stage = [&](auto issue) {
     umma::fence_proxy_async();
@@ -279,7 +306,8 @@ __global__ void __launch_bounds__(kGradThreads, 1) k_mlp_gradient(MlpWeights w, 
       float o[16], l = 0.0f;
       if (sy.ok)
         umma::tmem_ld16(T3 + lanes, o);
-      const float *target = batch.target + (keep ? source(row) : 0) * 16;
+      const float target[16] = {last[0].x, last[0].y, last[0].z, last[0].w, last[1].x, last[1].y, last[1].z, last[1].w,
+                                last[2].x, last[2].y, last[2].z, last[2].w, last[3].x, last[3].y, last[3].z, last[3].w};
       const float wr = keep ? target[15] : 0.0f, norm = 1.0f / (float)(B * SURROGATE_TARGETS);
 #pragma unroll
       for (int c = 0; c < kMlpOut; ++c) {
@@ -295,8 +323,10 @@ __global__ void __launch_bounds__(kGradThreads, 1) k_mlp_gradient(MlpWeights w, 
         atomicAdd(batch.loss, l);
     } else {
 #pragma unroll
-      for (int c = 0; c < kMlpOut; ++c)
-        dz4[c] = keep ? batch.gout[row * kMlpOut + c] : 0.0f;
+      for (int c = 0; c < 4; ++c) {
+        dz4[4 * c] = keep ? last[c].x : 0.0f, dz4[4 * c + 1] = keep ? last[c].y : 0.0f;
+        dz4[4 * c + 2] = keep ? last[c].z : 0.0f, dz4[4 * c + 3] = keep ? last[c].w : 0.0f;
+      }
     }
     __align__(16) __nv_bfloat16 zb[16];
 #pragma unroll
@@ -338,15 +368,23 @@ __global__ void __launch_bounds__(kGradThreads, 1) k_mlp_gradient(MlpWeights w, 
       float v[32], z[32];
       umma::tmem_ld32(T3 + lanes + c0, v);
       umma::tmem_ld32(Z + lanes + c0, z);
-      __align__(16) __nv_bfloat16 zb[32];
+      __align__(16) __nv_bfloat162 zb[16];
 #pragma unroll
-      for (int c = 0; c < 32; ++c) {
-        v[c] = keep ? v[c] * silu_grad(z[c] + bias[c0 + c]) : 0.0f;
-        zb[c] = __float2bfloat16(v[c]);
+      for (int q = 0; q < 8; ++q) {
+        const float4 bb = *reinterpret_cast<const float4 *>(bias + c0 + 4 * q);
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const int c = 4 * q + 2 * e;
+          float2 d = silu_grad2(make_float2(v[c], v[c + 1]), make_float2(z[c], z[c + 1]),
+                                e ? make_float2(bb.z, bb.w) : make_float2(bb.x, bb.y));
+          d = keep ? d : make_float2(0.0f, 0.0f);
+          v[c] = d.x, v[c + 1] = d.y;
+          zb[2 * q + e] = __floats2bfloat162_rn(d.x, d.y);
+        }
       }
 #pragma unroll
       for (int k = 0; k < 4; ++k)
-        *reinterpret_cast<uint4 *>(sDZ + kmajor_offset(t, c0 + 8 * k, H)) = *reinterpret_cast<const uint4 *>(zb + 8 * k);
+        *reinterpret_cast<uint4 *>(sDZ + kmajor_offset(t, c0 + 8 * k, H)) = *reinterpret_cast<const uint4 *>(zb + 4 * k);
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         float slab[16];
@@ -378,10 +416,24 @@ __global__ void __launch_bounds__(kGradThreads, 1) k_mlp_gradient(MlpWeights w, 
       if (layer > 1) {  // this thread's 32 columns of row t of dW [out][in]
         float v[32];
         umma::tmem_ld32(Z + lanes + c0, v);
-        float4 *dst = reinterpret_cast<float4 *>((layer == 3 ? grad.w3 : grad.w2) + (size_t)t * H + c0);
+        // through the warp's 2 KB of Y3 (not needed any more), 16 columns at a time: a store then covers 64 bytes of
+        // eight rows instead of 16 bytes of 32 (the 16-byte chunks swizzled against bank conflicts)
+        float4 *turn = reinterpret_cast<float4 *>(sY3) + warp * 128;
+        float *dst = (layer == 3 ? grad.w3 : grad.w2) + (size_t)(quarter * 32) * H + c0;
 #pragma unroll
-        for (int q = 0; q < 8; ++q)
-          dst[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+        for (int h = 0; h < 2; ++h) {
+#pragma unroll
+          for (int q = 0; q < 4; ++q)
+            turn[lane * 4 + (q ^ ((lane >> 1) & 3))] =
+                make_float4(v[16 * h + 4 * q], v[16 * h + 4 * q + 1], v[16 * h + 4 * q + 2], v[16 * h + 4 * q + 3]);
+          __syncwarp();
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const int rr = 8 * k + (lane >> 2), q = lane & 3;
+            *reinterpret_cast<float4 *>(dst + (size_t)rr * H + 16 * h + 4 * q) = turn[rr * 4 + (q ^ ((rr >> 1) & 3))];
+          }
+          __syncwarp();
+        }
       } else if (group == 0) {
         float v[16];
         umma::tmem_ld16(Z + lanes, v);
@@ -413,7 +465,8 @@ __global__ void k_sum_partials(const float *partials, int nblocks, float *grad) 
     grad[i] = partial_sum(partials, nblocks, i);
 }
 
-// One Adam step on the summed gradient; the weights (the first kMlpWeights parameters) also to their BF16 copy.
+// One Adam step on the summed gradient; the weights (the first kMlpWeights parameters) also to their BF16 copy, in
+// tiled storage.
 __global__ void k_adam(const float *partials, int nblocks, float *p, float *m, float *v, __nv_bfloat16 *pb, float lr,
                        float b1, float b2, float eps, float c1, float c2) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -426,7 +479,7 @@ __global__ void k_adam(const float *partials, int nblocks, float *p, float *m, f
   const float pi = p[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
   p[i] = pi;
   if (i < kMlpWeights)
-    pb[i] = __float2bfloat16(pi);
+    pb[mlp_tile_index(i)] = __float2bfloat16(pi);
 }
 
 int mlp_forward(const MlpWeights &w, const float *x, int64_t B, float *out, unsigned *err, cudaStream_t s) {

@@ -20,7 +20,17 @@ constexpr int64_t kMlpParams = kMlpWeights + 128 * 3 + 16;
 struct MlpWeights {
   const __nv_bfloat16 *w1, *w2, *w3, *w4;
   const float *b1, *b2, *b3, *b4;
+  // the four matrices, one after the other, stored as the operand tiles (mlp_tile_index) instead of row-major: a
+  // block then stages all of them with one bulk copy
+  bool tiled = false;
 };
+// Where the flat parameter i (< kMlpWeights) stands in tiled storage: in its matrix, core matrices of 8 rows x 8
+// columns follow one another along a row.
+__host__ __device__ inline int mlp_tile_index(int i) {
+  const int base = i < 2048 ? 0 : (i < 2048 + 32768 ? 2048 + ((i - 2048) & ~16383) : 2048 + 32768);
+  const int cols = i < 2048 ? 16 : 128, r = (i - base) / cols, c = (i - base) % cols;
+  return base + (r >> 3) * 8 * cols + (c >> 3) * 64 + (r & 7) * 8 + (c & 7);
+}
 
 struct MlpGrads {  // FP32 accumulators, same shapes as the parameters
   float *w1, *w2, *w3, *w4, *b1, *b2, *b3, *b4;
@@ -53,7 +63,8 @@ int mlp_gradient_partials(const MlpWeights &w, const MlpBatch &batch, int64_t B,
                           cudaStream_t s);
 // grad [kMlpParams] = the partials' sum in block order.
 int mlp_sum_partials(const float *partials, int64_t blocks, float *grad, cudaStream_t s);
-// The same sum taken straight into one Adam step on the parameters p (m, v: moments); wb: the weights' BF16 copy.
+// The same sum taken straight into one Adam step on the parameters p (m, v: moments); wb: the weights' BF16 copy
+// (tiled storage).
 int mlp_adam(const float *partials, int64_t blocks, float *p, float *m, float *v, __nv_bfloat16 *wb, float lr,
              int step, cudaStream_t s);
 

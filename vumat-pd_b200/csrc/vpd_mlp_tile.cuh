@@ -32,9 +32,14 @@ __device__ __forceinline__ __nv_bfloat162 silu2(float2 v, float2 bias) {
   const float2 y = __ffma2_rn(h, make_float2(tanh_approx(h.x), tanh_approx(h.y)), h);
   return __floats2bfloat162_rn(y.x, y.y);
 }
-__device__ __forceinline__ float silu_grad(float z) {
-  const float s = fmaf(0.5f, tanh_approx(0.5f * z), 0.5f);
-  return s * fmaf(z, 1.0f - s, 1.0f);
+// dy silu'(v + bias) of two columns as packed pairs, with sigma = (1 + tanh(z / 2)) / 2: silu'(z) = sigma (1 + z (1 -
+// sigma)).
+__device__ __forceinline__ float2 silu_grad2(float2 dy, float2 v, float2 bias) {
+  const float2 one = make_float2(1.0f, 1.0f), half = make_float2(0.5f, 0.5f);
+  const float2 z = __fadd2_rn(v, bias), h = __fmul2_rn(half, z);
+  const float2 s = __ffma2_rn(half, make_float2(tanh_approx(h.x), tanh_approx(h.y)), half);
+  const float2 c = __ffma2_rn(s, make_float2(-1.0f, -1.0f), one);  // 1 - s
+  return __fmul2_rn(dy, __fmul2_rn(s, __ffma2_rn(z, c, one)));
 }
 
 // Shared-memory store of one bf16 element at (row, k) of a K-major tile.
@@ -42,13 +47,15 @@ __device__ __forceinline__ void st_bf16(unsigned char *tile, int row, int k, int
   *reinterpret_cast<__nv_bfloat16 *>(tile + kmajor_offset(row, k, ktotal)) = __float2bfloat16(v);
 }
 
-// Copies a row-major bf16 matrix [rows][cols] (16-byte aligned) into a K-major tile (K = cols),
-// 16 bytes at a time with cp.async: every copy of the thread is in flight at once. The copies
-// complete at stage_wait(), which every thread calls before the barrier that publishes them.
+// Copies a row-major bf16 matrix [rows][cols] (16-byte aligned; rows a multiple of 8) into a K-major tile (K = cols),
+// 16 bytes at a time with cp.async: every copy of the thread is in flight at once. Eight consecutive threads
+// take the eight rows of a core matrix, 128 consecutive bytes of the tile (along a row their copies all fell into
+// the same banks). The copies complete at stage_wait(), which every thread calls before the barrier that
+// publishes them.
 __device__ __forceinline__ void stage_rowmajor(unsigned char *tile, const __nv_bfloat16 *src, int rows, int cols) {
   const int chunks = rows * cols / 8;
   for (int c = threadIdx.x; c < chunks; c += blockDim.x) {
-    const int row = c / (cols / 8), k = (c % (cols / 8)) * 8;
+    const int core = c >> 3, row = core / (cols / 8) * 8 + (c & 7), k = (core % (cols / 8)) * 8;
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(tile + kmajor_offset(row, k, cols))),
                  "l"(src + (size_t)row * cols + k)
                  : "memory");

@@ -147,10 +147,11 @@ int surrogate_samples_dev(const JcParams &jc, uint64_t seed, int64_t count, floa
 }
 
 // ------------------------------------------------------------------ training
-__global__ void k_to_bf16(const float *p, __nv_bfloat16 *q, int64_t n) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n)
-    q[i] = __float2bfloat16(p[i]);
+// The weights' BF16 copy in tiled storage.
+__global__ void k_to_bf16(const float *p, __nv_bfloat16 *q) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < kMlpWeights)
+    q[mlp_tile_index(i)] = __float2bfloat16(p[i]);
 }
 
 // *sum += the plastic rows among the training targets (row weight 1 in column 15).
@@ -266,10 +267,11 @@ int train_surrogate(const vpd_surrogate_config &cfg, uint16_t *w_out, float *b_o
   VPD_CUDA(cudaGetLastError());
   VPD_CUDA(cudaMemsetAsync(loss, 0, sizeof(float) * (VPD_SURROGATE_MAX_EPOCHS + 1), s));
   VPD_CUDA(cudaMemsetAsync(err, 0, sizeof(unsigned), s));
-  k_to_bf16<<<(unsigned)((kMlpWeights + 255) / 256), 256, 0, s>>>(P, Wb, kMlpWeights);
+  k_to_bf16<<<(unsigned)((kMlpWeights + 255) / 256), 256, 0, s>>>(P, Wb);
   VPD_CUDA(cudaGetLastError());
 
-  const MlpWeights w = mlp_weights(Wb, P + kMlpWeights);
+  MlpWeights w = mlp_weights(Wb, P + kMlpWeights);
+  w.tiled = true;
   const int64_t steps = T / B;
   int adam_step = 0;
   MlpBatch batch{};
@@ -308,7 +310,8 @@ int train_surrogate(const vpd_surrogate_config &cfg, uint16_t *w_out, float *b_o
   VPD_CUDA(cudaStreamSynchronize(s));
   if (herr)
     return set_error(VPD_ERR_CUDA, "vpd_train_surrogate: tensor-core wait timed out");
-  std::copy(hw.begin(), hw.end(), w_out);
+  for (int64_t i = 0; i < kMlpWeights; ++i)
+    w_out[i] = hw[(size_t)mlp_tile_index((int)i)];
   if (rep) {
     *rep = vpd_surrogate_report{};
     rep->epochs_run = cfg.epochs;

@@ -79,6 +79,16 @@ __device__ __forceinline__ void mbar_init(uint64_t *mbar, uint32_t count) {
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
 
+// Copies `bytes` (a multiple of 16; both addresses on 16-byte boundaries) of global memory into shared memory as one
+// asynchronous bulk copy; the mbarrier's phase completes with it.
+__device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t bytes, uint64_t *mbar) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(mbar)), "r"(bytes) : "memory");
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                   smem_u32(dst)),
+               "l"(src), "r"(bytes), "r"(smem_u32(mbar))
+               : "memory");
+}
+
 // Waits for the mbarrier phase with the given parity; gives up after `limit` polls and
 // returns false (the caller reports the timeout instead of spinning forever).
 __device__ __forceinline__ bool mbar_wait(uint64_t *mbar, uint32_t parity, uint32_t limit) {
