@@ -36,12 +36,17 @@ __device__ __forceinline__ StagedWeights stage_weights(unsigned char *s, const M
 
 // ------------------------------------------------------------------ forward
 // Persistent blocks, one per SM: the weights are staged once, and four groups of 128 threads run a tile each
-// (thread t of a group = row t = TMEM lane t), with their own operand tile, 128 TMEM columns, mbarrier and
+// (thread t of a group = TMEM lane t), with their own operand tile, 128 TMEM columns, mbarrier and
 // named barrier. A tile's four products and epilogues are a serial chain; the four groups of a block
-// overlap theirs. What bounds it is the epilogue: 384 tanh per row at 16 per SM and clock, 83 us for 1M rows,
-// against 43 us of tensor work and 20 us of memory traffic. Measured on a B200: 161 us for 1M rows (490 with a
-// block per tile that staged the 72 KB of weights each time), the tanh unit about half busy; the rest is the chain's
-// waits (barriers, TMEM loads) at 16 warps.
+// overlap theirs. The hidden layers are formed as Y^T = W Y_prev^T, features along the lanes, so that a thread
+// has one bias a layer, in a register: with batch rows along the lanes a thread read all 128 from shared memory. The
+// activations are stored [feature][batch row], for the next product to read through MN-major descriptors; the output
+// layer reads them as its first operand, so its batch rows are lanes again.
+// What bounds it is the epilogue: 384 tanh per row at 16 per SM and clock, 83 us for 1M rows,
+// against 43 us of tensor work and 20 us of memory traffic. Measured on a B200: 137 us for 1M rows (152 with
+// the batch rows along the lanes; 490 with a block per tile that staged the 72 KB of weights each time), the
+// tanh unit about 60 % busy; without its tanh the kernel takes 106 us, without its tensor work 130. Two warps a
+// TMEM quarter (142 us) and two half tiles a group in turn (148) have shorter waits but more of them.
 constexpr int kGroups = 4;
 constexpr size_t kFwdSmem = kWeightBytes + kGroups * 32768 + (kGroups + 1) * 16 + 4 * kBiasFloats;
 
@@ -94,23 +99,25 @@ __global__ void __launch_bounds__(128 * kGroups, 1) k_mlp_forward(MlpWeights w, 
   umma::fence_before_sync();
   __syncthreads();
   umma::fence_after_sync();
-  unsigned char *sA = sAll + g * 32768;  // the layer's input rows (the 16 features in its first 4 KB)
+  unsigned char *sA = sAll + g * 32768;  // the batch rows' 16 features (in its first 4 KB), then the activations
   uint64_t *mbar = mbars + 2 * g;
   const uint32_t tmem = s_tmem + 128u * g;
   const uint32_t trow = tmem + ((uint32_t)(t & ~31) << 16);  // this warp's TMEM lanes
   uint32_t phase = 0;
   bool ok = !w.tiled || group_all(g, umma::mbar_wait(wbar, 0u, kWaitLimit));
-  // D = A B^T by the group's first thread, awaited by the group
-  auto product = [&](const unsigned char *b, int K, int N) {
+  const float b1 = sBias[t], b2 = sBias[kMlpHidden + t], b3 = sBias[2 * kMlpHidden + t];
+  // D = A B^T by the group's first thread, awaited by the group. A wait that runs out leaves ok false; the group
+  // votes on it once a tile.
+  auto product = [&](const umma::Operand &a, const umma::Operand &b, int K, int N) {
     umma::fence_proxy_async();
     umma::fence_before_sync();
     group_sync(g);
     if (t == 0) {
       umma::fence_after_sync();
-      umma::gemm_issue(tmem, umma::k_major(sA, K), umma::k_major(b, K), K, N);
+      umma::gemm_issue(tmem, a, b, K, N);
       umma::commit(mbar);
     }
-    ok = group_all(g, umma::mbar_wait(mbar, phase, kWaitLimit));
+    ok = umma::mbar_wait(mbar, phase, kWaitLimit) && ok;
     phase ^= 1u;
     umma::fence_after_sync();
   };
@@ -139,13 +146,15 @@ __global__ void __launch_bounds__(128 * kGroups, 1) k_mlp_forward(MlpWeights w, 
     *reinterpret_cast<uint4 *>(sA + kmajor_offset(t, 8, kMlpIn)) = *reinterpret_cast<const uint4 *>(xb + 8);
     if (tile + stride < tiles)
       load(tile + stride);
-    product(sw.w1, kMlpIn, kMlpHidden);
-    if (ok)
-      hidden_epilogue(trow, sBias, sA, t), product(sw.w2, kMlpHidden, kMlpHidden);
-    if (ok)
-      hidden_epilogue(trow, sBias + kMlpHidden, sA, t), product(sw.w3, kMlpHidden, kMlpHidden);
-    if (ok)
-      hidden_epilogue(trow, sBias + 2 * kMlpHidden, sA, t), product(sw.w4, kMlpHidden, kMlpOut);
+    const umma::Operand y = umma::mn_major(sA, 128);
+    product(umma::k_major(sw.w1, kMlpIn), umma::k_major(sA, kMlpIn), kMlpIn, 128);
+    feature_epilogue(trow, b1, sA, t);
+    product(umma::k_major(sw.w2, kMlpHidden), y, kMlpHidden, 128);
+    feature_epilogue(trow, b2, sA, t);
+    product(umma::k_major(sw.w3, kMlpHidden), y, kMlpHidden, 128);
+    feature_epilogue(trow, b3, sA, t);
+    product(y, umma::k_major(sw.w4, kMlpHidden), kMlpHidden, kMlpOut);
+    ok = group_all(g, ok);
     const int64_t row = tile * 128 + t;
     float v[16];
     if (ok)

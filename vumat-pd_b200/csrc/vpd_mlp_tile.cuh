@@ -132,4 +132,22 @@ __device__ __forceinline__ void hidden_epilogue(uint32_t trow, const float *bias
   }
 }
 
+// The same with the features along the TMEM lanes (thread t: feature t and its bias) and the 128 batch rows along
+// the columns: row t of the next layer's operand A, stored [feature][batch row].
+__device__ __forceinline__ void feature_epilogue(uint32_t trow, float bias, unsigned char *A, int t) {
+#pragma unroll 1
+  for (int c0 = 0; c0 < 128; c0 += 32) {
+    float v[32];
+    umma::tmem_ld32(trow + c0, v);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      __align__(16) __nv_bfloat162 yb[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        yb[q] = silu2(make_float2(v[8 * k + 2 * q], v[8 * k + 2 * q + 1]), make_float2(bias, bias));
+      *reinterpret_cast<uint4 *>(A + kmajor_offset(t, c0 + 8 * k, 128)) = *reinterpret_cast<const uint4 *>(yb);
+    }
+  }
+}
+
 }  // namespace vpd
