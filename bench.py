@@ -245,13 +245,17 @@ def cpu_reference(steps, warmup, preload):
     without bond damage: `preload` increments from rest into plastic flow, `warmup` more, then
     `steps` timed increments. The library's runMaterial order calls the damage module every
     increment even with the model "none" (it copies the per-bond damage arrays,
-    PdSimpleDamage.cpp:61,94), so that stage stays in its time."""
+    PdSimpleDamage.cpp:61,94), so that stage stays in its time. {"unavailable": why} where the
+    library has not been built (its sources are absent)."""
     sys.path.insert(0, os.path.join(ROOT, "oracle"))
     import oracle as O
     import vpd
     from vpd.case import tensile_bar
     case = tensile_bar(3, nx=SAMPLE_NX, precision=0, damage_mode=0)
-    sim = O.RefSim(case)
+    try:
+        sim = O.RefSim(case)
+    except FileNotFoundError as e:
+        return {"unavailable": f"{os.path.basename(str(e).split()[0])} is not built"}
     sim.step(preload + warmup)
     before = sim.stage_seconds()
     t0 = time.perf_counter()
@@ -287,6 +291,9 @@ def run_reference(args, world, rank):
     if rank != 0:
         return
     base = cpu_reference(args.steps, args.warmup, args.cpu_preload)
+    if "unavailable" in base:
+        print(json.dumps({"impl": "reference", **base}), flush=True)
+        return
     print(json.dumps({
         "impl": "reference", "metric": METRIC, "value": base["value"], "unit": UNIT,
         "n_gpus": args.gpus, "steps": args.steps, "warmup": args.warmup,
@@ -519,8 +526,9 @@ def run_gpu(args, world, rank, local):
                           "frac": step_alg / (ms_step * 1e-3) / 1e9 / peak,
                           "index_formulation_bytes": survey,
                           "index_formulation_frac": survey / (ms_step * 1e-3) / 1e9 / peak},
-        "cpu_baseline": {k: cpu[k] for k in ("value", "unit", "cores", "kind", "sample", "stage_seconds",
-                                             "one_thread_value", "plastic_fraction", "ms_per_step")},
+        "cpu_baseline": cpu if "unavailable" in cpu else {
+            k: cpu[k] for k in ("value", "unit", "cores", "kind", "sample", "stage_seconds",
+                                "one_thread_value", "plastic_fraction", "ms_per_step")},
         "plain_fp64_roofline": plain_roofline(n, nb, ref["ms_per_step"], peak),
         "e2e": {"value": job_throughput(n, total, e2e_s * 1e3, world), "unit": UNIT,
                 "h2d_bytes_per_step": h2d / total, "d2h_bytes_per_step": d2h / total,
