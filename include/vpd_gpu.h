@@ -246,7 +246,8 @@ int vpd_checkpoint_load(vpd_handle *h, const void *buffer, int64_t bytes);
 
 /* Sorted neighbour lists of n points (positions n*3 doubles). First call with col == NULL:
    fills row_ptr[n+1] and *total. Second call with col of *total ints fills the rows. Both
-   calls synchronise the stream. Scratch memory is allocated and freed internally. */
+   calls synchronise the stream. Scratch memory, here and below, comes from a stream-ordered pool
+   of the library, which keeps at most 256 MiB idle per device until the next vpd_destroy. */
 int vpd_build_neighbor_list(const double *positions, int64_t n, double horizon,
                             int64_t *row_ptr, int32_t *col, int64_t *total, void *stream);
 int vpd_shape_tensor_inverse(const double *positions, const double *volumes, int64_t n,

@@ -247,7 +247,14 @@ namespace {
 
 template <typename T> int dalloc(vpd_handle *h, T **p, size_t count) {
   void *q = nullptr;
-  VPD_CUDA(cudaMalloc(&q, std::max<size_t>(count, 1) * sizeof(T)));
+  const size_t bytes = std::max<size_t>(count, 1) * sizeof(T);
+  cudaError_t e = cudaMalloc(&q, bytes);
+  if (e == cudaErrorMemoryAllocation) {  // again without the memory the workspace pool holds idle
+    cudaGetLastError();
+    workspace_trim();
+    e = cudaMalloc(&q, bytes);
+  }
+  VPD_CUDA(e);
   h->allocations.push_back(q);
   *p = static_cast<T *>(q);
   return VPD_OK;

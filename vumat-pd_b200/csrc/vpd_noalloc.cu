@@ -4,9 +4,9 @@
 // Some hosts cannot call cudaMalloc while they run a time step: a solver that hands all of
 // the device memory to its own pool before the run starts, or a step loop that drives other
 // streams concurrently and cannot accept the device-wide synchronisation cudaMalloc and
-// cudaFree imply. vpd_force_density allocates its force-map scratch (9 doubles per point)
-// and a status word on every call; this variant uses a fixed scratch array compiled into the
-// library instead, so it allocates nothing. The caller still passes every input and output.
+// cudaFree imply. vpd_force_density takes its force-map scratch (9 doubles per point) from the
+// library's memory pool, which grows by allocating; this variant uses a fixed scratch array compiled
+// into the library instead, so it allocates nothing. The caller still passes every input and output.
 //
 // Limits and sharing:
 //   * at most kNoAllocMaxPoints = 65,536 points per call; larger calls are rejected with
