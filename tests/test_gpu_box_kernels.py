@@ -70,3 +70,20 @@ def test_plane_split_mixed_kernels_match_bitwise(monkeypatch, dims, ratio, damag
     for kind in ("planes", ""):
         for f, want in out["pair"].items():
             assert np.array_equal(out[kind][f], want), (kind, f)
+
+
+# the thread-per-tile mixed kernels' block shapes against the plane split: one wave of 128 threads, one of 192, between two
+# and three waves, above three (192 threads for the force, 256 for the damaged deformation)
+@pytest.mark.parametrize("dims", [(500, 16, 16), (97, 43, 37), (200, 40, 45), (260, 50, 50)])
+@pytest.mark.parametrize("damage", [0, 1])
+def test_pair_shapes_match_plane_split_bitwise(monkeypatch, dims, damage):
+    nx, ny, nz = dims
+    case = tensile_bar(3, nx=nx, ny=ny, nz=nz, damage_mode=damage, damage_initiation=0.004, precision=PRECISION_MIXED)
+    out = {}
+    for kind in ("pair", "planes"):
+        monkeypatch.setenv("VPD_BOND_KERNEL", kind)
+        with vpd.Simulation(case) as sim:
+            sim.step(60)
+            out[kind] = {f: sim.field(f) for f in ("displacement", "force_density", "damage_index")}
+    for f, want in out["pair"].items():
+        assert np.array_equal(out["planes"][f], want), f

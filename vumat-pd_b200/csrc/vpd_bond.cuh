@@ -4,6 +4,8 @@
 #include "vpd_math.cuh"
 #include "vpd_step.cuh"
 
+#include <cmath>
+
 namespace vpd {
 
 __device__ __forceinline__ float4 ldgf4(const float4 *p) { return __ldg(p); }
@@ -160,6 +162,22 @@ template <int kTileP, int kThreads> static unsigned tiled_blocks(const StepParam
   const int64_t threads = (int64_t)p.lat_nx * ((p.lat_ny + kTileP - 1) / kTileP) * p.lat_nz;
   return (unsigned)((threads + kThreads - 1) / kThreads);
 }
+
+// Waves of a grid of one thread per P points, threads_per_sm of them resident, and their cost in full waves: a last
+// one that is partly filled takes a third of a full one and more as it fills.
+template <int P> static double tile_waves(const StepParams &p, int threads_per_sm) {
+  return (double)p.lat_nx * ((p.lat_ny + P - 1) / P) * p.lat_nz / (148.0 * threads_per_sm);
+}
+static inline double wave_cost(double waves) {
+  const double full = std::floor(waves), part = waves - full;
+  return full + (part > 0.0 ? 0.33 + 0.67 * std::sqrt(part) : 0.0);
+}
+
+// Where the last of one or two waves of 16 warps per SM is over three quarters full, blocks of 128 threads leave no SM
+// less loaded than blocks of 256 do, and a block of 256 keeps neighbouring halves in one L1: 2 % of an increment at
+// 128,000 points, 1 % at 270,000. (Otherwise the smaller blocks spread better: 3 to 10 % of a kernel at 100,000 and
+// 400,000.)
+static inline bool halves_together(double waves) { return waves <= 2.0 && waves - (std::ceil(waves) - 1.0) > 0.76; }
 
 // 32-bit window indices need every index within a stencil reach of the lattice below 2^31
 static inline bool index32(const StepParams &p) { return p.n < (int64_t(1) << 30); }

@@ -79,7 +79,6 @@ struct StepParams {
   const int64_t *slice_off;   // sliced-ELL slice offsets
   const int32_t *sell;        // sliced-ELL neighbour indices
   uint32_t *words;            // broken-bond bits, one word per (slice, column)
-  StencilLayout st;           // lattice-stencil layout; used instead of the ELL when st.nw > 0
   int lat_nx, lat_ny, lat_nz; // the lattice (points in index order (x ny + y) nz + z)
   double lat_h;               // lattice spacing
   int tiled;                  // bond kernels (VPD_BOND_KERNEL): 0 per slot, 2 by precision and size; mixed 1 tiled
@@ -98,9 +97,6 @@ struct StepParams {
   // fmap[r * n + i] = (VM_r0, VM_r1, VM_r2, X_r), so one bond reads three 32-byte records
   double4 *fmap;
   double4 *vxi;               // sum over all bonds of V_j xi (FP64, set once; stencil layout)
-  BoxTiles box;               // the small-lattice FP64 kernels' boxes
-  StagedTiles staged;         // the TMA-staged FP64 force kernel's tiles and box
-  CUtensorMap fmap_tmap;      // ... and its tensor map over fmap (lane, z, y, x, row)
   // mixed precision (VPD_PRECISION_MIXED): FP32 copies gathered by the bond kernels
   int mixed;
   // mixed precision: jit, uf and fmapf carry st.halo zero records before and after their n
@@ -147,6 +143,11 @@ struct StepParams {
   int mat_blocks;
   // diagnostic constants
   double interior, gauge, lat_gauge, area, sign, n_lat_pos, n_lat_neg;
+  // bond layouts and tiles
+  StencilLayout st;           // lattice-stencil layout; used instead of the ELL when st.nw > 0
+  BoxTiles box;               // the small-lattice FP64 kernels' boxes
+  StagedTiles staged;         // the TMA-staged FP64 force kernel's tiles and box
+  CUtensorMap fmap_tmap;      // ... and its tensor map over fmap (lane, z, y, x, row)
 };
 
 // The increment's kernels, in order: deformation (+ bond breaking), material, force bond sum,

@@ -703,7 +703,6 @@ __global__ void __launch_bounds__(THREADS, MINB) k_deformation_planes(const __gr
 // lanes, and row 2 is three scalar ones; no neighbour value is copied to both lanes of a pair.
 // Point q's offsets from the group's window position 0, o - J_q, on both lanes of a pair
 // (ey at window position t adds t h):
-constexpr int kForcePairThreads = 192;
 struct ForceOffsets {
   float2 ex[2], ey[2], ez[2];
 };
@@ -859,11 +858,8 @@ __device__ __forceinline__ void force_pair_finish(const StepParams &p, int64_t i
 }
 
 // f = sum (V_j M_j) xi over intact bonds + M_i s_i with s_i = vxi_i - sum_{broken j} V_j xi.
-// Three blocks of 192 threads per SM (up to 112 registers, no spills): on the 1M-point bar 0.373 ms, as two blocks of
-// 256, against 0.393 at three blocks of those (80 registers and spills); 154,000 points fit one wave of it
-// (75 against 98 us).
-template <bool DAMAGE, bool UNROLL>
-__global__ void __launch_bounds__(kForcePairThreads, 3) k_force_pair(const __grid_constant__ StepParams p) {
+template <bool DAMAGE, bool UNROLL, int TPB, int MINB>
+__global__ void __launch_bounds__(TPB, MINB) k_force_pair(const __grid_constant__ StepParams p) {
   const float h = (float)p.lat_h;
   const PairTile tile = pair_tile(p, (int64_t)blockIdx.x * blockDim.x + threadIdx.x);
   float jx[2], jy[2], jz[2];
@@ -940,9 +936,12 @@ __global__ void __launch_bounds__(THREADS, MINB) k_force_planes(const __grid_con
 // microseconds, a thread per tile | a warp per plane, horizon 4.015 h: 1,600 points 96 | 37, 4,000 99 | 38, 10,605
 // 118 | 48, 20,400 101 | 62, 54,000 106 | 91, 79,360 145 | 139, 108,900 168 | 189; at 3.015 h: 4,000 63 | 34, 54,000
 // 70 | 67, 79,360 95 | 102; with damage at 4.015 h: 4,000 128 | 44, 54,000 138 | 123, 79,360 176 | 189.
-constexpr int64_t kPlanesPoints = 60000;
+// Over thin and thick cross-sections 50,000 points keep 7 % (seven planes) and 20 % (nine) of an increment; 58,000
+// lose 5 % with seven planes and keep 6 % with nine.
+constexpr int64_t kPlanesPoints = 60000, kPlanesPoints7 = 54000;
 static bool by_planes(const StepParams &p) {
-  return p.st.nplanes > 1 && (p.tiled == 5 || (p.tiled != 8 && p.n <= kPlanesPoints));
+  const int64_t most = p.st.nplanes <= 7 ? kPlanesPoints7 : kPlanesPoints;
+  return p.st.nplanes > 1 && (p.tiled == 5 || (p.tiled != 8 && p.n <= most));
 }
 
 // launch(std::integral_constant<int, THREADS>, <int, MINB>) with the bounds that fit a block of nplanes warps: two blocks
@@ -960,18 +959,24 @@ template <typename F> static void with_plane_threads(const StepParams &p, F &&la
 // With damage the scalar deformation kernel keeps the runtime window loop (unrolled, its
 // stretch tests made it slower: 0.28 against 0.25 ms on the 250k-point bar); the packed-pair
 // kernel unrolls its windows with damage too (0.698 against 0.783 ms on the 1M-point bar).
+//
+// Block shapes (16 warps per SM in blocks of 128 or 256 threads, 18 in blocks of 192), microseconds over lattices with
+// cross-sections from 8 x 3 to 50 x 50, 128 | 192 | 256: horizon 3.015 h without damage, 62,000 points 28-30 | 33-35 |
+// 28-30, 154,000 43-49 | 40-44 | 46-52 (one wave of 192), 400,000 81-86 | 91-101 | 86-92, 1M 180-194 | 190-212 |
+// 187-201; with damage 400,000 124-135 | 145-150 | 130-135, 650,000 196-209 | 211-224 | 195-202, 1M 293-312 | 312-335 |
+// 286-299.
 template <bool DAMAGE, bool UNROLL> static void launch_deformation_pair(const StepParams &p, cudaStream_t s) {
-  const int64_t tiles = (int64_t)p.lat_nx * ((p.lat_ny + 1) / 2) * p.lat_nz;
+  const double waves = tile_waves<2>(p, 512);
   if (by_planes(p))
     with_plane_threads(p, [&](auto threads, auto minb) {
       k_deformation_planes<DAMAGE, UNROLL, decltype(threads)::value, decltype(minb)::value>
           <<<tiled_blocks<2, 32>(p), 32 * p.st.nplanes, sizeof(float2) * 9 * 32 * p.st.nplanes, s>>>(p);
     });
-  else if (tiles > 148 * 512 && tiles <= 148 * 576)  // one wave of 18 warps per SM, not of 16: 82 against 87 us
+  else if (waves > 1.01 && tile_waves<2>(p, 576) <= 1.0)
     k_deformation_pair<DAMAGE, UNROLL, 192, 3><<<tiled_blocks<2, 192>(p), 192, 0, s>>>(p);
-  else if (DAMAGE)  // 161 against 165 us in 128-thread blocks at 500,000 points
+  else if (halves_together(waves) || (DAMAGE && waves > 3.0))
     k_deformation_pair<DAMAGE, UNROLL, 256, 2><<<tiled_blocks<2, 256>(p), 256, 0, s>>>(p);
-  else  // 365 against 372 us in 256-thread blocks at 1M points
+  else
     k_deformation_pair<DAMAGE, UNROLL, 128, 4><<<tiled_blocks<2, 128>(p), 128, 0, s>>>(p);
 }
 template <bool UNROLL> static void launch_deformation(const StepParams &p, cudaStream_t s) {
@@ -994,14 +999,23 @@ int launch_deformation_tiled(const StepParams &p, cudaStream_t s) {
   return VPD_OK;
 }
 
+// Blocks of 128 threads, or of 192 where the larger waves (112 registers, 18 warps per SM) cost less: a full one takes
+// 1.1 times as long, 1.2 with damage. Microseconds over the same lattices at horizon 3.015 h, 128 | 192 | 256 threads:
+// without damage 62,000 points 26-32 | 28-36 | 26-32, 154,000 43-69 | 38-48 | 44-71, 260,000 60-80 | 60-88 | 61-81,
+// 400,000 84-117 | 86-127 | 87-118, 650,000 130-181 | 125-170 | 132-188, 1M 185-258 | 180-250 | 191-263; with damage
+// 154,000 46-69 | 42-51 | 47-69, 650,000 135-181 | 138-176 | 138-184, 1M 195-260 | 199-258 | 202-266.
 template <bool DAMAGE, bool UNROLL> static void launch_force_pair(const StepParams &p, cudaStream_t s) {
   if (by_planes(p))
     with_plane_threads(p, [&](auto threads, auto minb) {
       k_force_planes<DAMAGE, UNROLL, decltype(threads)::value, decltype(minb)::value>
           <<<tiled_blocks<2, 32>(p), 32 * p.st.nplanes, sizeof(float2) * 96 * p.st.nplanes, s>>>(p);
     });
+  else if ((DAMAGE ? 1.2 : 1.1) * wave_cost(tile_waves<2>(p, 576)) < wave_cost(tile_waves<2>(p, 512)))
+    k_force_pair<DAMAGE, UNROLL, 192, 3><<<tiled_blocks<2, 192>(p), 192, 0, s>>>(p);
+  else if (halves_together(tile_waves<2>(p, 512)))
+    k_force_pair<DAMAGE, UNROLL, 256, 2><<<tiled_blocks<2, 256>(p), 256, 0, s>>>(p);
   else
-    k_force_pair<DAMAGE, UNROLL><<<tiled_blocks<2, kForcePairThreads>(p), kForcePairThreads, 0, s>>>(p);
+    k_force_pair<DAMAGE, UNROLL, 128, 4><<<tiled_blocks<2, 128>(p), 128, 0, s>>>(p);
 }
 
 int launch_force_tiled(const StepParams &p, cudaStream_t s) {

@@ -301,13 +301,6 @@ __global__ void __launch_bounds__(TPB, MINB) k_force_tiled64(const __grid_consta
 // (207), 250,000 293 | 260 | 317 (270), 1M 982 | 894 | 933 (896).
 // Force (1 x 128 four blocks per SM | 3 x 128 three | 3 x 384 one, the one shape before): 20,400 points 48 | 67 |
 // 108, 40,900 64 | 67 | 105, 54,000 69 | 67 | 101, 108,900 161 | 93 | 106, 154,000 189 | 125 | 113, 1M 1077 | 689 | 617.
-template <int P> static double tile_waves(const StepParams &p, int threads_per_sm) {
-  return (double)p.lat_nx * ((p.lat_ny + P - 1) / P) * p.lat_nz / (148.0 * threads_per_sm);
-}
-static double wave_cost(double waves) {
-  const double full = std::floor(waves), part = waves - full;
-  return full + (part > 0.0 ? 0.33 + 0.67 * std::sqrt(part) : 0.0);
-}
 
 // With damage the groups with live bonds keep the runtime window loop (unrolled, the FP64 stretch
 // tests spill about 1 KB per thread and the kernel slowed from 0.96 to 1.29 ms at 1M points); the
@@ -329,6 +322,8 @@ int launch_deformation_tiled64(const StepParams &p, cudaStream_t s) {
   const double three = (p.damage ? 1.25 : 1.11) * std::ceil(tile_waves<3>(p, 384));
   if (one <= (p.damage ? 1.0 : 0.75))
     deformation_tiled64<1, 128, 6>(p, s);
+  else if (two <= three && halves_together(tile_waves<2>(p, 512)))
+    deformation_tiled64<2, kBondThreads, 2>(p, s);
   else if (two <= three)
     deformation_tiled64<2, 128, 4>(p, s);
   else
