@@ -642,7 +642,10 @@ static int launch_cells(const double4 *xv, const NeighborGrid &grid, const Neigh
   const CellSearch cs{inv, grid.dist2_max, (float)(r2 * (1.0 - 2.0e-5)), (float)(r2 * (1.0 + 2.0e-5))};
   const int width = cell_width(grid.candidates);
   const size_t smem = cell_smem(width);
-  VPD_CUDA(cudaFuncSetAttribute(k_nb_cell<FILL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  // the largest search's amount, whatever this one's: the attribute is the function's, and another thread's call may
+  // set it between this one's and its launch
+  VPD_CUDA(cudaFuncSetAttribute(k_nb_cell<FILL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)cell_smem(kMaxCandidates)));
   k_nb_cell<FILL><<<(unsigned)grid.ncells, kCellThreads, smem, s>>>(xv, g, scr.cell_start, scr.sorted, cs, width, row_ptr,
                                                                     col, scr.len, scr.reduce);
   VPD_CUDA(cudaGetLastError());
