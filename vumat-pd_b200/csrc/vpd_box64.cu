@@ -273,7 +273,10 @@ constexpr int kBoxMaxRecords = 2304;
 
 // The boxes of a lattice: the extents whose tiles need the fewest waves of 148 blocks, then the
 // smallest staged regions, of at most 32 points (one block per SM up to 4,736 points), 64 or 128
-// (more points per staged region where several blocks would queue per SM anyway).
+// (more points per staged region where several blocks would queue per SM anyway). Boxes that need a second wave are
+// not taken (unless asked for, p.tiled 7): a long reach leaves room for a few points beside it in a region, and each
+// box stages it again. Per increment in microseconds, boxes | tiles: one wave, 10,605 points at 4.5 h, 118 | 112; two,
+// 9,000 points at 5 h, 175 | 99; twelve, 4,913 points at 5 h, 877 | 148.
 int setup_box64(StepParams &p) {
   p.box = BoxTiles{};
   const int points = p.n <= 148 * 32 ? 32 : (p.n <= 148 * 48 ? 64 : 128);
@@ -294,6 +297,8 @@ int setup_box64(StepParams &p) {
         if (!p.box.threads || cost < best)
           best = cost, p.box = b;
       }
+  if (p.box.tiles > 148 && p.tiled != 7)
+    p.box = BoxTiles{};
   if (!p.box.threads)
     return VPD_OK;
   return with_records(p.box.records, [&](auto m) {
