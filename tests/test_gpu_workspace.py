@@ -1,0 +1,116 @@
+"""Device memory of the module functions: what allocates and what does not, under capture too, and how much of it
+stays with the library."""
+import ctypes
+
+import numpy as np
+import pytest
+
+import vpd
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+def cuda(a, dtype=torch.float64):
+    return torch.as_tensor(np.ascontiguousarray(a)).to(dtype=dtype, device="cuda").contiguous()
+
+
+class Step:
+    """A ring of n points, each bonded to the next six, and the calls of an increment on it into buffers of its own."""
+
+    def __init__(self, n):
+        rng = np.random.default_rng(n)
+        self.n = n
+        self.pos, self.disp = cuda(rng.standard_normal((n, 3))), cuda(0.01 * rng.standard_normal((n, 3)))
+        self.vol = cuda(0.5 + rng.random(n))
+        self.row_ptr = cuda(6 * np.arange(n + 1), torch.int64)
+        self.col = cuda((np.arange(n)[:, None] + np.arange(1, 7)) % n, torch.int32)
+        self.kinv, self.F = torch.empty((n, 9), dtype=torch.float64, device="cuda"), cuda(np.tile(np.eye(3).ravel(), (n, 1)))
+        self.sigma = cuda(rng.standard_normal((n, 9)))
+        self.bond = torch.zeros(6 * n, dtype=torch.float64, device="cuda")
+        self.index = torch.zeros(n, dtype=torch.float64, device="cuda")
+        self.force = torch.zeros((n, 3), dtype=torch.float64, device="cuda")
+        torch.cuda.synchronize()
+
+    def call(self, name, *args):
+        a = [vpd._ptr(v) if torch.is_tensor(v) else v for v in args]
+        vpd._check(getattr(vpd.library(), name)(*a, vpd._stream()))
+
+    def shape(self):
+        self.call("vpd_shape_tensor_inverse", self.pos, self.vol, self.n, self.row_ptr, self.col, self.kinv)
+
+    def deformation(self):
+        self.call("vpd_deformation_gradients", self.pos, self.disp, self.vol, self.n, self.row_ptr, self.col, self.kinv,
+                  self.F)
+
+    def damage(self):
+        self.call("vpd_damage_update", self.pos, self.disp, self.vol, self.n, self.row_ptr, self.col, 0.005, 0.0,
+                  self.bond, self.index)
+
+    def noalloc_force(self):
+        self.call("vpd_force_density_noalloc", self.pos, self.vol, self.n, self.row_ptr, self.col, self.kinv, self.F,
+                  self.sigma, self.bond, self.force)
+
+
+def free_bytes():
+    torch.cuda.synchronize()
+    return torch.cuda.mem_get_info()[0]
+
+
+def loaded():
+    """Every kernel of the step's calls loaded (CUDA loads them lazily)."""
+    for n in (64, 60_000):
+        body = Step(n)
+        body.shape(), body.deformation(), body.damage(), body.noalloc_force()
+
+
+@pytest.mark.parametrize("n", [65536, 151_000])
+def test_the_calls_of_an_increment_allocate_nothing(n):
+    """For hosts that hand all device memory to their own pool (vpd_force_density_noalloc: up to 65,536 points)."""
+    loaded()
+    body = Step(n)
+    before = free_bytes()
+    body.shape(), body.deformation(), body.damage()
+    if n <= 65536:
+        body.noalloc_force()
+    assert free_bytes() == before
+
+
+def test_captured_calls_hold_kernels_only():
+    """The two calls that do not synchronise, at a size where packed records pay."""
+    body = Step(151_000)
+    body.shape(), body.deformation(), body.damage()
+    torch.cuda.synchronize()
+    want = body.F.clone(), body.bond.clone(), body.index.clone()
+    body.F.zero_(), body.bond.zero_(), body.index.zero_()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        body.deformation(), body.damage()
+    driver = ctypes.CDLL("libcuda.so.1")
+    count = ctypes.c_size_t()
+    raw = ctypes.c_void_p(graph.raw_cuda_graph())
+    assert driver.cuGraphGetNodes(raw, None, ctypes.byref(count)) == 0
+    nodes = (ctypes.c_void_p * count.value)()
+    assert driver.cuGraphGetNodes(raw, nodes, ctypes.byref(count)) == 0
+    kinds = []
+    for node in nodes:
+        kind = ctypes.c_int()
+        assert driver.cuGraphNodeGetType(ctypes.c_void_p(node), ctypes.byref(kind)) == 0
+        kinds.append(kind.value)
+    graph.instantiate()
+    graph.replay()
+    torch.cuda.synchronize()
+    for got, expected in zip((body.F, body.bond, body.index), want):
+        assert torch.equal(got, expected)
+    assert kinds and set(kinds) == {0}  # CU_GRAPH_NODE_TYPE_KERNEL
+
+
+def test_records_must_lie_on_a_32_byte_boundary():
+    body = Step(64)
+    records = torch.empty(8 * body.n + 4, dtype=torch.float64, device="cuda")
+    for bad in (None, ctypes.c_void_p(records.data_ptr() + 8)):
+        with pytest.raises(vpd.VpdError) as e:
+            body.call("vpd_shape_tensor_inverse_packed", body.pos, body.vol, body.n, body.row_ptr, body.col, body.kinv, bad)
+        assert e.value.status == 1
+
+

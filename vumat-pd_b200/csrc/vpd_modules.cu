@@ -72,8 +72,8 @@ template <typename F> __device__ __forceinline__ void for_row(const RowPoint &r,
   }
 }
 
-// Where the bond sums read the points: the caller's arrays, or 32-byte records packed in temporary memory
-// first, one load per vector.
+// Where the bond sums read the points: the caller's arrays, or 32-byte records packed into memory of the caller's
+// first (the entry points with records), one load per vector.
 struct PointsPlain {
   const double *pos, *vol;
   __device__ __forceinline__ double4 xv(int64_t j) const {
@@ -108,11 +108,11 @@ __global__ void k_pack_points(const double *pos, const double *vol, const double
     st256(vec + i, VectorsPlain<CURRENT>{pos, disp}.at(i));
 }
 
-// From these many points on the records pay for their pass. Calls at horizon 4.015 h, plain | packed:
+// Where the records pay for their pass. Calls at horizon 4.015 h, plain | packed:
 // damage 16,000 points 34 | 30 us, 36,000 73 | 64, 154,000 295 | 238; deformation 36,000 51 | 53, 154,000
-// 203 | 203, 250,000 345 | 324; shape tensors 154,000 165 | 158, 250,000 251 | 226. (Not in the force
+// 203 | 203, 250,000 345 | 324; shape tensors 154,000 165 | 158, 250,000 251 | 226; the same points in no order,
+// 250,000: deformation 955 | 485, shape tensors 611 | 305. (Not in the force
 // sum: its nine words of M a bond outweigh the four of the point, 644 | 659 us at 250,000.)
-constexpr int64_t kPackDamage = 16000, kPackSums = 150000;
 
 // PdCorrespondenceSkeleton::initialize (:149-170)
 template <typename Points>
@@ -520,6 +520,73 @@ int launch_csr_force(const double *positions, const double *volumes, int64_t n, 
   return VPD_OK;
 }
 
+// The bond sums of the entry points, with or without room for packed records.
+static int check_records(const double *records, const char *entry) {
+  if (!records || (reinterpret_cast<uintptr_t>(records) & 31))
+    return set_error(VPD_ERR_INVALID, std::string(entry) + ": needs records on a 32-byte boundary");
+  return VPD_OK;
+}
+
+static int shape_tensor_inverse(const double *positions, const double *volumes, int64_t n, const int64_t *row_ptr,
+                                const int32_t *col, double *kinv, double4 *rec, cudaStream_t s) {
+  unsigned *st = thread_status();
+  if (!st)
+    return set_error(VPD_ERR_CUDA, "status word allocation failed");
+  if (n <= 0)
+    return VPD_OK;
+  VPD_CUDA(cudaMemsetAsync(st, 0, sizeof(unsigned), s));
+  if (rec) {
+    k_pack_points<false><<<blocks(n), 128, 0, s>>>(positions, volumes, nullptr, n, rec, nullptr);
+    k_csr_shape_inverse<<<row_blocks(n), kRowThreads, 0, s>>>(Packed{rec}, n, row_ptr, col, kinv, st);
+  } else {
+    k_csr_shape_inverse<<<row_blocks(n), kRowThreads, 0, s>>>(PointsPlain{positions, volumes}, n, row_ptr, col, kinv,
+                                                              st);
+  }
+  VPD_CUDA(cudaGetLastError());
+  return check_status(st, s);
+}
+
+static int deformation_gradients(const double *positions, const double *displacement, const double *volumes, int64_t n,
+                                 const int64_t *row_ptr, const int32_t *col, const double *kinv, double *defgrad,
+                                 double4 *rec, cudaStream_t s) {
+  if (n <= 0)
+    return VPD_OK;
+  if (rec) {
+    k_pack_points<false><<<blocks(n), 128, 0, s>>>(positions, volumes, displacement, n, rec, rec + n);
+    k_csr_deformation<<<row_blocks(n), kRowThreads, 0, s>>>(Packed{rec}, Packed{rec + n}, n, row_ptr, col, kinv,
+                                                            defgrad);
+  } else {
+    k_csr_deformation<<<row_blocks(n), kRowThreads, 0, s>>>(PointsPlain{positions, volumes},
+                                                            VectorsPlain<false>{positions, displacement}, n, row_ptr,
+                                                            col, kinv, defgrad);
+  }
+  VPD_CUDA(cudaGetLastError());
+  return VPD_OK;
+}
+
+static int damage_update(const double *positions, const double *displacement, const double *volumes, int64_t n,
+                         const int64_t *row_ptr, const int32_t *col, double initiation, double failure,
+                         double *bond_damage, double *damage_index, double4 *rec, cudaStream_t s) {
+  if (!(initiation > 0.0))
+    return set_error(VPD_ERR_INVALID, "critical_stretch requires initiation > 0.");
+  if (n <= 0)
+    return VPD_OK;
+  const int use_compression = failure > 0.0 && std::isfinite(failure);
+  const StretchTest test{initiation, failure, (1.0 + initiation) * (1.0 + initiation),
+                         failure < 1.0 ? (1.0 - failure) * (1.0 - failure) : 0.0, use_compression};
+  if (rec) {
+    k_pack_points<true><<<blocks(n), 128, 0, s>>>(positions, volumes, displacement, n, rec, rec + n);
+    k_csr_damage<<<row_blocks(n), kRowThreads, 0, s>>>(Packed{rec}, Packed{rec + n}, n, row_ptr, col, test,
+                                                       bond_damage, damage_index);
+  } else {
+    k_csr_damage<<<row_blocks(n), kRowThreads, 0, s>>>(PointsPlain{positions, volumes},
+                                                       VectorsPlain<true>{positions, displacement}, n, row_ptr, col,
+                                                       test, bond_damage, damage_index);
+  }
+  VPD_CUDA(cudaGetLastError());
+  return VPD_OK;
+}
+
 }  // namespace vpd
 
 using namespace vpd;
@@ -557,51 +624,29 @@ int vpd_build_neighbor_list(const double *positions, int64_t n, double horizon, 
 
 int vpd_shape_tensor_inverse(const double *positions, const double *volumes, int64_t n,
                              const int64_t *row_ptr, const int32_t *col, double *kinv, void *stream) {
-  cudaStream_t s = (cudaStream_t)stream;
-  unsigned *st = thread_status();
-  if (!st)
-    return set_error(VPD_ERR_CUDA, "status word allocation failed");
-  if (n <= 0)
-    return VPD_OK;
-  VPD_CUDA(cudaMemsetAsync(st, 0, sizeof(unsigned), s));
-  Workspace ws(s);
-  if (n >= kPackSums) {
-    double4 *rec = nullptr;
-    const int rc = ws.alloc(&rec, n);
-    if (rc)
-      return rc;
-    k_pack_points<false><<<blocks(n), 128, 0, s>>>(positions, volumes, nullptr, n, rec, nullptr);
-    k_csr_shape_inverse<<<row_blocks(n), kRowThreads, 0, s>>>(Packed{rec}, n, row_ptr, col, kinv, st);
-  } else {
-    k_csr_shape_inverse<<<row_blocks(n), kRowThreads, 0, s>>>(PointsPlain{positions, volumes}, n, row_ptr, col, kinv,
-                                                              st);
-  }
-  VPD_CUDA(cudaGetLastError());
-  return check_status(st, s);
+  return shape_tensor_inverse(positions, volumes, n, row_ptr, col, kinv, nullptr, (cudaStream_t)stream);
+}
+int vpd_shape_tensor_inverse_packed(const double *positions, const double *volumes, int64_t n, const int64_t *row_ptr,
+                                    const int32_t *col, double *kinv, double *records, void *stream) {
+  const int rc = check_records(records, "vpd_shape_tensor_inverse_packed");
+  return rc ? rc
+            : shape_tensor_inverse(positions, volumes, n, row_ptr, col, kinv, reinterpret_cast<double4 *>(records),
+                                   (cudaStream_t)stream);
 }
 
 int vpd_deformation_gradients(const double *positions, const double *displacement, const double *volumes,
                               int64_t n, const int64_t *row_ptr, const int32_t *col, const double *kinv,
                               double *defgrad, void *stream) {
-  if (n <= 0)
-    return VPD_OK;
-  cudaStream_t s = (cudaStream_t)stream;
-  Workspace ws(s);
-  if (n >= kPackSums) {
-    double4 *rec = nullptr;
-    const int rc = ws.alloc(&rec, 2 * n);
-    if (rc)
-      return rc;
-    k_pack_points<false><<<blocks(n), 128, 0, s>>>(positions, volumes, displacement, n, rec, rec + n);
-    k_csr_deformation<<<row_blocks(n), kRowThreads, 0, s>>>(Packed{rec}, Packed{rec + n}, n, row_ptr, col, kinv,
-                                                            defgrad);
-  } else {
-    k_csr_deformation<<<row_blocks(n), kRowThreads, 0, s>>>(PointsPlain{positions, volumes},
-                                                            VectorsPlain<false>{positions, displacement}, n, row_ptr,
-                                                            col, kinv, defgrad);
-  }
-  VPD_CUDA(cudaGetLastError());
-  return VPD_OK;
+  return deformation_gradients(positions, displacement, volumes, n, row_ptr, col, kinv, defgrad, nullptr,
+                               (cudaStream_t)stream);
+}
+int vpd_deformation_gradients_packed(const double *positions, const double *displacement, const double *volumes,
+                                     int64_t n, const int64_t *row_ptr, const int32_t *col, const double *kinv,
+                                     double *defgrad, double *records, void *stream) {
+  const int rc = check_records(records, "vpd_deformation_gradients_packed");
+  return rc ? rc
+            : deformation_gradients(positions, displacement, volumes, n, row_ptr, col, kinv, defgrad,
+                                    reinterpret_cast<double4 *>(records), (cudaStream_t)stream);
 }
 
 int vpd_force_density(const double *positions, const double *volumes, int64_t n, const int64_t *row_ptr,
@@ -693,30 +738,16 @@ int vpd_jc_return_map(int64_t n, const double *props, double dt, const double *s
 int vpd_damage_update(const double *positions, const double *displacement, const double *volumes, int64_t n,
                       const int64_t *row_ptr, const int32_t *col, double initiation, double failure,
                       double *bond_damage, double *damage_index, void *stream) {
-  if (!(initiation > 0.0))
-    return set_error(VPD_ERR_INVALID, "critical_stretch requires initiation > 0.");
-  if (n <= 0)
-    return VPD_OK;
-  const int use_compression = failure > 0.0 && std::isfinite(failure);
-  const StretchTest test{initiation, failure, (1.0 + initiation) * (1.0 + initiation),
-                         failure < 1.0 ? (1.0 - failure) * (1.0 - failure) : 0.0, use_compression};
-  cudaStream_t s = (cudaStream_t)stream;
-  Workspace ws(s);
-  if (n >= kPackDamage) {
-    double4 *rec = nullptr;
-    const int rc = ws.alloc(&rec, 2 * n);
-    if (rc)
-      return rc;
-    k_pack_points<true><<<blocks(n), 128, 0, s>>>(positions, volumes, displacement, n, rec, rec + n);
-    k_csr_damage<<<row_blocks(n), kRowThreads, 0, s>>>(Packed{rec}, Packed{rec + n}, n, row_ptr, col, test,
-                                                       bond_damage, damage_index);
-  } else {
-    k_csr_damage<<<row_blocks(n), kRowThreads, 0, s>>>(PointsPlain{positions, volumes},
-                                                       VectorsPlain<true>{positions, displacement}, n, row_ptr, col,
-                                                       test, bond_damage, damage_index);
-  }
-  VPD_CUDA(cudaGetLastError());
-  return VPD_OK;
+  return damage_update(positions, displacement, volumes, n, row_ptr, col, initiation, failure, bond_damage,
+                       damage_index, nullptr, (cudaStream_t)stream);
+}
+int vpd_damage_update_packed(const double *positions, const double *displacement, const double *volumes, int64_t n,
+                             const int64_t *row_ptr, const int32_t *col, double initiation, double failure,
+                             double *bond_damage, double *damage_index, double *records, void *stream) {
+  const int rc = check_records(records, "vpd_damage_update_packed");
+  return rc ? rc
+            : damage_update(positions, displacement, volumes, n, row_ptr, col, initiation, failure, bond_damage,
+                            damage_index, reinterpret_cast<double4 *>(records), (cudaStream_t)stream);
 }
 
 void vumat_adapter_call(int *nblock, int *ndir, int *nshr, int *nstatev, int *nfieldv, int *nprops,

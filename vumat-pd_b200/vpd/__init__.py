@@ -80,6 +80,8 @@ def library():
     lib.vpd_build_neighbor_list.argtypes = [_VP, ctypes.c_int64, ctypes.c_double, _VP, _VP, _I64, _VP]
     lib.vpd_shape_tensor_inverse.argtypes = [_VP, _VP, ctypes.c_int64, _VP, _VP, _VP, _VP]
     lib.vpd_deformation_gradients.argtypes = [_VP, _VP, _VP, ctypes.c_int64, _VP, _VP, _VP, _VP, _VP]
+    lib.vpd_shape_tensor_inverse_packed.argtypes = lib.vpd_shape_tensor_inverse.argtypes + [_VP]
+    lib.vpd_deformation_gradients_packed.argtypes = lib.vpd_deformation_gradients.argtypes + [_VP]
     lib.vpd_force_density.argtypes = [_VP, _VP, ctypes.c_int64, _VP, _VP, _VP, _VP, _VP, _VP, _VP, _VP]
     lib.vpd_force_density_noalloc.argtypes = [_VP, _VP, ctypes.c_int64, _VP, _VP, _VP, _VP, _VP,
                                               _VP, _VP, _VP]
@@ -90,6 +92,7 @@ def library():
                                       ctypes.c_int32, _VP, _VP, _VP, _VP]
     lib.vpd_damage_update.argtypes = [_VP, _VP, _VP, ctypes.c_int64, _VP, _VP, ctypes.c_double,
                                       ctypes.c_double, _VP, _VP, _VP]
+    lib.vpd_damage_update_packed.argtypes = lib.vpd_damage_update.argtypes + [_VP]
     lib.vpd_mlp_forward.argtypes = [_VP, _VP, _VP, ctypes.c_int64, _VP, _VP]
     lib.vpd_surrogate_samples.argtypes = [_D, ctypes.c_uint64, ctypes.c_int64, _VP, _VP, _VP]
     lib.vpd_train_surrogate.argtypes = [ctypes.POINTER(SurrogateConfig), _VP, _VP,
@@ -321,20 +324,37 @@ def build_neighbor_list(positions, horizon: float):
     return row_ptr, col[: total.value]
 
 
+def _records(positions, vectors, points):
+    """Room for the packed records of a bond sum over `vectors` vectors a point, for bodies of `points` points or
+    more: None for smaller ones and where there is no memory (the sums then read the arrays as they are)."""
+    import torch
+    n = positions.shape[0]
+    if n < points:
+        return None
+    try:
+        return torch.empty((vectors * n, 4), dtype=torch.float64, device=positions.device)
+    except torch.OutOfMemoryError:
+        return None
+
+
 def shape_tensor_inverse(positions, volumes, row_ptr, col):
     import torch
     out = torch.empty((positions.shape[0], 9), dtype=torch.float64, device=positions.device)
-    _check(library().vpd_shape_tensor_inverse(_ptr(positions), _ptr(volumes), positions.shape[0],
-                                              _ptr(row_ptr), _ptr(col), _ptr(out), _stream()))
+    args = (_ptr(positions), _ptr(volumes), positions.shape[0], _ptr(row_ptr), _ptr(col), _ptr(out))
+    records = _records(positions, 1, 150_000)
+    _check(library().vpd_shape_tensor_inverse(*args, _stream()) if records is None else
+           library().vpd_shape_tensor_inverse_packed(*args, _ptr(records), _stream()))
     return out
 
 
 def deformation_gradients(positions, displacement, volumes, row_ptr, col, kinv):
     import torch
     out = torch.empty((positions.shape[0], 9), dtype=torch.float64, device=positions.device)
-    _check(library().vpd_deformation_gradients(_ptr(positions), _ptr(displacement), _ptr(volumes),
-                                               positions.shape[0], _ptr(row_ptr), _ptr(col),
-                                               _ptr(kinv), _ptr(out), _stream()))
+    args = (_ptr(positions), _ptr(displacement), _ptr(volumes), positions.shape[0], _ptr(row_ptr), _ptr(col),
+            _ptr(kinv), _ptr(out))
+    records = _records(positions, 2, 150_000)
+    _check(library().vpd_deformation_gradients(*args, _stream()) if records is None else
+           library().vpd_deformation_gradients_packed(*args, _ptr(records), _stream()))
     return out
 
 
@@ -430,7 +450,9 @@ def damage_update(positions, displacement, volumes, row_ptr, col, initiation, fa
                   bond_damage):
     import torch
     idx = torch.empty(positions.shape[0], dtype=torch.float64, device=positions.device)
-    _check(library().vpd_damage_update(_ptr(positions), _ptr(displacement), _ptr(volumes),
-                                       positions.shape[0], _ptr(row_ptr), _ptr(col), initiation,
-                                       failure, _ptr(bond_damage), _ptr(idx), _stream()))
+    args = (_ptr(positions), _ptr(displacement), _ptr(volumes), positions.shape[0], _ptr(row_ptr), _ptr(col),
+            initiation, failure, _ptr(bond_damage), _ptr(idx))
+    records = _records(positions, 2, 16_000)
+    _check(library().vpd_damage_update(*args, _stream()) if records is None else
+           library().vpd_damage_update_packed(*args, _ptr(records), _stream()))
     return idx
