@@ -27,3 +27,38 @@ def test_small_lattice_increment_takes_at_most_half_as_long_again_as_the_tiles(m
             sim.step(32)
             best[kind] = min((sim.step(32), sim.last_step_ms())[1] for _ in range(5))
     assert best[""] <= 1.5 * best["tiles"]
+
+
+def seconds(call, count=20):
+    for _ in range(3):
+        call()
+    best = float("inf")
+    for _ in range(5):
+        torch.cuda.synchronize()
+        start = time.perf_counter()
+        for _ in range(count):
+            call()
+        torch.cuda.synchronize()
+        best = min(best, (time.perf_counter() - start) / count)
+    return best
+
+
+# a large body with a few bonds a point: all but the row's lengths and indices is a pass over memory
+@pytest.mark.parametrize("bonds", [4, 8, 18])
+def test_bond_sums_over_short_rows_take_at_most_four_times_a_copy(bonds):
+    n = 1_000_000
+    pos, disp = (torch.randn((n, 3), dtype=torch.float64, device="cuda") for _ in range(2))
+    vol = torch.rand(n, dtype=torch.float64, device="cuda") + 0.5
+    row_ptr = bonds * torch.arange(n + 1, dtype=torch.int64, device="cuda")
+    col = (torch.arange(n, dtype=torch.int32, device="cuda")[:, None] +
+           torch.arange(1, bonds + 1, dtype=torch.int32, device="cuda")).remainder(n).to(torch.int32).reshape(-1).contiguous()
+    kinv = torch.randn((n, 9), dtype=torch.float64, device="cuda")
+    bond = torch.zeros(bonds * n, dtype=torch.float64, device="cuda")
+    # read: rows and their indices, points and displacements; K^-1, F or the bonds' damage and the index
+    deformation = 8 * n + 4 * bonds * n + 56 * n + 144 * n
+    damage = 8 * n + 4 * bonds * n + 56 * n + 8 * bonds * n + 8 * n
+    for moved, call in ((deformation, lambda: vpd.deformation_gradients(pos, disp, vol, row_ptr, col, kinv)),
+                        (damage, lambda: vpd.damage_update(pos, disp, vol, row_ptr, col, 0.5, 0.0, bond))):
+        a = torch.empty(moved // 2, dtype=torch.uint8, device="cuda")
+        b = torch.empty_like(a)
+        assert seconds(call) <= 4.0 * seconds(lambda: b.copy_(a))

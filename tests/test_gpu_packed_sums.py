@@ -1,5 +1,5 @@
-"""The module functions' CSR sums at the sizes where they change to packed point records, against plain NumPy in
-float64: short rows in no order, of another length each."""
+"""The module functions' CSR sums at the sizes and mean row lengths where their lanes per row change and where they
+take packed point records, against plain NumPy in float64: rows in no order, of another length each."""
 import numpy as np
 import pytest
 
@@ -28,9 +28,10 @@ def row_sums(values, row_ptr):
     return np.add.reduceat(values, row_ptr[:-1], axis=0)
 
 
-@pytest.mark.parametrize("n", [39_999, 40_000, 149_999, 150_000, 150_001])
-def test_shape_tensors_and_deformation_gradients(n):
-    rng, pos, vol, row_ptr, owner, col = body(n)
+@pytest.mark.parametrize("n,bonds", [(39_999, 8), (40_000, 8), (40_000, 23), (40_001, 25), (149_999, 8), (150_000, 8),
+                                     (150_001, 19), (150_000, 21), (150_001, 63), (150_000, 65)])
+def test_sums_match_numpy(n, bonds):
+    rng, pos, vol, row_ptr, owner, col = body(n, bonds)
     disp = 0.01 * rng.standard_normal((n, 3))
     xi = pos[col] - pos[owner]
     X, V, P, C = cuda(pos), cuda(vol), cuda(row_ptr, torch.int64), cuda(col, torch.int32)
@@ -40,7 +41,7 @@ def test_shape_tensors_and_deformation_gradients(n):
     assert ok.mean() > 0.5
     got = vpd.shape_tensor_inverse(X, V, P, C).cpu().numpy().reshape(n, 3, 3)
     want = np.linalg.inv(K[ok])
-    # a determinant and cofactors of sums of 11 terms: roundings of some 50 ulp, grown by the condition number twice
+    # a determinant and cofactors of sums of at most 68 terms: roundings of some 50 ulp, grown by the condition number twice
     bound = 50 * 2.0 ** -52 * cond[ok] ** 2 * np.abs(want).max(axis=(1, 2))
     assert (np.abs(got[ok] - want).max(axis=(1, 2)) <= bound).all()
     kinv = rng.standard_normal((n, 9))
@@ -48,12 +49,22 @@ def test_shape_tensors_and_deformation_gradients(n):
     want = np.eye(3) + G @ kinv.reshape(n, 3, 3)
     got = vpd.deformation_gradients(X, cuda(disp), V, P, C, cuda(kinv)).cpu().numpy().reshape(n, 3, 3)
     assert np.abs(got - want).max() <= 1e-12 * max(1.0, np.abs(want).max())
+    F = np.eye(3) + 0.1 * rng.standard_normal((n, 3, 3))
+    sigma = rng.standard_normal((n, 3, 3))
+    bond = np.where(rng.random(len(col)) < 0.3, rng.choice([1.0, 0.25, -1.0, 2.0], len(col)), 0.0)
+    M = np.linalg.det(F)[:, None, None] * sigma @ np.linalg.inv(F).transpose(0, 2, 1) @ kinv.reshape(n, 3, 3)
+    w = (1.0 - np.clip(bond, 0, 1)) * vol[col]
+    want = row_sums(w[:, None] * np.einsum("qab,qb->qa", M[owner] + M[col], xi), row_ptr)
+    got = vpd.force_density(X, V, P, C, cuda(kinv), cuda(F.reshape(n, 9)), cuda(sigma.reshape(n, 9)), cuda(bond))
+    # (a few of the random F are nearly singular: their M is large)
+    assert np.abs(got.cpu().numpy() - want).max() <= 1e-12 * max(1.0, np.abs(M).max() * 70)
 
 
-@pytest.mark.parametrize("n", [15_999, 16_000, 16_001, 40_000, 70_001])
+@pytest.mark.parametrize("n,bonds", [(15_999, 30), (16_000, 23), (16_000, 25), (16_001, 30), (40_000, 8), (40_001, 30),
+                                     (150_001, 8), (150_000, 21), (150_001, 66)])
 @pytest.mark.parametrize("failure", [0.0, 0.01])
-def test_damage_decisions_match_the_reference_formula(n, failure):
-    rng, pos, vol, row_ptr, owner, col = body(n)
+def test_damage_decisions_match_the_reference_formula(n, bonds, failure):
+    rng, pos, vol, row_ptr, owner, col = body(n, bonds)
     eps = 0.02
     # points scaled about the origin, so that stretches straddle the thresholds, some to the last bits
     disp = pos * (eps * (1.0 + 1e-12 * rng.standard_normal((n, 1)))) * rng.choice([1.0, 0.0, -0.6], (n, 1))

@@ -9,6 +9,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 namespace vpd {
@@ -20,53 +21,93 @@ __global__ void k_pack_positions(const double *pos, int64_t n, double4 *xv) {
 }
 
 // ------------------------------------------------------------------ CSR bond sums
-// Eight lanes per point (kRowLanes), each taking every eighth bond of the point's row; a fixed shuffle
-// tree joins the eight partial sums. The lanes of a row read its neighbour indices (and bond damage) as
-// consecutive words, and its sorted neighbours, mostly runs of consecutive points, from a few cache
-// lines; the next bond's index is read before the current bond's gathers are used. With one thread per
-// point every lane of a warp read another row's index, 32 lines per load that L1 could not hold until
-// their next use, and a few thousand points were too few warps.
-// What bounds them now is L1 (93 % of its wavefronts): the gathers of 32 bonds touch about eight lines a
-// load in any arrangement tried (records of 32 bytes, one array per component, lane = point with the
-// indices transposed through shared memory, which jitter misaligns: 1.1 to 1.8 times slower).
-// Kernel times on a B200, one thread per point | now: 154,000 jittered points, horizon 4.015 h (33M bonds): deformation
-// 254 | 200 us, damage 466 | 230, force 732 | 385; 4,000 points at 3.015 h: 28 | 7, 78 | 9, 60 | 11 us.
-constexpr int kRowLanes = 8;
+// A row's bonds are dealt out to 1, 2, 4 or 8 lanes, whose partial sums a fixed shuffle tree joins. Many lanes read a
+// long row's neighbour indices as consecutive words and fill the GPU where points are few; with one lane per row the
+// lanes of a warp share the lines of short rows, and neighbouring rows of a regular lattice gather consecutive points.
+// The next bond's index is read before the current bond's gathers are used. What bounds the sums is L1 (93 % of its
+// wavefronts at 154,000 jittered points): the gathers of 32 bonds touch about eight lines a load in any arrangement
+// tried.
 constexpr int kRowThreads = 256;
 
-static unsigned row_blocks(int64_t n) { return (unsigned)((n * kRowLanes + kRowThreads - 1) / kRowThreads); }
+// Bodies below kLargeBody points take eight lanes a row. From there on the lanes follow the mean row length, which
+// only the device knows without a synchronisation: a grid has threads for four lanes per row, from kLargestBody on for
+// two; threads of fewer lanes than that end at once, those of more pass over two rows. Calls on lattices, microseconds,
+// one lane always | eight always | now: 250,000 points with 4 bonds each, deformation 18 | 47 | 19, damage 14 | 40 | 15,
+// with 28, 38 | 87 | 36 and 73 | 88 | 53; 1M points with 6, 61 | 200 | 63 and 52 | 163 | 52, with 118,
+// 548 | 770 | 533 and 1210 | 838 | 651; 108,000 points with 229, 198 | 133 | 122 and 394 | 169 | 164; the force sum of
+// 1M points with 6, eight always | now, 263 | 145.
+constexpr int64_t kLargeBody = 40000, kLargestBody = 150000;
+__device__ __forceinline__ int row_lanes(int64_t n, const int64_t *row_ptr) {
+  const int64_t bonds = __ldg(row_ptr + n) - __ldg(row_ptr);
+  if (n < kLargestBody)
+    return bonds < 24 * n ? 2 : 4;
+  return bonds < 20 * n ? 1 : (bonds < 64 * n ? 2 : 4);
+}
+static unsigned row_blocks(int64_t n) {
+  const int64_t lanes = n < kLargeBody ? 8 : (n < kLargestBody ? 4 : 2);
+  return (unsigned)((n * lanes + kRowThreads - 1) / kRowThreads);
+}
 
-// The eight lanes' sum, in every lane.
-__device__ __forceinline__ double row_sum(double v) {
+// launch(LARGE): the sums' kernels come in both forms.
+template <typename F> static void launch_rows(int64_t n, F &&launch) {
+  if (n < kLargeBody)
+    launch(std::false_type{});
+  else
+    launch(std::true_type{});
+}
+
+// Calls pass(lanes, thread) for the calling thread's passes over the rows; whole warps make the same passes.
+template <int LANES, typename F> __device__ __forceinline__ void row_passes(int64_t n, F &&pass) {
+  const int64_t thread = (int64_t)blockIdx.x * kRowThreads + threadIdx.x, threads = (int64_t)gridDim.x * kRowThreads;
+  for (int64_t t = thread; (t & ~int64_t(31)) < n * LANES; t += threads)
+    pass(std::integral_constant<int, LANES>{}, t);
+}
+template <bool LARGE, typename F>
+__device__ __forceinline__ void row_passes(int64_t n, const int64_t *row_ptr, F &&pass) {
+  if (!LARGE) {
+    pass(std::integral_constant<int, 8>{}, (int64_t)blockIdx.x * kRowThreads + threadIdx.x);
+    return;
+  }
+  const int lanes = row_lanes(n, row_ptr);
+  if (lanes == 1)
+    row_passes<1>(n, pass);
+  else if (lanes == 2)
+    row_passes<2>(n, pass);
+  else
+    row_passes<4>(n, pass);
+}
+
+// The sum over a row's lanes, in every lane.
+template <int LANES> __device__ __forceinline__ double row_sum(double v) {
 #pragma unroll
-  for (int o = kRowLanes / 2; o > 0; o >>= 1)
+  for (int o = LANES / 2; o > 0; o >>= 1)
     v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
 
-// The calling lane's row; a lane past the end takes an empty one, so that whole warps take part in the shuffles.
+// Thread t's row; a thread past the end takes an empty one, so that whole warps take part in the shuffles.
 struct RowPoint {
   int64_t i, begin, end;
   int lane;
   bool valid;
 };
-__device__ __forceinline__ RowPoint row_point(int64_t n, const int64_t *row_ptr) {
-  const int64_t k = ((int64_t)blockIdx.x * kRowThreads + threadIdx.x) / kRowLanes;
+template <int LANES> __device__ __forceinline__ RowPoint row_point(int64_t n, const int64_t *row_ptr, int64_t t) {
+  const int64_t k = t / LANES;
   RowPoint r;
   r.valid = k < n;
   r.i = r.valid ? k : 0;
   r.begin = r.valid ? row_ptr[k] : 0, r.end = r.valid ? row_ptr[k + 1] : 0;
-  r.lane = threadIdx.x & (kRowLanes - 1);
+  r.lane = (int)t & (LANES - 1);
   return r;
 }
 
 // Calls bond(q, j) for the calling lane's bonds q of its row and their neighbours j.
-template <typename F> __device__ __forceinline__ void for_row(const RowPoint &r, const int32_t *col, F &&bond) {
+template <int LANES, typename F> __device__ __forceinline__ void for_row(const RowPoint &r, const int32_t *col, F &&bond) {
   int64_t q = r.begin + r.lane;
   int32_t j = q < r.end ? __ldg(col + q) : 0;
 #pragma unroll 2
-  for (; q < r.end; q += kRowLanes) {
-    const int32_t next = q + kRowLanes < r.end ? __ldg(col + q + kRowLanes) : 0;
+  for (; q < r.end; q += LANES) {
+    const int32_t next = q + LANES < r.end ? __ldg(col + q + LANES) : 0;
     bond(q, (int64_t)j);
     j = next;
   }
@@ -91,6 +132,10 @@ template <bool CURRENT> struct VectorsPlain {
     return make_double4(v[0], v[1], v[2], 0.0);
   }
 };
+// The records pay where rows are long and points are many. Calls at horizon 4.015 h, plain | packed: damage 36,000
+// points 83 | 66 us, 108,000 187 | 156, 250,000 405 | 328; deformation 250,000 261 | 273, 1M 1056 | 1042; shape
+// tensors 250,000 204 | 205, 1M 718 | 665; with the 250,000 points in no order, damage 2 times as fast, the other two
+// 1.9 times. (Not in the force sum: its nine words of M a bond outweigh the four of the point.)
 struct Packed {
   const double4 *rec;
   __device__ __forceinline__ double4 xv(int64_t j) const { return ldg256(rec + j); }
@@ -108,28 +153,22 @@ __global__ void k_pack_points(const double *pos, const double *vol, const double
     st256(vec + i, VectorsPlain<CURRENT>{pos, disp}.at(i));
 }
 
-// Where the records pay for their pass. Calls at horizon 4.015 h, plain | packed:
-// damage 16,000 points 34 | 30 us, 36,000 73 | 64, 154,000 295 | 238; deformation 36,000 51 | 53, 154,000
-// 203 | 203, 250,000 345 | 324; shape tensors 154,000 165 | 158, 250,000 251 | 226; the same points in no order,
-// 250,000: deformation 955 | 485, shape tensors 611 | 305. (Not in the force
-// sum: its nine words of M a bond outweigh the four of the point, 644 | 659 us at 250,000.)
-
 // PdCorrespondenceSkeleton::initialize (:149-170)
-template <typename Points>
-__global__ void __launch_bounds__(kRowThreads) k_csr_shape_inverse(Points points, int64_t n, const int64_t *row_ptr,
-                                                                   const int32_t *col, double *kinv,
-                                                                   unsigned *status) {
-  const RowPoint r = row_point(n, row_ptr);
-  const double4 x = points.xv(r.i);
+template <int LANES, typename Points>
+__device__ __forceinline__ void shape_inverse_row(Points points, int64_t t, int64_t n, const int64_t *row_ptr, const int32_t *col,
+                                                   double *kinv, unsigned *status) {
+  const RowPoint r = row_point<LANES>(n, row_ptr, t);
+  const int64_t i = r.i;
+  const double4 x = points.xv(i);
   double k00 = 0, k01 = 0, k02 = 0, k11 = 0, k12 = 0, k22 = 0;
-  for_row(r, col, [&](int64_t, int64_t j) {
+  for_row<LANES>(r, col, [&](int64_t, int64_t j) {
     const double4 p = points.xv(j);
     const double e0 = p.x - x.x, e1 = p.y - x.y, e2 = p.z - x.z, v = p.w, w0 = v * e0, w1 = v * e1;
     k00 += w0 * e0, k01 += w0 * e1, k02 += w0 * e2;
     k11 += w1 * e1, k12 += w1 * e2, k22 += v * e2 * e2;
   });
-  k00 = row_sum(k00), k01 = row_sum(k01), k02 = row_sum(k02);
-  k11 = row_sum(k11), k12 = row_sum(k12), k22 = row_sum(k22);
+  k00 = row_sum<LANES>(k00), k01 = row_sum<LANES>(k01), k02 = row_sum<LANES>(k02);
+  k11 = row_sum<LANES>(k11), k12 = row_sum<LANES>(k12), k22 = row_sum<LANES>(k22);
   if (!r.valid || r.lane != 0)
     return;
   const double K[9] = {k00, k01, k02, k01, k11, k12, k02, k12, k22};
@@ -140,19 +179,27 @@ __global__ void __launch_bounds__(kRowThreads) k_csr_shape_inverse(Points points
       Ki[c] = 0.0;
   }
   for (int c = 0; c < 9; ++c)
-    kinv[9 * r.i + c] = Ki[c];
+    kinv[9 * i + c] = Ki[c];
+}
+template <bool LARGE, typename Points>
+__global__ void __launch_bounds__(kRowThreads) k_csr_shape_inverse(Points points, int64_t n, const int64_t *row_ptr,
+                                                                   const int32_t *col, double *kinv,
+                                                                   unsigned *status) {
+  row_passes<LARGE>(n, row_ptr, [&](auto lanes, int64_t t) {
+    shape_inverse_row<decltype(lanes)::value>(points, t, n, row_ptr, col, kinv, status);
+  });
 }
 
 // computeDeformationGradients (:172-197), in displacement-gradient form
 // F = I + [sum_j V_j (u_j - u_i) (x) xi] K^-1.
-template <typename Points, typename Vectors>
-__global__ void __launch_bounds__(kRowThreads) k_csr_deformation(Points points, Vectors disp, int64_t n,
-                                                                 const int64_t *row_ptr, const int32_t *col,
-                                                                 const double *kinv, double *F) {
-  const RowPoint r = row_point(n, row_ptr);
-  const double4 x = points.xv(r.i), u = disp.at(r.i);
+template <int LANES, typename Points, typename Vectors>
+__device__ __forceinline__ void deformation_row(Points points, Vectors disp, int64_t t, int64_t n, const int64_t *row_ptr,
+                                                 const int32_t *col, const double *kinv, double *F) {
+  const RowPoint r = row_point<LANES>(n, row_ptr, t);
+  const int64_t i = r.i;
+  const double4 x = points.xv(i), u = disp.at(i);
   double G[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-  for_row(r, col, [&](int64_t, int64_t j) {
+  for_row<LANES>(r, col, [&](int64_t, int64_t j) {
     const double4 p = points.xv(j), uj = disp.at(j);
     const double e[3] = {p.x - x.x, p.y - x.y, p.z - x.z};
     const double d[3] = {p.w * (uj.x - u.x), p.w * (uj.y - u.y), p.w * (uj.z - u.z)};
@@ -164,16 +211,28 @@ __global__ void __launch_bounds__(kRowThreads) k_csr_deformation(Points points, 
   });
 #pragma unroll
   for (int c = 0; c < 9; ++c)
-    G[c] = row_sum(G[c]);
-  const int a = r.lane;  // lanes 0..2 write rows 0..2 of F
-  if (!r.valid || a >= 3)
+    G[c] = row_sum<LANES>(G[c]);
+  if (!r.valid)
     return;
-  const double g0 = a == 0 ? G[0] : (a == 1 ? G[3] : G[6]), g1 = a == 0 ? G[1] : (a == 1 ? G[4] : G[7]),
-               g2 = a == 0 ? G[2] : (a == 1 ? G[5] : G[8]);
-  const double *K = kinv + 9 * r.i;
+  double K[9];
 #pragma unroll
-  for (int b = 0; b < 3; ++b)
-    F[9 * r.i + 3 * a + b] = (a == b ? 1.0 : 0.0) + (g0 * K[b] + g1 * K[3 + b] + g2 * K[6 + b]);
+  for (int c = 0; c < 9; ++c)
+    K[c] = kinv[9 * i + c];
+#pragma unroll
+  for (int a = 0; a < 3; ++a)  // the row's lanes write the rows of F in turn
+    if (a % LANES == r.lane)
+#pragma unroll
+      for (int b = 0; b < 3; ++b)
+        F[9 * i + 3 * a + b] =
+            (a == b ? 1.0 : 0.0) + (G[3 * a] * K[b] + G[3 * a + 1] * K[3 + b] + G[3 * a + 2] * K[6 + b]);
+}
+template <bool LARGE, typename Points, typename Vectors>
+__global__ void __launch_bounds__(kRowThreads, 4) k_csr_deformation(Points points, Vectors disp, int64_t n,
+                                                                    const int64_t *row_ptr, const int32_t *col,
+                                                                    const double *kinv, double *F) {
+  row_passes<LARGE>(n, row_ptr, [&](auto lanes, int64_t t) {
+    deformation_row<decltype(lanes)::value>(points, disp, t, n, row_ptr, col, kinv, F);
+  });
 }
 
 // The force map M = J sigma F^-T K^-1 of every point as the bond sum gathers it: entries 0..7 as four
@@ -199,17 +258,18 @@ __global__ void k_csr_force_map(const double *sigma, const double *F, const doub
 }
 
 // computeForceDensity (:199-230): f_i = sum (1 - clamp(d)) (M_i + M_j) xi V_j
-__global__ void __launch_bounds__(kRowThreads) k_csr_force(PointsPlain points, int64_t n, const int64_t *row_ptr,
-                                                           const int32_t *col, const double *M,
-                                                           const double *bond_damage, double *force) {
-  const RowPoint r = row_point(n, row_ptr);
+template <int LANES>
+__device__ __forceinline__ void force_row(PointsPlain points, int64_t t, int64_t n, const int64_t *row_ptr, const int32_t *col,
+                                           const double *M, const double *bond_damage, double *force) {
   const double2 *pairs = reinterpret_cast<const double2 *>(M);
-  const double4 x = points.xv(r.i);
-  const double2 ai = __ldg(pairs + r.i), bi = __ldg(pairs + n + r.i), ci = __ldg(pairs + 2 * n + r.i),
-                di = __ldg(pairs + 3 * n + r.i);
-  const double m8i = __ldg(M + 8 * n + r.i);
+  const RowPoint r = row_point<LANES>(n, row_ptr, t);
+  const int64_t i = r.i;
+  const double4 x = points.xv(i);
+  const double2 ai = __ldg(pairs + i), bi = __ldg(pairs + n + i), ci = __ldg(pairs + 2 * n + i),
+                di = __ldg(pairs + 3 * n + i);
+  const double m8i = __ldg(M + 8 * n + i);
   double f0 = 0, f1 = 0, f2 = 0;
-  for_row(r, col, [&](int64_t q, int64_t j) {
+  for_row<LANES>(r, col, [&](int64_t q, int64_t j) {
     const double4 p = points.xv(j);
     const double e0 = p.x - x.x, e1 = p.y - x.y, e2 = p.z - x.z;
     double dmg = bond_damage ? __ldg(bond_damage + q) : 0.0;
@@ -222,9 +282,17 @@ __global__ void __launch_bounds__(kRowThreads) k_csr_force(PointsPlain points, i
     f1 += w * ((bi.y + b.y) * e0 + (ci.x + c.x) * e1 + (ci.y + c.y) * e2);
     f2 += w * ((di.x + d.x) * e0 + (di.y + d.y) * e1 + (m8i + m8) * e2);
   });
-  f0 = row_sum(f0), f1 = row_sum(f1), f2 = row_sum(f2);
+  f0 = row_sum<LANES>(f0), f1 = row_sum<LANES>(f1), f2 = row_sum<LANES>(f2);
   if (r.valid && r.lane == 0)
-    force[3 * r.i] = f0, force[3 * r.i + 1] = f1, force[3 * r.i + 2] = f2;
+    force[3 * i] = f0, force[3 * i + 1] = f1, force[3 * i + 2] = f2;
+}
+template <bool LARGE>
+__global__ void __launch_bounds__(kRowThreads, 3) k_csr_force(PointsPlain points, int64_t n, const int64_t *row_ptr,
+                                                              const int32_t *col, const double *M,
+                                                              const double *bond_damage, double *force) {
+  row_passes<LARGE>(n, row_ptr, [&](auto lanes, int64_t t) {
+    force_row<decltype(lanes)::value>(points, t, n, row_ptr, col, M, bond_damage, force);
+  });
 }
 
 // ------------------------------------------------------------------ pointwise kernels
@@ -434,15 +502,15 @@ __device__ __forceinline__ bool stretch_breaks(const StretchTest &t, const doubl
   return stretch > t.initiation || (t.use_compression && stretch < -t.failure);
 }
 
-template <typename Points, typename Vectors>
-__global__ void __launch_bounds__(kRowThreads) k_csr_damage(Points points, Vectors current, int64_t n,
-                                                            const int64_t *row_ptr, const int32_t *col,
-                                                            StretchTest test, double *bond_damage,
-                                                            double *damage_index) {
-  const RowPoint r = row_point(n, row_ptr);
-  const double4 x = points.xv(r.i), yi = current.at(r.i);
+template <int LANES, typename Points, typename Vectors>
+__device__ __forceinline__ void damage_row(Points points, Vectors current, int64_t t, int64_t n, const int64_t *row_ptr,
+                                            const int32_t *col, const StretchTest &test, double *bond_damage,
+                                            double *damage_index) {
+  const RowPoint r = row_point<LANES>(n, row_ptr, t);
+  const int64_t i = r.i;
+  const double4 x = points.xv(i), yi = current.at(i);
   double damaged = 0.0, total = 0.0;
-  for_row(r, col, [&](int64_t q, int64_t j) {
+  for_row<LANES>(r, col, [&](int64_t q, int64_t j) {
     const double4 p = points.xv(j), yj = current.at(j);
     const double e[3] = {__dsub_rn(p.x, x.x), __dsub_rn(p.y, x.y), __dsub_rn(p.z, x.z)};
     const double y[3] = {__dsub_rn(yj.x, yi.x), __dsub_rn(yj.y, yi.y), __dsub_rn(yj.z, yi.z)};
@@ -452,9 +520,18 @@ __global__ void __launch_bounds__(kRowThreads) k_csr_damage(Points points, Vecto
     damaged += d * p.w;
     total += p.w;
   });
-  damaged = row_sum(damaged), total = row_sum(total);
+  damaged = row_sum<LANES>(damaged), total = row_sum<LANES>(total);
   if (damage_index && r.valid && r.lane == 0)
-    damage_index[r.i] = total > 0.0 ? damaged / total : 0.0;
+    damage_index[i] = total > 0.0 ? damaged / total : 0.0;
+}
+template <bool LARGE, typename Points, typename Vectors>
+__global__ void __launch_bounds__(kRowThreads, 4) k_csr_damage(Points points, Vectors current, int64_t n,
+                                                               const int64_t *row_ptr, const int32_t *col,
+                                                               StretchTest test, double *bond_damage,
+                                                               double *damage_index) {
+  row_passes<LARGE>(n, row_ptr, [&](auto lanes, int64_t t) {
+    damage_row<decltype(lanes)::value>(points, current, t, n, row_ptr, col, test, bond_damage, damage_index);
+  });
 }
 
 // Johnson-Cook on one column-major block (the plugin ABI).
@@ -514,8 +591,10 @@ int launch_csr_force(const double *positions, const double *volumes, int64_t n, 
                      const int32_t *col, const double *kinv, const double *defgrad, const double *cauchy_stress,
                      const double *bond_damage, double *force, double *M, unsigned *status, cudaStream_t s) {
   k_csr_force_map<<<blocks(n), 128, 0, s>>>(cauchy_stress, defgrad, kinv, n, M, status);
-  k_csr_force<<<row_blocks(n), kRowThreads, 0, s>>>(PointsPlain{positions, volumes}, n, row_ptr, col, M, bond_damage,
-                                                    force);
+  launch_rows(n, [&](auto large) {
+    k_csr_force<decltype(large)::value><<<row_blocks(n), kRowThreads, 0, s>>>(PointsPlain{positions, volumes}, n,
+        row_ptr, col, M, bond_damage, force);
+  });
   VPD_CUDA(cudaGetLastError());
   return VPD_OK;
 }
@@ -537,10 +616,15 @@ static int shape_tensor_inverse(const double *positions, const double *volumes, 
   VPD_CUDA(cudaMemsetAsync(st, 0, sizeof(unsigned), s));
   if (rec) {
     k_pack_points<false><<<blocks(n), 128, 0, s>>>(positions, volumes, nullptr, n, rec, nullptr);
-    k_csr_shape_inverse<<<row_blocks(n), kRowThreads, 0, s>>>(Packed{rec}, n, row_ptr, col, kinv, st);
+    launch_rows(n, [&](auto large) {
+      k_csr_shape_inverse<decltype(large)::value><<<row_blocks(n), kRowThreads, 0, s>>>(Packed{rec}, n, row_ptr,
+          col, kinv, st);
+    });
   } else {
-    k_csr_shape_inverse<<<row_blocks(n), kRowThreads, 0, s>>>(PointsPlain{positions, volumes}, n, row_ptr, col, kinv,
-                                                              st);
+    launch_rows(n, [&](auto large) {
+      k_csr_shape_inverse<decltype(large)::value><<<row_blocks(n), kRowThreads, 0, s>>>(PointsPlain{positions,
+          volumes}, n, row_ptr, col, kinv, st);
+    });
   }
   VPD_CUDA(cudaGetLastError());
   return check_status(st, s);
@@ -553,12 +637,15 @@ static int deformation_gradients(const double *positions, const double *displace
     return VPD_OK;
   if (rec) {
     k_pack_points<false><<<blocks(n), 128, 0, s>>>(positions, volumes, displacement, n, rec, rec + n);
-    k_csr_deformation<<<row_blocks(n), kRowThreads, 0, s>>>(Packed{rec}, Packed{rec + n}, n, row_ptr, col, kinv,
-                                                            defgrad);
+    launch_rows(n, [&](auto large) {
+      k_csr_deformation<decltype(large)::value><<<row_blocks(n), kRowThreads, 0, s>>>(Packed{rec}, Packed{rec + n},
+          n, row_ptr, col, kinv, defgrad);
+    });
   } else {
-    k_csr_deformation<<<row_blocks(n), kRowThreads, 0, s>>>(PointsPlain{positions, volumes},
-                                                            VectorsPlain<false>{positions, displacement}, n, row_ptr,
-                                                            col, kinv, defgrad);
+    launch_rows(n, [&](auto large) {
+      k_csr_deformation<decltype(large)::value><<<row_blocks(n), kRowThreads, 0, s>>>(PointsPlain{positions,
+          volumes}, VectorsPlain<false>{positions, displacement}, n, row_ptr, col, kinv, defgrad);
+    });
   }
   VPD_CUDA(cudaGetLastError());
   return VPD_OK;
@@ -576,12 +663,15 @@ static int damage_update(const double *positions, const double *displacement, co
                          failure < 1.0 ? (1.0 - failure) * (1.0 - failure) : 0.0, use_compression};
   if (rec) {
     k_pack_points<true><<<blocks(n), 128, 0, s>>>(positions, volumes, displacement, n, rec, rec + n);
-    k_csr_damage<<<row_blocks(n), kRowThreads, 0, s>>>(Packed{rec}, Packed{rec + n}, n, row_ptr, col, test,
-                                                       bond_damage, damage_index);
+    launch_rows(n, [&](auto large) {
+      k_csr_damage<decltype(large)::value><<<row_blocks(n), kRowThreads, 0, s>>>(Packed{rec}, Packed{rec + n}, n,
+          row_ptr, col, test, bond_damage, damage_index);
+    });
   } else {
-    k_csr_damage<<<row_blocks(n), kRowThreads, 0, s>>>(PointsPlain{positions, volumes},
-                                                       VectorsPlain<true>{positions, displacement}, n, row_ptr, col,
-                                                       test, bond_damage, damage_index);
+    launch_rows(n, [&](auto large) {
+      k_csr_damage<decltype(large)::value><<<row_blocks(n), kRowThreads, 0, s>>>(PointsPlain{positions, volumes},
+          VectorsPlain<true>{positions, displacement}, n, row_ptr, col, test, bond_damage, damage_index);
+    });
   }
   VPD_CUDA(cudaGetLastError());
   return VPD_OK;

@@ -324,12 +324,13 @@ def build_neighbor_list(positions, horizon: float):
     return row_ptr, col[: total.value]
 
 
-def _records(positions, vectors, points):
-    """Room for the packed records of a bond sum over `vectors` vectors a point, for bodies of `points` points or
-    more: None for smaller ones and where there is no memory (the sums then read the arrays as they are)."""
+def _records(positions, col, vectors, points, bonds):
+    """Room for the packed records of a bond sum over `vectors` vectors a point, for bodies of `points` points and
+    `bonds` bonds a point or more: None for smaller ones and where there is no memory (the sums then read the arrays
+    as they are)."""
     import torch
     n = positions.shape[0]
-    if n < points:
+    if n < points or col.numel() < bonds * n:
         return None
     try:
         return torch.empty((vectors * n, 4), dtype=torch.float64, device=positions.device)
@@ -341,7 +342,7 @@ def shape_tensor_inverse(positions, volumes, row_ptr, col):
     import torch
     out = torch.empty((positions.shape[0], 9), dtype=torch.float64, device=positions.device)
     args = (_ptr(positions), _ptr(volumes), positions.shape[0], _ptr(row_ptr), _ptr(col), _ptr(out))
-    records = _records(positions, 1, 150_000)
+    records = _records(positions, col, 1, 150_000, 64)
     _check(library().vpd_shape_tensor_inverse(*args, _stream()) if records is None else
            library().vpd_shape_tensor_inverse_packed(*args, _ptr(records), _stream()))
     return out
@@ -352,7 +353,7 @@ def deformation_gradients(positions, displacement, volumes, row_ptr, col, kinv):
     out = torch.empty((positions.shape[0], 9), dtype=torch.float64, device=positions.device)
     args = (_ptr(positions), _ptr(displacement), _ptr(volumes), positions.shape[0], _ptr(row_ptr), _ptr(col),
             _ptr(kinv), _ptr(out))
-    records = _records(positions, 2, 150_000)
+    records = _records(positions, col, 2, 150_000, 64)
     _check(library().vpd_deformation_gradients(*args, _stream()) if records is None else
            library().vpd_deformation_gradients_packed(*args, _ptr(records), _stream()))
     return out
@@ -452,7 +453,7 @@ def damage_update(positions, displacement, volumes, row_ptr, col, initiation, fa
     idx = torch.empty(positions.shape[0], dtype=torch.float64, device=positions.device)
     args = (_ptr(positions), _ptr(displacement), _ptr(volumes), positions.shape[0], _ptr(row_ptr), _ptr(col),
             initiation, failure, _ptr(bond_damage), _ptr(idx))
-    records = _records(positions, 2, 16_000)
+    records = _records(positions, col, 2, 16_000, 24)
     _check(library().vpd_damage_update(*args, _stream()) if records is None else
            library().vpd_damage_update_packed(*args, _ptr(records), _stream()))
     return idx
