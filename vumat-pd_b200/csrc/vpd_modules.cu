@@ -473,11 +473,25 @@ __global__ void __launch_bounds__(kPointThreads, 8) k_jc_return_map(int64_t n, J
 // PdSimpleDamage::update critical_stretch (:51-82) with the reference's rounding, and the
 // damage index (:23-36). A bond whose squared lengths lie clear of both thresholds (by 1e-9 of them,
 // against roundings of 1e-15) is decided from those; the others, and lengths whose squares may not be
-// normal numbers, take the reference's square roots and division.
+// normal numbers, take the reference's square roots and division. In compression the formula's stretch carries a
+// rounding of 1e-16 of the initial length, which may be any part of the current one: where the threshold leaves less
+// than kLeastLeft of a bond, every bond shorter than twice that takes the formula.
 struct StretchTest {
-  double initiation, failure, tension2, compression2;  // thresholds on the stretch and on (1 + it)^2
+  double initiation, failure, tension2;  // thresholds on the stretch, and on (1 + it)^2
+  double surely_broken2, surely_whole2;  // current over initial length squared, in compression: below, above
   int use_compression;
 };
+constexpr double kLeastLeft = 0.01;
+static StretchTest stretch_test(double initiation, double failure) {
+  StretchTest t{initiation, failure, (1.0 + initiation) * (1.0 + initiation), -1.0, 0.0,
+                failure > 0.0 && std::isfinite(failure)};
+  const double left = 1.0 - failure;
+  if (left >= kLeastLeft)
+    t.surely_broken2 = left * left * (1.0 - 1.0e-9), t.surely_whole2 = left * left * (1.0 + 1.0e-9);
+  else if (left > 0.0)
+    t.surely_whole2 = 4.0 * kLeastLeft * kLeastLeft;
+  return t;
+}
 __device__ __forceinline__ bool stretch_breaks(const StretchTest &t, const double (&e)[3], const double (&y)[3]) {
   const double xx =
       __dadd_rn(__dadd_rn(__dmul_rn(e[0], e[0]), __dmul_rn(e[1], e[1])), __dmul_rn(e[2], e[2]));
@@ -490,10 +504,9 @@ __device__ __forceinline__ bool stretch_breaks(const StretchTest &t, const doubl
     if (yy < tt * (1.0 - 1.0e-9)) {
       if (!t.use_compression)
         return false;
-      const double c = t.compression2 * xx;
-      if (yy < c * (1.0 - 1.0e-9))
+      if (yy < t.surely_broken2 * xx)
         return true;
-      if (yy > c * (1.0 + 1.0e-9))
+      if (yy > t.surely_whole2 * xx)
         return false;
     }
   }
@@ -658,9 +671,7 @@ static int damage_update(const double *positions, const double *displacement, co
     return set_error(VPD_ERR_INVALID, "critical_stretch requires initiation > 0.");
   if (n <= 0)
     return VPD_OK;
-  const int use_compression = failure > 0.0 && std::isfinite(failure);
-  const StretchTest test{initiation, failure, (1.0 + initiation) * (1.0 + initiation),
-                         failure < 1.0 ? (1.0 - failure) * (1.0 - failure) : 0.0, use_compression};
+  const StretchTest test = stretch_test(initiation, failure);
   if (rec) {
     k_pack_points<true><<<blocks(n), 128, 0, s>>>(positions, volumes, displacement, n, rec, rec + n);
     launch_rows(n, [&](auto large) {
