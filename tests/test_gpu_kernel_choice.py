@@ -62,3 +62,10 @@ def test_bond_sums_over_short_rows_take_at_most_four_times_a_copy(bonds):
         a = torch.empty(moved // 2, dtype=torch.uint8, device="cuda")
         b = torch.empty_like(a)
         assert seconds(call) <= 4.0 * seconds(lambda: b.copy_(a))
+
+
+def test_neighbour_lists_of_one_cell_take_at_most_six_times_those_of_many():
+    """All points in one cell (3,374 bonds each) against the same body in 125 cells (96 bonds)."""
+    pos = np.stack(np.meshgrid(*[np.arange(15.0)] * 3, indexing="ij"), -1).reshape(-1, 3)
+    x = torch.as_tensor(pos).cuda()
+    assert seconds(lambda: vpd.build_neighbor_list(x, 30.0)) <= 6.0 * seconds(lambda: vpd.build_neighbor_list(x, 3.015))

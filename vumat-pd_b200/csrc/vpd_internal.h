@@ -101,6 +101,7 @@ struct NeighborGrid {
   int64_t ncells = 0;
   int max_len = 0;
   int candidates = 0;  // most points in the 27 cells around one, where k_nb_cell searches (0: the per-point search)
+  int cell_blocks = 1; // its blocks per cell
 };
 
 // Maximum neighbours per point the sorted fill supports (shared-memory row buffer).

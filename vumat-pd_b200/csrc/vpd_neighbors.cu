@@ -13,7 +13,7 @@
 // of points into a dense cell grid; the matches of every point counted; an exclusive scan
 // gives row_ptr; the matches written in ascending order.
 //
-// The search runs a block per cell (k_nb_cell): the points of the 27 cells around it are sorted by
+// The search runs a block per cell, or several (k_nb_cell): the points of the 27 cells around it are sorted by
 // index once for all of its points, so a row's matches come out in order by ballot compaction and no row is
 // sorted by itself. Distances are decided in FP32, in units of the cell width and relative to a point of the
 // cell, outside a margin of 2e-5 of the squared radius (ten times their error), and by the exact test within it;
@@ -149,8 +149,8 @@ int scan_exclusive_i32(const int32_t *in, int64_t n, int64_t *out, int64_t *tmp,
 
 // ------------------------------------------------------------------ neighbour kernels
 // reduce words: [0] max row length, [1] flags (1: non-finite coordinate, 2: a row beyond its buffer), [2..4] min
-// coordinate, [5..7] max coordinate (order_key), [8] max candidates around a cell.
-constexpr int kReduceWords = 9;
+// coordinate, [5..7] max coordinate (order_key), [8..11] of the cells (k_cell_load).
+constexpr int kReduceWords = 12;
 
 // Doubles as integers of the same order (a finite number and its key determine each other).
 __host__ __device__ __forceinline__ long long order_key(long long bits) {
@@ -389,16 +389,36 @@ __device__ __forceinline__ CellRun cell_run(int64_t c, const GridDev &g, const i
   return {b, (int)(cell_start[row + hi + 1] - b)};
 }
 
-// The most candidates of any cell that holds points.
-__global__ void k_cell_candidates(int64_t ncells, GridDev g, const int64_t *cell_start, unsigned long long *most) {
+// load[0] the most candidates of any cell that holds points; of cells with up to kMaxCandidates, load[1] the most
+// points, load[2] the most pairs (points times candidates) and load[3] all pairs.
+__global__ void k_cell_load(int64_t ncells, GridDev g, const int64_t *cell_start, unsigned long long *load) {
   const int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  unsigned total = 0;
-  if (c < ncells && cell_start[c + 1] > cell_start[c])
+  unsigned total = 0, points = 0;
+  if (c < ncells && cell_start[c + 1] > cell_start[c]) {
     for (int k = 0; k < 9; ++k)
       total += (unsigned)cell_run(c, g, cell_start, k).count;
-  total = __reduce_max_sync(0xffffffffu, total);
-  if ((threadIdx.x & 31) == 0 && total)
-    atomicMax(most, (unsigned long long)total);
+    if (total <= kMaxCandidates)
+      points = (unsigned)(cell_start[c + 1] - cell_start[c]);
+  }
+  const unsigned pairs = points * total;  // below 2^24
+  total = __reduce_max_sync(0xffffffffu, total), points = __reduce_max_sync(0xffffffffu, points);
+  const unsigned most = __reduce_max_sync(0xffffffffu, pairs), sum = __reduce_add_sync(0xffffffffu, pairs);
+  if ((threadIdx.x & 31) == 0 && total) {
+    atomicMax(load, (unsigned long long)total);
+    atomicMax(load + 1, (unsigned long long)points);
+    atomicMax(load + 2, (unsigned long long)most);
+    atomicAdd(load + 3, (unsigned long long)sum);
+  }
+}
+
+// Blocks per cell: one, unless the busiest cell has more pairs than a fair share of the GPU's four blocks per SM
+// (a body of a few cells, or a cluster among sparse points); each block then searches for some of the cell's points, 32
+// or more. The two calls that build the list, microseconds, a block per cell | so: 3,375 points in one cell 9938 | 415,
+// 2,744 points in eight cells 5376 | 415 (3200 both with a warp per point and allocations in the calls).
+static int cell_blocks(const unsigned long long *load) {
+  const unsigned long long fair = std::max(load[3] / (4 * 148), 32 * load[0]);
+  const unsigned long long wanted = (load[2] + fair - 1) / fair;
+  return (int)std::min(wanted, (load[1] + 31) / 32);
 }
 
 // Ascending bitonic sort of `width` (a power of two, at least 32) shared-memory ints by the whole block.
@@ -469,8 +489,8 @@ struct CellSearch {
   float r2lo, r2hi;  // (radius / cell width)^2 less and plus the margin
 };
 
-// One block per cell. FILL: the rows of the cell's points into col; else their lengths into len (and the largest to
-// *longest).
+// gridDim.y blocks per cell (blockIdx.x). FILL: the rows of the cell's points into col; else their lengths into len (and
+// the largest to *longest).
 template <bool FILL>
 __global__ void __launch_bounds__(kCellThreads) k_nb_cell(const double4 *xv, GridDev g, const int64_t *cell_start,
                                                           const int32_t *sorted, CellSearch cs, int width,
@@ -484,7 +504,12 @@ __global__ void __launch_bounds__(kCellThreads) k_nb_cell(const double4 *xv, Gri
   __shared__ int64_t s_begin[9];
   __shared__ int s_off[10], s_lo, s_hi;
   const int64_t c = blockIdx.x, first = cell_start[c], last = cell_start[c + 1];
-  if (first == last)
+  // this block's share of the cell's points (in ascending order): pairs of points for every warp
+  constexpr int kPairs = 2 * (kCellThreads / 32);
+  const int points = (int)(last - first);
+  const int share = ((points + (int)gridDim.y - 1) / (int)gridDim.y + kPairs - 1) / kPairs * kPairs;
+  const int q0 = (int)blockIdx.y * share, q1 = min(points, q0 + share);
+  if (q0 >= q1)
     return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (threadIdx.x < 32) {
@@ -527,7 +552,6 @@ __global__ void __launch_bounds__(kCellThreads) k_nb_cell(const double4 *xv, Gri
     atomicMin(&s_lo, lo), atomicMax(&s_hi, hi);
   __syncthreads();
   const int words = (s_hi - s_lo) / 32 + 1;
-  const int points = (int)(last - first);
   if (words <= 4 * width) {  // the candidates' positions are not there yet: 16 bytes each
     block_sort_bits(index, total, s_lo, reinterpret_cast<uint32_t *>(cand), words);
     block_sort_bits(own, points, s_lo, reinterpret_cast<uint32_t *>(cand), words);
@@ -557,14 +581,14 @@ __global__ void __launch_bounds__(kCellThreads) k_nb_cell(const double4 *xv, Gri
   // and packed FP32 arithmetic for both
   const unsigned lt = (1u << lane) - 1u;
   int most = 0;
-  for (int q = 2 * warp; q < points; q += 2 * (kCellThreads / 32)) {
+  for (int q = q0 + 2 * warp; q < q1; q += kPairs) {
     int32_t i[2];
     float x[2], y[2], z[2];
     int32_t *row[2];
     int cnt[2] = {0, 0};
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-      i[h] = own[min(q + h, points - 1)];
+      i[h] = own[min(q + h, q1 - 1)];
       const double4 pi = xv[i[h]];
       x[h] = (float)((pi.x - ref.x) * cs.inv_width), y[h] = (float)((pi.y - ref.y) * cs.inv_width);
       z[h] = (float)((pi.z - ref.z) * cs.inv_width);
@@ -601,7 +625,7 @@ __global__ void __launch_bounds__(kCellThreads) k_nb_cell(const double4 *xv, Gri
           const bool k = keep[h] && j != i[h];
           if (FILL) {
             const unsigned hit = __ballot_sync(0xffffffffu, k);
-            if (k && q + h < points)
+            if (k && q + h < q1)
               row[h][cnt[h] + __popc(hit & lt)] = j;
             cnt[h] += __popc(hit);
           } else {
@@ -646,8 +670,9 @@ static int launch_cells(const double4 *xv, const NeighborGrid &grid, const Neigh
   // set it between this one's and its launch
   VPD_CUDA(cudaFuncSetAttribute(k_nb_cell<FILL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)cell_smem(kMaxCandidates)));
-  k_nb_cell<FILL><<<(unsigned)grid.ncells, kCellThreads, smem, s>>>(xv, g, scr.cell_start, scr.sorted, cs, width, row_ptr,
-                                                                    col, scr.len, scr.reduce);
+  const dim3 blocks((unsigned)grid.ncells, (unsigned)grid.cell_blocks);
+  k_nb_cell<FILL><<<blocks, kCellThreads, smem, s>>>(xv, g, scr.cell_start, scr.sorted, cs, width, row_ptr, col, scr.len,
+                                                     scr.reduce);
   VPD_CUDA(cudaGetLastError());
   return VPD_OK;
 }
@@ -697,7 +722,7 @@ int neighbor_count(const double4 *xv, int64_t n, double horizon, int64_t *row_pt
   unsigned long long init[kReduceWords] = {0, 0,
                                            (unsigned long long)LLONG_MAX, (unsigned long long)LLONG_MAX,
                                            (unsigned long long)LLONG_MAX, (unsigned long long)LLONG_MIN,
-                                           (unsigned long long)LLONG_MIN, (unsigned long long)LLONG_MIN, 0};
+                                           (unsigned long long)LLONG_MIN, (unsigned long long)LLONG_MIN, 0, 0, 0, 0};
   VPD_CUDA(cudaMemcpyAsync(scr.reduce, init, sizeof init, cudaMemcpyHostToDevice, s));
   k_bounds<<<grid_for(n, 256), 256, 0, s>>>(xv, n, scr.reduce);
   unsigned long long red[kReduceWords];
@@ -750,12 +775,11 @@ int neighbor_count(const double4 *xv, int64_t n, double horizon, int64_t *row_pt
   // reciprocal and square are ordinary numbers
   grid.candidates = 0;
   if (grid.ncells * kMinCellPoints <= n && grid.cell_width > 1.0e-100 && grid.cell_width < 1.0e100) {
-    k_cell_candidates<<<(unsigned)((grid.ncells + 255) / 256), 256, 0, s>>>(grid.ncells, g, scr.cell_start,
-                                                                           scr.reduce + 8);
+    k_cell_load<<<(unsigned)((grid.ncells + 255) / 256), 256, 0, s>>>(grid.ncells, g, scr.cell_start, scr.reduce + 8);
     VPD_CUDA(cudaMemcpyAsync(red, scr.reduce, sizeof red, cudaMemcpyDeviceToHost, s));
     VPD_CUDA(cudaStreamSynchronize(s));
     if (red[8] <= (unsigned long long)kMaxCandidates)
-      grid.candidates = (int)red[8];
+      grid.candidates = (int)red[8], grid.cell_blocks = cell_blocks(red + 8);
   }
   if (grid.candidates) {
     if ((rc = launch_cells<false>(xv, grid, scr, nullptr, nullptr, s)))
