@@ -114,3 +114,13 @@ def test_records_must_lie_on_a_32_byte_boundary():
         assert e.value.status == 1
 
 
+def test_idle_memory_is_bounded_when_a_call_returns():
+    w = torch.zeros(vpd.MLP_WEIGHTS, dtype=torch.int16, device="cuda")
+    b = torch.zeros(vpd.MLP_PARAMS - vpd.MLP_WEIGHTS, dtype=torch.float32, device="cuda")
+    x = torch.randn((400_000, 16), dtype=torch.float32, device="cuda")
+    first = vpd.mlp_gradients(w, b, x[:128], x[:128])
+    before = free_bytes()
+    second = vpd.mlp_gradients(w, b, x, x)  # 466 MB of partial gradients
+    # (not free_bytes(): its synchronisation would give memory back too)
+    assert before - torch.cuda.mem_get_info()[0] <= 256 << 20
+    del first, second

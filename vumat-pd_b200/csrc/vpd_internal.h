@@ -37,9 +37,12 @@ struct Workspace {
   explicit Workspace(cudaStream_t s) : stream(s) {}
   Workspace(const Workspace &) = delete;
   Workspace &operator=(const Workspace &) = delete;
-  ~Workspace() {
-    for (int k = 0; k < used; ++k)
-      workspace_free(ptrs[k], stream);
+  ~Workspace() { release(); }
+  // Gives everything back in stream order. Before a call's last synchronisation, so that the pool's bound holds when
+  // the call returns (memory given back after it stays idle until the next one).
+  void release() {
+    while (used > 0)
+      workspace_free(ptrs[--used], stream);
   }
   template <typename T> int alloc(T **p, size_t count) {
     if (used == kMax)

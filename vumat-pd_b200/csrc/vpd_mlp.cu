@@ -534,9 +534,11 @@ int mlp_adam(const float *partials, int64_t blocks, float *p, float *m, float *v
 
 // ------------------------------------------------------------------ C ABI (device pointers)
 namespace {
-int check_err(unsigned *derr, cudaStream_t s) {
+// The end of a call: its timeout word (in ws) read, its memory given back, its work done.
+int check_err(unsigned *derr, vpd::Workspace &ws, cudaStream_t s) {
   unsigned e = 0;
   VPD_CUDA(cudaMemcpyAsync(&e, derr, sizeof e, cudaMemcpyDeviceToHost, s));
+  ws.release();
   VPD_CUDA(cudaStreamSynchronize(s));
   if (e)
     return vpd::set_error(VPD_ERR_CUDA, "surrogate network: tensor-core wait timed out");
@@ -559,7 +561,7 @@ extern "C" int vpd_mlp_forward(const uint16_t *weights, const float *biases, con
   VPD_CUDA(cudaMemsetAsync(derr, 0, sizeof(unsigned), s));
   const MlpWeights w = mlp_weights(reinterpret_cast<const __nv_bfloat16 *>(weights), biases);
   rc = mlp_forward(w, x, batch, out, derr, s);
-  return rc == VPD_OK ? check_err(derr, s) : rc;
+  return rc == VPD_OK ? check_err(derr, ws, s) : rc;
 }
 
 extern "C" int vpd_mlp_gradients(const uint16_t *weights, const float *biases, const float *x,
@@ -581,5 +583,5 @@ extern "C" int vpd_mlp_gradients(const uint16_t *weights, const float *biases, c
   if ((rc = mlp_gradient_partials(w, rows, batch, partials, derr, s)) ||
       (rc = mlp_sum_partials(partials, blocks, grad, s)))
     return rc;
-  return check_err(derr, s);
+  return check_err(derr, ws, s);
 }

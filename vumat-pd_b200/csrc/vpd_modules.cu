@@ -720,7 +720,9 @@ int vpd_build_neighbor_list(const double *positions, int64_t n, double horizon, 
   if (rc == VPD_OK && col)
     rc = neighbor_fill(xv, n, row_ptr, col, grid, scr, s);
   neighbor_scratch_free(scr);
-  return rc;
+  ws.release();
+  const cudaError_t e = cudaStreamSynchronize(s);
+  return rc == VPD_OK && e != cudaSuccess ? cuda_error(e, "neighbour list") : rc;
 }
 
 int vpd_shape_tensor_inverse(const double *positions, const double *volumes, int64_t n,
@@ -769,6 +771,7 @@ int vpd_force_density(const double *positions, const double *volumes, int64_t n,
   if ((rc = launch_csr_force(positions, volumes, n, row_ptr, col, kinv, defgrad, cauchy_stress, bond_damage, force, M,
                              st, s)))
     return rc;
+  ws.release();
   return check_status(st, s);
 }
 

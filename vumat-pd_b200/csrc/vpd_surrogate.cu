@@ -307,6 +307,7 @@ int train_surrogate(const vpd_surrogate_config &cfg, uint16_t *w_out, float *b_o
                            cudaMemcpyDeviceToHost, s));
   unsigned long long nplastic = 0;
   VPD_CUDA(cudaMemcpyAsync(&nplastic, plastic, sizeof nplastic, cudaMemcpyDeviceToHost, s));
+  buf.release();
   VPD_CUDA(cudaStreamSynchronize(s));
   if (herr)
     return set_error(VPD_ERR_CUDA, "vpd_train_surrogate: tensor-core wait timed out");
@@ -625,6 +626,8 @@ extern "C" int vpd_surrogate_samples(const double *props, uint64_t seed, int64_t
   VPD_CUDA(cudaMemcpy(targets, Y, sizeof(float) * count * 16, cudaMemcpyDeviceToHost));
   if (records)
     VPD_CUDA(cudaMemcpy(records, R, sizeof(double) * count * VPD_SAMPLE_RECORD, cudaMemcpyDeviceToHost));
+  buf.release();
+  VPD_CUDA(cudaStreamSynchronize(0));
   return VPD_OK;
 }
 
