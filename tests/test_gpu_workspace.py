@@ -124,3 +124,20 @@ def test_idle_memory_is_bounded_when_a_call_returns():
     # (not free_bytes(): its synchronisation would give memory back too)
     assert before - torch.cuda.mem_get_info()[0] <= 256 << 20
     del first, second
+
+
+def test_idle_memory_is_given_back_on_request_and_with_a_handle():
+    from vpd.case import tensile_bar
+    rng = np.random.default_rng(4)
+    x = cuda(rng.random((100_000, 3)))
+    rows = vpd.build_neighbor_list(x, 0.04)
+    vpd.release_workspace()
+    before = free_bytes()
+    for give_back in (vpd.release_workspace, lambda: vpd.Simulation(tensile_bar(1)).close()):
+        again = vpd.build_neighbor_list(x, 0.04)
+        del again
+        assert free_bytes() < before  # the search's memory, idle
+        give_back()
+        give_back()  # (the second time with every kernel loaded)
+        assert free_bytes() == before
+    del rows

@@ -214,6 +214,7 @@ using namespace vpd;
 
 struct vpd_handle {
   vpd_case c{};
+  int device = -1;  // it was created on
   int64_t n = 0, nbonds = 0, sell_total = 0;
   cudaStream_t stream = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -251,7 +252,7 @@ template <typename T> int dalloc(vpd_handle *h, T **p, size_t count) {
   cudaError_t e = cudaMalloc(&q, bytes);
   if (e == cudaErrorMemoryAllocation) {  // again without the memory the workspace pool holds idle
     cudaGetLastError();
-    workspace_trim();
+    workspace_trim(h->device);
     e = cudaMalloc(&q, bytes);
   }
   VPD_CUDA(e);
@@ -374,6 +375,7 @@ int create_impl(vpd_handle *h, const vpd_case *c, const double *positions, const
   if ((rc = build_sets(*c, nominal, vol, sets)))
     return rc;
   trace.mark("host sets");
+  VPD_CUDA(cudaGetDevice(&h->device));
   VPD_CUDA(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking));
   VPD_CUDA(cudaEventCreate(&h->ev0));
   VPD_CUDA(cudaEventCreate(&h->ev1));
@@ -799,8 +801,9 @@ int vpd_create(const vpd_case *c, const double *positions, const double *volumes
 
 int vpd_destroy(vpd_handle *h) {
   if (h) {
+    const int device = h->device;
     destroy_impl(h);
-    workspace_trim();
+    workspace_trim(device);
   }
   return VPD_OK;
 }

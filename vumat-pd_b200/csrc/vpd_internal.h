@@ -25,10 +25,10 @@ int cuda_error(cudaError_t e, const char *what);
 // Device memory that a call needs only until the work it queues on `stream` has run: taken from a
 // memory pool of this library (one per device, stream-ordered, so safe with any streams and
 // threads) and returned to it in stream order. The pool keeps at most kWorkspaceKeep bytes of idle
-// memory at the next synchronisation; vpd_destroy gives that back too (workspace_trim).
+// memory at the next synchronisation; vpd_destroy and vpd_release_workspace give that back too (workspace_trim).
 constexpr uint64_t kWorkspaceKeep = uint64_t(256) << 20;
 int workspace_alloc(void **p, size_t bytes, cudaStream_t stream);
-void workspace_trim();
+int workspace_trim(int device);
 inline void workspace_free(void *p, cudaStream_t stream) {
   if (p)
     cudaFreeAsync(p, stream);

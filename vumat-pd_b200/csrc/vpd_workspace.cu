@@ -51,13 +51,19 @@ int workspace_alloc(void **p, size_t bytes, cudaStream_t stream) {
   return VPD_OK;
 }
 
-void workspace_trim() {
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices)
-    return;
+int workspace_trim(int dev) {
+  if (dev < 0 || dev >= kMaxDevices)
+    return VPD_OK;
   std::lock_guard<std::mutex> lock(g_pool_mutex);
   if (g_pools[dev])
-    cudaMemPoolTrimTo(g_pools[dev], 0);
+    VPD_CUDA(cudaMemPoolTrimTo(g_pools[dev], 0));
+  return VPD_OK;
 }
 
 }  // namespace vpd
+
+extern "C" int vpd_release_workspace(void) {
+  int dev = 0;
+  VPD_CUDA(cudaGetDevice(&dev));
+  return vpd::workspace_trim(dev);
+}

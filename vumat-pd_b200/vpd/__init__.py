@@ -309,6 +309,11 @@ def _stream():
     return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
 
 
+def release_workspace():
+    """Gives the memory that the library's pool holds idle between calls (at most 256 MiB) back to the current device."""
+    _check(library().vpd_release_workspace())
+
+
 def build_neighbor_list(positions, horizon: float):
     """buildNeighborList on a CUDA float64 tensor [n,3] -> (row_ptr int64[n+1], col int32)."""
     import torch
