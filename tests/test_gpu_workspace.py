@@ -128,16 +128,15 @@ def test_idle_memory_is_bounded_when_a_call_returns():
 
 def test_idle_memory_is_given_back_on_request_and_with_a_handle():
     from vpd.case import tensile_bar
-    rng = np.random.default_rng(4)
-    x = cuda(rng.random((100_000, 3)))
-    rows = vpd.build_neighbor_list(x, 0.04)
+    w = torch.zeros(vpd.MLP_WEIGHTS, dtype=torch.int16, device="cuda")
+    b = torch.zeros(vpd.MLP_PARAMS - vpd.MLP_WEIGHTS, dtype=torch.float32, device="cuda")
+    x = torch.randn((100_000, 16), dtype=torch.float32, device="cuda")
+    vpd.mlp_gradients(w, b, x[:128], x[:128])
+    vpd.Simulation(tensile_bar(1)).close()  # every kernel loaded
     vpd.release_workspace()
     before = free_bytes()
-    for give_back in (vpd.release_workspace, lambda: vpd.Simulation(tensile_bar(1)).close()):
-        again = vpd.build_neighbor_list(x, 0.04)
-        del again
-        assert free_bytes() < before  # the search's memory, idle
+    for give_back, left in ((vpd.release_workspace, 0), (lambda: vpd.Simulation(tensile_bar(1)).close(), 32 << 20)):
+        vpd.mlp_gradients(w, b, x, x)  # 117 MB of partial gradients
+        assert before - free_bytes() > 100_000_000
         give_back()
-        give_back()  # (the second time with every kernel loaded)
-        assert free_bytes() == before
-    del rows
+        assert before - free_bytes() <= left

@@ -803,7 +803,7 @@ int vpd_destroy(vpd_handle *h) {
   if (h) {
     const int device = h->device;
     destroy_impl(h);
-    workspace_trim(device);
+    workspace_trim(device, kWorkspaceSmall);
   }
   return VPD_OK;
 }

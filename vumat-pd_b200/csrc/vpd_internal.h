@@ -25,10 +25,11 @@ int cuda_error(cudaError_t e, const char *what);
 // Device memory that a call needs only until the work it queues on `stream` has run: taken from a
 // memory pool of this library (one per device, stream-ordered, so safe with any streams and
 // threads) and returned to it in stream order. The pool keeps at most kWorkspaceKeep bytes of idle
-// memory at the next synchronisation; vpd_destroy and vpd_release_workspace give that back too (workspace_trim).
-constexpr uint64_t kWorkspaceKeep = uint64_t(256) << 20;
+// memory at the next synchronisation. vpd_release_workspace gives that back too, vpd_destroy all but kWorkspaceSmall (the
+// pool's smallest step: given back, it cost the next vpd_create 0.25 ms of 1.25 to map again, and vpd_destroy 0.2).
+constexpr uint64_t kWorkspaceKeep = uint64_t(256) << 20, kWorkspaceSmall = uint64_t(32) << 20;
 int workspace_alloc(void **p, size_t bytes, cudaStream_t stream);
-int workspace_trim(int device);
+int workspace_trim(int device, uint64_t keep = 0);
 inline void workspace_free(void *p, cudaStream_t stream) {
   if (p)
     cudaFreeAsync(p, stream);
@@ -38,24 +39,31 @@ struct Workspace {
   Workspace(const Workspace &) = delete;
   Workspace &operator=(const Workspace &) = delete;
   ~Workspace() { release(); }
-  // Gives everything back in stream order. Before a call's last synchronisation, so that the pool's bound holds when
-  // the call returns (memory given back after it stays idle until the next one).
+  // Gives everything back in stream order.
   void release() {
     while (used > 0)
       workspace_free(ptrs[--used], stream);
   }
+  // Before a call's last synchronisation: gives a large workspace back, so that the pool's bound holds when the call
+  // returns (memory given back after it stays idle until the next one). Small ones need not: 2.5 us of a call.
+  void finish() {
+    if (bytes >= kWorkspaceSmall)
+      release();
+  }
   template <typename T> int alloc(T **p, size_t count) {
     if (used == kMax)
       return set_error(VPD_ERR_CAPACITY, "workspace slots exhausted");
-    const int rc = workspace_alloc(&ptrs[used], (count ? count : 1) * sizeof(T), stream);
+    const size_t size = (count ? count : 1) * sizeof(T);
+    const int rc = workspace_alloc(&ptrs[used], size, stream);
     if (rc == VPD_OK)
-      *p = static_cast<T *>(ptrs[used++]);
+      *p = static_cast<T *>(ptrs[used++]), bytes += size;
     return rc;
   }
   static constexpr int kMax = 32;
   cudaStream_t stream;
   void *ptrs[kMax];
   int used = 0;
+  size_t bytes = 0;
 };
 
 // ---- device status word bits (ORed by kernels, read by the host) ----

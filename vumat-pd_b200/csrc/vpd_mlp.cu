@@ -534,11 +534,11 @@ int mlp_adam(const float *partials, int64_t blocks, float *p, float *m, float *v
 
 // ------------------------------------------------------------------ C ABI (device pointers)
 namespace {
-// The end of a call: its timeout word (in ws) read, its memory given back, its work done.
+// The end of a call: its timeout word (in ws) read, its work done.
 int check_err(unsigned *derr, vpd::Workspace &ws, cudaStream_t s) {
   unsigned e = 0;
   VPD_CUDA(cudaMemcpyAsync(&e, derr, sizeof e, cudaMemcpyDeviceToHost, s));
-  ws.release();
+  ws.finish();
   VPD_CUDA(cudaStreamSynchronize(s));
   if (e)
     return vpd::set_error(VPD_ERR_CUDA, "surrogate network: tensor-core wait timed out");

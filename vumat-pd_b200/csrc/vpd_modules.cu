@@ -720,9 +720,13 @@ int vpd_build_neighbor_list(const double *positions, int64_t n, double horizon, 
   if (rc == VPD_OK && col)
     rc = neighbor_fill(xv, n, row_ptr, col, grid, scr, s);
   neighbor_scratch_free(scr);
-  ws.release();
-  const cudaError_t e = cudaStreamSynchronize(s);
-  return rc == VPD_OK && e != cudaSuccess ? cuda_error(e, "neighbour list") : rc;
+  if (ws.bytes >= kWorkspaceSmall / 2) {  // (the search's own scratch is about as large as the packed positions)
+    ws.release();
+    const cudaError_t e = cudaStreamSynchronize(s);
+    if (rc == VPD_OK && e != cudaSuccess)
+      rc = cuda_error(e, "neighbour list");
+  }
+  return rc;
 }
 
 int vpd_shape_tensor_inverse(const double *positions, const double *volumes, int64_t n,
@@ -771,7 +775,7 @@ int vpd_force_density(const double *positions, const double *volumes, int64_t n,
   if ((rc = launch_csr_force(positions, volumes, n, row_ptr, col, kinv, defgrad, cauchy_stress, bond_damage, force, M,
                              st, s)))
     return rc;
-  ws.release();
+  ws.finish();
   return check_status(st, s);
 }
 

@@ -307,7 +307,7 @@ int train_surrogate(const vpd_surrogate_config &cfg, uint16_t *w_out, float *b_o
                            cudaMemcpyDeviceToHost, s));
   unsigned long long nplastic = 0;
   VPD_CUDA(cudaMemcpyAsync(&nplastic, plastic, sizeof nplastic, cudaMemcpyDeviceToHost, s));
-  buf.release();
+  buf.finish();
   VPD_CUDA(cudaStreamSynchronize(s));
   if (herr)
     return set_error(VPD_ERR_CUDA, "vpd_train_surrogate: tensor-core wait timed out");

@@ -51,12 +51,12 @@ int workspace_alloc(void **p, size_t bytes, cudaStream_t stream) {
   return VPD_OK;
 }
 
-int workspace_trim(int dev) {
+int workspace_trim(int dev, uint64_t keep) {
   if (dev < 0 || dev >= kMaxDevices)
     return VPD_OK;
   std::lock_guard<std::mutex> lock(g_pool_mutex);
   if (g_pools[dev])
-    VPD_CUDA(cudaMemPoolTrimTo(g_pools[dev], 0));
+    VPD_CUDA(cudaMemPoolTrimTo(g_pools[dev], keep));
   return VPD_OK;
 }
 
