@@ -350,53 +350,32 @@ __device__ __forceinline__ void put9(TensorTile &tile, const double (&v)[9]) {
     tile[9 * threadIdx.x + c] = v[c];
 }
 
-// (less than a block of points: read and written by their threads, which is 3 us shorter, 10 with an odd count: 53 | 63
-// us of a call on one point)
 constexpr int kCorotationalTiles = 5;
-template <bool TILES>
 __global__ void __launch_bounds__(kPointThreads, 4)
     k_corotational(int64_t n, const double *fN, const double *fNP1, const double *vN, const double *rN, double dt,
                    double *dbar, double *spin, double *rNew, double *vNew, double *strain, unsigned *status) {
   extern __shared__ __align__(16) double s_points[];
   TensorTile *tile = reinterpret_cast<TensorTile *>(s_points);
-  const int64_t first = (int64_t)blockIdx.x * kPointThreads, own = 9 * (first + threadIdx.x);
+  const int64_t first = (int64_t)blockIdx.x * kPointThreads;
   const int count = (int)min((int64_t)kPointThreads, n - first);
-  if (TILES) {
-    tile_in(fN, tile[0], first, count), tile_in(fNP1, tile[1], first, count);
-    tile_in(vN, tile[2], first, count), tile_in(rN, tile[3], first, count);
-    tiles_ready();
-  }
-  auto get = [&](int t, const double *src, double (&v)[9]) {
-    if (TILES)
-      get9(tile[t], v);
-    else
-      for (int c = 0; c < 9; ++c)
-        v[c] = src[own + c];
-  };
-  auto put = [&](int t, double *dst, const double (&v)[9]) {
-    if (TILES)
-      put9(tile[t], v);
-    else
-      for (int c = 0; c < 9; ++c)
-        dst[own + c] = v[c];
-  };
+  tile_in(fN, tile[0], first, count), tile_in(fNP1, tile[1], first, count);
+  tile_in(vN, tile[2], first, count), tile_in(rN, tile[3], first, count);
+  tiles_ready();
   if ((int)threadIdx.x < count) {
     double a[9], b[9], v[9], r[9];
-    get(0, fN, a), get(1, fNP1, b), get(2, vN, v), get(3, rN, r);
+    get9(tile[0], a), get9(tile[1], b), get9(tile[2], v), get9(tile[3], r);
     Corotational co;
     if (!corotational_update(a, b, v, r, dt, co))
       atomicOr(status, STATUS_SINGULAR_KINEMATICS);
     double e6[6], e[9];
     green_lagrange6(b, e6);
     voigt_to_full(e6, e);
-    put(0, dbar, co.dbar), put(1, spin, co.spin), put(2, vNew, co.v), put(3, rNew, co.r), put(4, strain, e);
+    put9(tile[0], co.dbar), put9(tile[1], co.spin), put9(tile[2], co.v), put9(tile[3], co.r), put9(tile[4], e);
   }
-  if (TILES) {
-    __syncthreads();
-    tile_out(dbar, tile[0], first, count), tile_out(spin, tile[1], first, count);
-    tile_out(vNew, tile[2], first, count), tile_out(rNew, tile[3], first, count);
-    tile_out(strain, tile[4], first, count);
-  }
+  __syncthreads();
+  tile_out(dbar, tile[0], first, count), tile_out(spin, tile[1], first, count);
+  tile_out(vNew, tile[2], first, count), tile_out(rNew, tile[3], first, count);
+  tile_out(strain, tile[4], first, count);
 }
 
 // VumatPdCorrespondenceMaterial::update for one point (:155-170,195-210).
@@ -813,14 +792,11 @@ int vpd_corotational_update(int64_t n, const double *defgrad_old, const double *
   VPD_CUDA(cudaMemsetAsync(st, 0, sizeof(unsigned), s));
   if (n <= 0)
     return check_status(st, s);
-  const bool tiles = n >= kPointThreads;
-  const size_t smem = tiles ? kCorotationalTiles * sizeof(TensorTile) : 0;
-  auto *kernel = tiles ? k_corotational<true> : k_corotational<false>;
-  if (tiles)
-    VPD_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  kernel<<<blocks(n), kPointThreads, smem, s>>>(n, defgrad_old, defgrad_new, stretch_old, rotation_old, dt,
-                                                rate_of_deformation, relative_spin, rotation_new, stretch_new,
-                                                strain_new, st);
+  VPD_CUDA(cudaFuncSetAttribute(k_corotational, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)(kCorotationalTiles * sizeof(TensorTile))));
+  k_corotational<<<blocks(n), kPointThreads, kCorotationalTiles * sizeof(TensorTile), s>>>(n, defgrad_old, defgrad_new, stretch_old, rotation_old, dt,
+                                           rate_of_deformation, relative_spin, rotation_new, stretch_new,
+                                           strain_new, st);
   VPD_CUDA(cudaGetLastError());
   return check_status(st, s);
 }
