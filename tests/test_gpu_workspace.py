@@ -120,7 +120,7 @@ def test_idle_memory_is_bounded_when_a_call_returns():
     x = torch.randn((400_000, 16), dtype=torch.float32, device="cuda")
     first = vpd.mlp_gradients(w, b, x[:128], x[:128])
     before = free_bytes()
-    second = vpd.mlp_gradients(w, b, x, x)  # 466 MB of partial gradients
+    second = vpd.mlp_gradients(w, b, x, x)  # 466 MB of partial gradients in all
     # (not free_bytes(): its synchronisation would give memory back too)
     assert before - torch.cuda.mem_get_info()[0] <= 256 << 20
     del first, second
@@ -140,3 +140,20 @@ def test_idle_memory_is_given_back_on_request_and_with_a_handle():
         assert before - free_bytes() > 100_000_000
         give_back()
         assert before - free_bytes() <= left
+
+
+def test_gradients_in_parts_sum_in_the_same_order():
+    """A batch beyond the rows whose partial gradients are held at once (7 x 148 blocks of 128 rows): the rows after them
+    add to the sum of those before, block by block, so a zero output gradient leaves it as it was."""
+    rows = 7 * 148 * 128
+    g = torch.Generator(device="cuda").manual_seed(5)
+    w = (0.1 * torch.randn(vpd.MLP_WEIGHTS, generator=g, device="cuda")).to(torch.bfloat16).view(torch.int16)
+    b = 0.1 * torch.randn(vpd.MLP_PARAMS - vpd.MLP_WEIGHTS, generator=g, device="cuda")
+    x, gout = (torch.randn((rows + 129, 16), generator=g, device="cuda") for _ in range(2))
+    first, rest = vpd.mlp_gradients(w, b, x[:rows], gout[:rows]), vpd.mlp_gradients(w, b, x[rows:], gout[rows:])
+    both = vpd.mlp_gradients(w, b, x, gout)
+    # one float addition against another order of the last 129 rows' sum
+    assert (both - (first + rest)).abs().max() <= 4 * 2.0 ** -23 * (first.abs() + rest.abs()).max()
+    assert rest.abs().max() > 0
+    gout[rows:] = 0.0
+    assert torch.equal(vpd.mlp_gradients(w, b, x, gout), first)

@@ -460,18 +460,18 @@ __global__ void __launch_bounds__(kGradThreads, 1) k_mlp_gradient(MlpWeights w, 
     umma::tmem_dealloc(tmem, 512);
 }
 
-// sum over blocks b (in order) of partials[b][i]
-__device__ __forceinline__ float partial_sum(const float *partials, int nblocks, int i) {
-  float s = 0.0f;
+// s + the sum over blocks b (in order) of partials[b][i]
+__device__ __forceinline__ float partial_sum(const float *partials, int nblocks, int i, float s = 0.0f) {
 #pragma unroll 32
   for (int b = 0; b < nblocks; ++b)
     s += partials[(size_t)b * kMlpParams + i];
   return s;
 }
-__global__ void k_sum_partials(const float *partials, int nblocks, float *grad) {
+// (first: the sum begins with these partials, else grad holds that of the blocks before them)
+__global__ void k_sum_partials(const float *partials, int nblocks, float *grad, bool first) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < kMlpParams)
-    grad[i] = partial_sum(partials, nblocks, i);
+    grad[i] = partial_sum(partials, nblocks, i, first ? 0.0f : grad[i]);
 }
 
 // One Adam step on the summed gradient; the weights (the first kMlpWeights parameters) also to their BF16 copy, in
@@ -515,8 +515,8 @@ int mlp_gradient_partials(const MlpWeights &w, const MlpBatch &batch, int64_t B,
 
 constexpr unsigned kParamBlocks = (unsigned)((kMlpParams + 127) / 128);
 
-int mlp_sum_partials(const float *partials, int64_t blocks, float *grad, cudaStream_t s) {
-  k_sum_partials<<<kParamBlocks, 128, 0, s>>>(partials, (int)blocks, grad);
+int mlp_sum_partials(const float *partials, int64_t blocks, float *grad, bool first, cudaStream_t s) {
+  k_sum_partials<<<kParamBlocks, 128, 0, s>>>(partials, (int)blocks, grad, first);
   VPD_CUDA(cudaGetLastError());
   return VPD_OK;
 }
@@ -570,18 +570,24 @@ extern "C" int vpd_mlp_gradients(const uint16_t *weights, const float *biases, c
     return set_error(VPD_ERR_INVALID, "vpd_mlp_gradients: invalid argument");
   cudaStream_t s = (cudaStream_t)stream;
   const MlpWeights w = mlp_weights(reinterpret_cast<const __nv_bfloat16 *>(weights), biases);
+  // in parts of at most kPartBlocks blocks, whose partials (154 MB) stay within what the pool keeps; the sum runs on over
+  // the parts in block order
+  constexpr int64_t kPartBlocks = 7 * 148;
   const int64_t blocks = mlp_gradient_blocks(batch);
   Workspace ws(s);
   unsigned *derr = nullptr;
   float *partials = nullptr;
   int rc;
-  if ((rc = ws.alloc(&derr, 1)) || (rc = ws.alloc(&partials, (size_t)blocks * kMlpParams)))
+  if ((rc = ws.alloc(&derr, 1)) || (rc = ws.alloc(&partials, (size_t)std::min(blocks, kPartBlocks) * kMlpParams)))
     return rc;
   VPD_CUDA(cudaMemsetAsync(derr, 0, sizeof(unsigned), s));
-  MlpBatch rows{};
-  rows.x = x, rows.gout = gout;
-  if ((rc = mlp_gradient_partials(w, rows, batch, partials, derr, s)) ||
-      (rc = mlp_sum_partials(partials, blocks, grad, s)))
-    return rc;
+  for (int64_t b = 0; b < blocks; b += kPartBlocks) {
+    const int64_t row = 128 * b, count = std::min(kPartBlocks, blocks - b);
+    MlpBatch rows{};
+    rows.x = x + row * kMlpIn, rows.gout = gout + row * kMlpOut;
+    if ((rc = mlp_gradient_partials(w, rows, std::min(batch - row, 128 * count), partials, derr, s)) ||
+        (rc = mlp_sum_partials(partials, count, grad, b == 0, s)))
+      return rc;
+  }
   return check_err(derr, ws, s);
 }

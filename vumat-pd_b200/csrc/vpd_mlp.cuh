@@ -61,8 +61,8 @@ struct MlpBatch {
 };
 int mlp_gradient_partials(const MlpWeights &w, const MlpBatch &batch, int64_t B, float *partials, unsigned *err,
                           cudaStream_t s);
-// grad [kMlpParams] = the partials' sum in block order.
-int mlp_sum_partials(const float *partials, int64_t blocks, float *grad, cudaStream_t s);
+// grad [kMlpParams] = the partials' sum in block order (first: from 0, else from what grad holds).
+int mlp_sum_partials(const float *partials, int64_t blocks, float *grad, bool first, cudaStream_t s);
 // The same sum taken straight into one Adam step on the parameters p (m, v: moments); wb: the weights' BF16 copy
 // (tiled storage).
 int mlp_adam(const float *partials, int64_t blocks, float *p, float *m, float *v, __nv_bfloat16 *wb, float lr,
