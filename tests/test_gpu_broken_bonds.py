@@ -53,3 +53,11 @@ def test_pair_block_shapes_mixed(monkeypatch, dims):
     nx, ny, nz = dims
     case = tensile_bar(3, nx=nx, ny=ny, nz=nz, damage_mode=1, damage_initiation=0.001, precision=PRECISION_MIXED)
     run(case, monkeypatch, ("planes", "pair"), 60)
+
+
+# a stencil of 16 mask words and more takes 256 threads from the first wave on; 15 and fewer 128
+@pytest.mark.parametrize("ratio", [4.4, 4.515, 5.015])
+def test_pair_block_shapes_of_long_stencils_mixed(monkeypatch, ratio):
+    case = tensile_bar(3, nx=1000, ny=20, nz=10, horizon=ratio * 0.1, damage_mode=1, damage_initiation=0.001,
+                       precision=PRECISION_MIXED)
+    run(case, monkeypatch, ("planes", "pair"), 60)

@@ -964,7 +964,9 @@ template <typename F> static void with_plane_threads(const StepParams &p, F &&la
 // cross-sections from 8 x 3 to 50 x 50, 128 | 192 | 256: horizon 3.015 h without damage, 62,000 points 28-30 | 33-35 |
 // 28-30, 154,000 43-49 | 40-44 | 46-52 (one wave of 192), 400,000 81-86 | 91-101 | 86-92, 1M 180-194 | 190-212 |
 // 187-201; with damage 400,000 124-135 | 145-150 | 130-135, 650,000 196-209 | 211-224 | 195-202, 1M 293-312 | 312-335 |
-// 286-299.
+// 286-299. Long stencils with damage, 128 | 256: 4.515 h, 200,000 points 216 | 209 and 219 | 209, 384,000 375 | 363; 5.515 h,
+// 189,000 382 | 341, 200,000 392 | 342, 384,000 665 | 612 (4.015 h: 155 | 151 and 256 | 256).
+constexpr int kLongStencil = 16;  // mask words: horizons of about 4.5 spacings and more
 template <bool DAMAGE, bool UNROLL> static void launch_deformation_pair(const StepParams &p, cudaStream_t s) {
   const double waves = tile_waves<2>(p, 512);
   if (by_planes(p))
@@ -974,7 +976,7 @@ template <bool DAMAGE, bool UNROLL> static void launch_deformation_pair(const St
     });
   else if (waves > 1.01 && tile_waves<2>(p, 576) <= 1.0)
     k_deformation_pair<DAMAGE, UNROLL, 192, 3><<<tiled_blocks<2, 192>(p), 192, 0, s>>>(p);
-  else if (halves_together(waves) || (DAMAGE && waves > 3.0))
+  else if (halves_together(waves) || (DAMAGE && (waves > 3.0 || p.st.nw >= kLongStencil)))
     k_deformation_pair<DAMAGE, UNROLL, 256, 2><<<tiled_blocks<2, 256>(p), 256, 0, s>>>(p);
   else
     k_deformation_pair<DAMAGE, UNROLL, 128, 4><<<tiled_blocks<2, 128>(p), 128, 0, s>>>(p);
