@@ -55,9 +55,20 @@ def test_pair_block_shapes_mixed(monkeypatch, dims):
     run(case, monkeypatch, ("planes", "pair"), 60)
 
 
-# a stencil of 16 mask words and more takes 256 threads from the first wave on; 15 and fewer 128
-@pytest.mark.parametrize("ratio", [4.4, 4.515, 5.015])
+# stencils on either side of 16 and 22 mask words, from where on the blocks are larger
+@pytest.mark.parametrize("ratio", [4.4, 4.515, 4.9, 5.015])
 def test_pair_block_shapes_of_long_stencils_mixed(monkeypatch, ratio):
     case = tensile_bar(3, nx=1000, ny=20, nz=10, horizon=ratio * 0.1, damage_mode=1, damage_initiation=0.001,
                        precision=PRECISION_MIXED)
     run(case, monkeypatch, ("planes", "pair"), 60)
+
+
+# wide cross-sections: last waves of the deformation blocks filled by 0.37, 0.58 and 0.26
+@pytest.mark.parametrize("dims", [(100, 45, 45), (150, 40, 40), (70, 70, 70)])
+@pytest.mark.parametrize("ratio", [3.015, 4.015, 5.015])
+def test_block_shapes_of_wide_cross_sections(monkeypatch, dims, ratio):
+    nx, ny, nz = dims
+    for precision, kinds in ((PRECISION_MIXED, ("planes", "pair")), (PRECISION_FP64, ("slot", "tiles"))):
+        case = tensile_bar(3, nx=nx, ny=ny, nz=nz, horizon=ratio * 0.1, damage_mode=1, damage_initiation=0.001,
+                           precision=precision)
+        run(case, monkeypatch, kinds, 60)

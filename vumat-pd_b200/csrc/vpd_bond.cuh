@@ -179,6 +179,19 @@ static inline double wave_cost(double waves) {
 // 400,000.)
 static inline bool halves_together(double waves) { return waves <= 2.0 && waves - (std::ceil(waves) - 1.0) > 0.76; }
 
+// Lattices whose planes along y and z are wider than a block's tiles: two halves of a block of 256 share more of their
+// windows than two blocks of 128 on an SM do, the more the longer the stencil.
+static inline bool wide_planes(const StepParams &p) { return (int64_t)p.lat_nz * ((p.lat_ny + 1) / 2) >= 512; }
+// Stencil lengths in mask words: four spacings have 11, 4.5 have 16, five 22.
+constexpr int kMiddleStencil = 11, kLongStencil = 16, kLongestStencil = 22;
+// Where a last wave is about half full, the smaller blocks spread it better (150x40x40, 1.58 waves: 3 % of an increment
+// up to 4.5 spacings; 1.37, 2.26 and 3.30 waves lose 1 to 3 % with them).
+static inline bool half_wave(double waves) { return waves - std::floor(waves) >= 0.45; }
+static inline bool wide_halves(const StepParams &p, double waves) { return wide_planes(p) && !half_wave(waves); }
+static inline bool long_halves(const StepParams &p, double waves) {
+  return p.st.nw >= kLongestStencil || (p.st.nw >= kLongStencil && !half_wave(waves));
+}
+
 // 32-bit window indices need every index within a stencil reach of the lattice below 2^31
 static inline bool index32(const StepParams &p) { return p.n < (int64_t(1) << 30); }
 

@@ -966,7 +966,7 @@ template <typename F> static void with_plane_threads(const StepParams &p, F &&la
 // 187-201; with damage 400,000 124-135 | 145-150 | 130-135, 650,000 196-209 | 211-224 | 195-202, 1M 293-312 | 312-335 |
 // 286-299. Long stencils with damage, 128 | 256: 4.515 h, 200,000 points 216 | 209 and 219 | 209, 384,000 375 | 363; 5.515 h,
 // 189,000 382 | 341, 200,000 392 | 342, 384,000 665 | 612 (4.015 h: 155 | 151 and 256 | 256).
-constexpr int kLongStencil = 16;  // mask words: horizons of about 4.5 spacings and more
+// With damage on a wide cross-section the same at any length: 100x45x45 at 3.015 h 86 | 84, at 4.015 h 155 | 151.
 template <bool DAMAGE, bool UNROLL> static void launch_deformation_pair(const StepParams &p, cudaStream_t s) {
   const double waves = tile_waves<2>(p, 512);
   if (by_planes(p))
@@ -976,7 +976,7 @@ template <bool DAMAGE, bool UNROLL> static void launch_deformation_pair(const St
     });
   else if (waves > 1.01 && tile_waves<2>(p, 576) <= 1.0)
     k_deformation_pair<DAMAGE, UNROLL, 192, 3><<<tiled_blocks<2, 192>(p), 192, 0, s>>>(p);
-  else if (halves_together(waves) || (DAMAGE && (waves > 3.0 || p.st.nw >= kLongStencil)))
+  else if (halves_together(waves) || (DAMAGE && (waves > 3.0 || long_halves(p, waves) || wide_halves(p, waves))))
     k_deformation_pair<DAMAGE, UNROLL, 256, 2><<<tiled_blocks<2, 256>(p), 256, 0, s>>>(p);
   else
     k_deformation_pair<DAMAGE, UNROLL, 128, 4><<<tiled_blocks<2, 128>(p), 128, 0, s>>>(p);
@@ -1006,15 +1006,19 @@ int launch_deformation_tiled(const StepParams &p, cudaStream_t s) {
 // without damage 62,000 points 26-32 | 28-36 | 26-32, 154,000 43-69 | 38-48 | 44-71, 260,000 60-80 | 60-88 | 61-81,
 // 400,000 84-117 | 86-127 | 87-118, 650,000 130-181 | 125-170 | 132-188, 1M 185-258 | 180-250 | 191-263; with damage
 // 154,000 46-69 | 42-51 | 47-69, 650,000 135-181 | 138-176 | 138-184, 1M 195-260 | 199-258 | 202-266.
+// Long stencils on wide cross-sections, 128 | 192 | 256: 100x45x45 at 5.515 h 230 | 234 | 210 and with damage 243 | 270 |
+// 231, 200x50x50 with damage 485 | 494 | 466.
 template <bool DAMAGE, bool UNROLL> static void launch_force_pair(const StepParams &p, cudaStream_t s) {
+  const bool long_wide = wide_planes(p) && long_halves(p, tile_waves<2>(p, 512));
   if (by_planes(p))
     with_plane_threads(p, [&](auto threads, auto minb) {
       k_force_planes<DAMAGE, UNROLL, decltype(threads)::value, decltype(minb)::value>
           <<<tiled_blocks<2, 32>(p), 32 * p.st.nplanes, sizeof(float2) * 96 * p.st.nplanes, s>>>(p);
     });
-  else if ((DAMAGE ? 1.2 : 1.1) * wave_cost(tile_waves<2>(p, 576)) < wave_cost(tile_waves<2>(p, 512)))
+  else if (!(DAMAGE && long_wide) &&
+           (DAMAGE ? 1.2 : 1.1) * wave_cost(tile_waves<2>(p, 576)) < wave_cost(tile_waves<2>(p, 512)))
     k_force_pair<DAMAGE, UNROLL, 192, 3><<<tiled_blocks<2, 192>(p), 192, 0, s>>>(p);
-  else if (halves_together(tile_waves<2>(p, 512)))
+  else if (halves_together(tile_waves<2>(p, 512)) || long_wide)
     k_force_pair<DAMAGE, UNROLL, 256, 2><<<tiled_blocks<2, 256>(p), 256, 0, s>>>(p);
   else
     k_force_pair<DAMAGE, UNROLL, 128, 4><<<tiled_blocks<2, 128>(p), 128, 0, s>>>(p);

@@ -297,7 +297,8 @@ __global__ void __launch_bounds__(TPB, MINB) k_force_tiled64(const __grid_consta
 // Deformation, microseconds by shape (1 x 128 six blocks per SM | 2 x 128 four | 3 x 384 one; the one shape before
 // was 2 x 256, two blocks) at horizon 4.015 h without damage: 20,400 points 42 | 49 | 90 (57), 54,000 53 | 60 |
 // 91 (57), 108,900 87 | 76 | 94 (89), 154,000 140 | 111 | 97 (119), 250,000 213 | 155 | 181 (166), 1M 692 | 523 | 526
-// (529); from rest with damage: 20,400 67 | 95 | 159 (104), 108,900 125 | 127 | 160 (140), 154,000 191 | 206 | 165
+// (529); 2 x 128 | 2 x 256 on wide cross-sections, 100x45x45 at 3.015 h 71 | 67, at 5.515 h 299 | 287, with damage 125 |
+// 116 and 572 | 521; from rest with damage: 20,400 67 | 95 | 159 (104), 108,900 125 | 127 | 160 (140), 154,000 191 | 206 | 165
 // (207), 250,000 293 | 260 | 317 (270), 1M 982 | 894 | 933 (896).
 // Force (1 x 128 four blocks per SM | 3 x 128 three | 3 x 384 one, the one shape before): 20,400 points 48 | 67 |
 // 108, 40,900 64 | 67 | 105, 54,000 69 | 67 | 101, 108,900 161 | 93 | 106, 154,000 189 | 125 | 113, 1M 1077 | 689 | 617.
@@ -322,7 +323,7 @@ int launch_deformation_tiled64(const StepParams &p, cudaStream_t s) {
   const double three = (p.damage ? 1.25 : 1.11) * std::ceil(tile_waves<3>(p, 384));
   if (one <= (p.damage ? 1.0 : 0.75))
     deformation_tiled64<1, 128, 6>(p, s);
-  else if (two <= three && halves_together(tile_waves<2>(p, 512)))
+  else if (two <= three && (halves_together(tile_waves<2>(p, 512)) || wide_halves(p, tile_waves<2>(p, 512))))
     deformation_tiled64<2, kBondThreads, 2>(p, s);
   else if (two <= three)
     deformation_tiled64<2, 128, 4>(p, s);
@@ -352,12 +353,15 @@ int launch_force_tiled64(const StepParams &p, cudaStream_t s) {
   // 0.689 in 128-thread blocks, 0.787 for four points in 512-thread blocks and 0.821 for four points in two
   // 256-thread blocks per SM. Lattices that leave most of its blocks or a wave empty take the smaller blocks, the
   // smallest lattices single points.
+  // On wide cross-sections the smaller blocks cost more with longer stencils: 3 x 128 | 3 x 384, 70x70x70 at 3.015 h
+  // 142 | 143, at 4.015 h 282 | 269, at 5.515 h 637 | 568; 100x45x45 205 | 211 at 4.015 h, 498 | 467 at 5.515 h.
   const double waves = tile_waves<3>(p, 384);
+  const double small = !wide_planes(p) || p.st.nw < kMiddleStencil ? 1.14 : (p.st.nw < kLongStencil ? 1.2 : 1.3);
   if (p.tiled == 3)
     force_tiled64<2, kBondThreads, 2>(p, s);
   else if (tile_waves<1>(p, 512) <= 0.6)
     force_tiled64<1, 128, 4>(p, s);
-  else if (1.14 * wave_cost(waves) < std::ceil(waves))
+  else if (small * wave_cost(waves) < std::ceil(waves))
     force_tiled64<3, 128, 3>(p, s);
   else
     force_tiled64<3, 384, 1>(p, s);
