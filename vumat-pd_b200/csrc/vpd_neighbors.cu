@@ -411,14 +411,13 @@ __global__ void k_cell_load(int64_t ncells, GridDev g, const int64_t *cell_start
   }
 }
 
-// Blocks per cell: one, unless the busiest cell has more pairs than a fair share of the GPU's four blocks per SM
-// (a body of a few cells, or a cluster among sparse points); each block then searches for some of the cell's points, 32
-// or more. The two calls that build the list, microseconds, a block per cell | so: 3,375 points in one cell 9938 | 415,
-// 2,744 points in eight cells 5376 | 415 (3200 both with a warp per point and allocations in the calls).
+// Blocks per cell: one, unless the busiest cell has more than twice its share of the pairs of one block per SM (a body of
+// a few cells, or a cluster among sparse points); each block then searches for some of the cell's points, 32 or more, and
+// sorts the candidates again. The two calls that build the list, microseconds, a block per cell | so: 3,375 points in one
+// cell 9938 | 467, 2,744 points in eight cells 5376 | 442 (3200 both with a warp per point and allocations in the calls).
 static int cell_blocks(const unsigned long long *load) {
-  const unsigned long long fair = std::max(load[3] / (4 * 148), 32 * load[0]);
-  const unsigned long long wanted = (load[2] + fair - 1) / fair;
-  return (int)std::min(wanted, (load[1] + 31) / 32);
+  const unsigned long long share = std::max(load[3] / 148, 32 * load[0]);
+  return (int)std::max(1ull, std::min(load[2] / share, (load[1] + 31) / 32));
 }
 
 // Ascending bitonic sort of `width` (a power of two, at least 32) shared-memory ints by the whole block.
