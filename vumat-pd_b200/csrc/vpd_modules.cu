@@ -30,30 +30,31 @@ __global__ void k_pack_positions(const double *pos, int64_t n, double4 *xv) {
 constexpr int kRowThreads = 256;
 
 // Bodies below kLargeBody points take eight lanes a row. From there on the lanes follow the mean row length, which
-// only the device knows without a synchronisation: a grid has threads for four lanes per row, from kLargestBody on for
-// two; threads of fewer lanes than that end at once, those of more pass over two rows. Calls on lattices, microseconds,
+// only the device knows without a synchronisation: a grid has threads for four lanes per row, from kTwoLaneGrid on for
+// two; threads of fewer lanes than that end at once (3 to 10 % of a call over short rows at 1M points), those of more pass
+// over two rows (5 to 10 % over long ones at 154,000 to 315,000). Calls on lattices, microseconds,
 // one lane always | eight always | now: 250,000 points with 4 bonds each, deformation 18 | 47 | 19, damage 14 | 40 | 15,
 // with 28, 38 | 87 | 36 and 73 | 88 | 53; 1M points with 6, 61 | 200 | 63 and 52 | 163 | 52, with 118,
 // 548 | 770 | 533 and 1210 | 838 | 651; 108,000 points with 229, 198 | 133 | 122 and 394 | 169 | 164; the force sum of
 // 1M points with 6, eight always | now, 263 | 145.
-constexpr int64_t kLargeBody = 40000, kLargestBody = 150000;
+// With packed records (calls over long rows) eight lanes serve up to 100,000 points: damage of 50,000 points with 109
+// bonds, four | eight lanes 47 | 41, of 82,000 with 230, 135 | 124, of 108,000 with 229, 156 | 152.
+constexpr int64_t kLargeBody = 40000, kLargePackedBody = 100000, kShortRowBody = 150000, kTwoLaneGrid = 500000;
 __device__ __forceinline__ int row_lanes(int64_t n, const int64_t *row_ptr) {
   const int64_t bonds = __ldg(row_ptr + n) - __ldg(row_ptr);
-  if (n < kLargestBody)
+  if (n < kShortRowBody)
     return bonds < 24 * n ? 2 : 4;
   return bonds < 20 * n ? 1 : (bonds < 64 * n ? 2 : 4);
 }
-static unsigned row_blocks(int64_t n) {
-  const int64_t lanes = n < kLargeBody ? 8 : (n < kLargestBody ? 4 : 2);
-  return (unsigned)((n * lanes + kRowThreads - 1) / kRowThreads);
-}
-
-// launch(LARGE): the sums' kernels come in both forms.
-template <typename F> static void launch_rows(int64_t n, F &&launch) {
-  if (n < kLargeBody)
-    launch(std::false_type{});
+// launch(LARGE, blocks): the sums' kernels come in both forms.
+template <typename F> static void launch_rows(int64_t n, bool packed, F &&launch) {
+  const bool large = n >= (packed ? kLargePackedBody : kLargeBody);
+  const int64_t lanes = !large ? 8 : (n < kTwoLaneGrid ? 4 : 2);
+  const unsigned blocks = (unsigned)((n * lanes + kRowThreads - 1) / kRowThreads);
+  if (large)
+    launch(std::true_type{}, blocks);
   else
-    launch(std::true_type{});
+    launch(std::false_type{}, blocks);
 }
 
 // Calls pass(lanes, thread) for the calling thread's passes over the rows; whole warps make the same passes.
@@ -611,8 +612,8 @@ int launch_csr_force(const double *positions, const double *volumes, int64_t n, 
                      const int32_t *col, const double *kinv, const double *defgrad, const double *cauchy_stress,
                      const double *bond_damage, double *force, double *M, unsigned *status, cudaStream_t s) {
   k_csr_force_map<<<blocks(n), 128, 0, s>>>(cauchy_stress, defgrad, kinv, n, M, status);
-  launch_rows(n, [&](auto large) {
-    k_csr_force<decltype(large)::value><<<row_blocks(n), kRowThreads, 0, s>>>(PointsPlain{positions, volumes}, n,
+  launch_rows(n, false, [&](auto large, unsigned blocks) {
+    k_csr_force<decltype(large)::value><<<blocks, kRowThreads, 0, s>>>(PointsPlain{positions, volumes}, n,
         row_ptr, col, M, bond_damage, force);
   });
   VPD_CUDA(cudaGetLastError());
@@ -636,13 +637,13 @@ static int shape_tensor_inverse(const double *positions, const double *volumes, 
   VPD_CUDA(cudaMemsetAsync(st, 0, sizeof(unsigned), s));
   if (rec) {
     k_pack_points<false><<<blocks(n), 128, 0, s>>>(positions, volumes, nullptr, n, rec, nullptr);
-    launch_rows(n, [&](auto large) {
-      k_csr_shape_inverse<decltype(large)::value><<<row_blocks(n), kRowThreads, 0, s>>>(Packed{rec}, n, row_ptr,
+    launch_rows(n, true, [&](auto large, unsigned blocks) {
+      k_csr_shape_inverse<decltype(large)::value><<<blocks, kRowThreads, 0, s>>>(Packed{rec}, n, row_ptr,
           col, kinv, st);
     });
   } else {
-    launch_rows(n, [&](auto large) {
-      k_csr_shape_inverse<decltype(large)::value><<<row_blocks(n), kRowThreads, 0, s>>>(PointsPlain{positions,
+    launch_rows(n, false, [&](auto large, unsigned blocks) {
+      k_csr_shape_inverse<decltype(large)::value><<<blocks, kRowThreads, 0, s>>>(PointsPlain{positions,
           volumes}, n, row_ptr, col, kinv, st);
     });
   }
@@ -657,13 +658,13 @@ static int deformation_gradients(const double *positions, const double *displace
     return VPD_OK;
   if (rec) {
     k_pack_points<false><<<blocks(n), 128, 0, s>>>(positions, volumes, displacement, n, rec, rec + n);
-    launch_rows(n, [&](auto large) {
-      k_csr_deformation<decltype(large)::value><<<row_blocks(n), kRowThreads, 0, s>>>(Packed{rec}, Packed{rec + n},
+    launch_rows(n, true, [&](auto large, unsigned blocks) {
+      k_csr_deformation<decltype(large)::value><<<blocks, kRowThreads, 0, s>>>(Packed{rec}, Packed{rec + n},
           n, row_ptr, col, kinv, defgrad);
     });
   } else {
-    launch_rows(n, [&](auto large) {
-      k_csr_deformation<decltype(large)::value><<<row_blocks(n), kRowThreads, 0, s>>>(PointsPlain{positions,
+    launch_rows(n, false, [&](auto large, unsigned blocks) {
+      k_csr_deformation<decltype(large)::value><<<blocks, kRowThreads, 0, s>>>(PointsPlain{positions,
           volumes}, VectorsPlain<false>{positions, displacement}, n, row_ptr, col, kinv, defgrad);
     });
   }
@@ -681,13 +682,13 @@ static int damage_update(const double *positions, const double *displacement, co
   const StretchTest test = stretch_test(initiation, failure);
   if (rec) {
     k_pack_points<true><<<blocks(n), 128, 0, s>>>(positions, volumes, displacement, n, rec, rec + n);
-    launch_rows(n, [&](auto large) {
-      k_csr_damage<decltype(large)::value><<<row_blocks(n), kRowThreads, 0, s>>>(Packed{rec}, Packed{rec + n}, n,
+    launch_rows(n, true, [&](auto large, unsigned blocks) {
+      k_csr_damage<decltype(large)::value><<<blocks, kRowThreads, 0, s>>>(Packed{rec}, Packed{rec + n}, n,
           row_ptr, col, test, bond_damage, damage_index);
     });
   } else {
-    launch_rows(n, [&](auto large) {
-      k_csr_damage<decltype(large)::value><<<row_blocks(n), kRowThreads, 0, s>>>(PointsPlain{positions, volumes},
+    launch_rows(n, false, [&](auto large, unsigned blocks) {
+      k_csr_damage<decltype(large)::value><<<blocks, kRowThreads, 0, s>>>(PointsPlain{positions, volumes},
           VectorsPlain<true>{positions, displacement}, n, row_ptr, col, test, bond_damage, damage_index);
     });
   }

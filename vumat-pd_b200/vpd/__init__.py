@@ -329,13 +329,12 @@ def build_neighbor_list(positions, horizon: float):
     return row_ptr, col[: total.value]
 
 
-def _records(positions, col, vectors, points, bonds):
-    """Room for the packed records of a bond sum over `vectors` vectors a point, for bodies of `points` points and
-    `bonds` bonds a point or more: None for smaller ones and where there is no memory (the sums then read the arrays
-    as they are)."""
+def _records(positions, col, vectors, bonds):
+    """Room for the packed records of a bond sum over `vectors` vectors a point, where rows hold `bonds` bonds on average
+    or more: None for shorter ones and where there is no memory (the sums then read the arrays as they are)."""
     import torch
     n = positions.shape[0]
-    if n < points or col.numel() < bonds * n:
+    if col.numel() < bonds * n:
         return None
     try:
         return torch.empty((vectors * n, 4), dtype=torch.float64, device=positions.device)
@@ -345,9 +344,10 @@ def _records(positions, col, vectors, points, bonds):
 
 def shape_tensor_inverse(positions, volumes, row_ptr, col):
     import torch
-    out = torch.empty((positions.shape[0], 9), dtype=torch.float64, device=positions.device)
-    args = (_ptr(positions), _ptr(volumes), positions.shape[0], _ptr(row_ptr), _ptr(col), _ptr(out))
-    records = _records(positions, col, 1, 150_000, 64)
+    n = positions.shape[0]
+    out = torch.empty((n, 9), dtype=torch.float64, device=positions.device)
+    args = (_ptr(positions), _ptr(volumes), n, _ptr(row_ptr), _ptr(col), _ptr(out))
+    records = _records(positions, col, 1, 64) if n >= 150_000 else None
     _check(library().vpd_shape_tensor_inverse(*args, _stream()) if records is None else
            library().vpd_shape_tensor_inverse_packed(*args, _ptr(records), _stream()))
     return out
@@ -355,10 +355,10 @@ def shape_tensor_inverse(positions, volumes, row_ptr, col):
 
 def deformation_gradients(positions, displacement, volumes, row_ptr, col, kinv):
     import torch
-    out = torch.empty((positions.shape[0], 9), dtype=torch.float64, device=positions.device)
-    args = (_ptr(positions), _ptr(displacement), _ptr(volumes), positions.shape[0], _ptr(row_ptr), _ptr(col),
-            _ptr(kinv), _ptr(out))
-    records = _records(positions, col, 2, 150_000, 64)
+    n = positions.shape[0]
+    out = torch.empty((n, 9), dtype=torch.float64, device=positions.device)
+    args = (_ptr(positions), _ptr(displacement), _ptr(volumes), n, _ptr(row_ptr), _ptr(col), _ptr(kinv), _ptr(out))
+    records = _records(positions, col, 2, 64) if n >= 150_000 else None
     _check(library().vpd_deformation_gradients(*args, _stream()) if records is None else
            library().vpd_deformation_gradients_packed(*args, _ptr(records), _stream()))
     return out
@@ -455,10 +455,11 @@ MLP_PARAMS = 37264
 def damage_update(positions, displacement, volumes, row_ptr, col, initiation, failure,
                   bond_damage):
     import torch
-    idx = torch.empty(positions.shape[0], dtype=torch.float64, device=positions.device)
-    args = (_ptr(positions), _ptr(displacement), _ptr(volumes), positions.shape[0], _ptr(row_ptr), _ptr(col),
-            initiation, failure, _ptr(bond_damage), _ptr(idx))
-    records = _records(positions, col, 2, 16_000, 24)
+    n = positions.shape[0]
+    idx = torch.empty(n, dtype=torch.float64, device=positions.device)
+    args = (_ptr(positions), _ptr(displacement), _ptr(volumes), n, _ptr(row_ptr), _ptr(col), initiation, failure,
+            _ptr(bond_damage), _ptr(idx))
+    records = _records(positions, col, 2, 24) if n >= 16_000 else None
     _check(library().vpd_damage_update(*args, _stream()) if records is None else
            library().vpd_damage_update_packed(*args, _ptr(records), _stream()))
     return idx
