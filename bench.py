@@ -154,11 +154,11 @@ class ClockSampler:
 FP32_FLOP_PER_BOND = {"deformation": 27, "force": 24}
 FP32_NOMINAL_TFLOPS = 148 * 128 * 2 * 1.965e9 / 1e12  # 148 SMs x 128 FP32 lanes x FMA at 1965 MHz
 LIMITER = {
-    "deformation": "FP32 issue and latency: issue 49 % active at 16 warps per SM, math-pipe throttle, "
-                   "76 B/pt DRAM (ncu)",
-    "force": "L1 gathers: L1 data-pipe wavefronts 64 % of peak, issue 49 % active, long-scoreboard stalls, "
-             "140 B/pt DRAM (ncu)",
-    "material": "FP64 and memory latency at 12 warps per SM; DRAM traffic 810 of its 964 algorithmic B/pt (ncu)",
+    "deformation": "latency and instruction issue at 16 warps per SM: issue 49 % active, L1 35 % of peak, "
+                   "long-scoreboard and fixed-latency stalls (ncu, 250,000 points with damage)",
+    "force": "L1 gathers: L1 71 % of peak, issue 51 % active, long-scoreboard stalls (ncu, 250,000 points with damage)",
+    "material": "latency of its memory reads and of the FP64 chain at 16 warps per SM: DRAM 35 % of peak, issue 29 % "
+                "active, long-scoreboard stalls (ncu, 250,000 points with damage)",
     "integrate": "memory latency and the two-level diagnostics reduction (ncu)",
 }
 

@@ -246,10 +246,11 @@ int vpd_checkpoint_load(vpd_handle *h, const void *buffer, int64_t bytes);
 
 /* Sorted neighbour lists of n points (positions n*3 doubles). First call with col == NULL:
    fills row_ptr[n+1] and *total. Second call with col of *total ints fills the rows. Both
-   calls synchronise the stream. Scratch memory, here and in vpd_force_density and the network functions,
-   comes from a stream-ordered pool of the library, which keeps at most 256 MiB idle per device between
-   calls: vpd_release_workspace gives that back, every vpd_destroy all but 32 MiB. The other module functions allocate nothing (but one word per host thread, on its first
-   call). */
+   calls synchronise the stream. Scratch memory, here and in vpd_force_density and the network
+   functions, comes from a stream-ordered pool of the library, which keeps at most 256 MiB idle
+   per device between calls: vpd_release_workspace gives that back, every vpd_destroy all but
+   32 MiB. The other module functions allocate nothing (but one word per host thread, on its
+   first call of those that report singular points). */
 int vpd_build_neighbor_list(const double *positions, int64_t n, double horizon,
                             int64_t *row_ptr, int32_t *col, int64_t *total, void *stream);
 /* Gives the idle memory of the library's pool on the current device back to the device. */

@@ -44,8 +44,8 @@ __device__ __forceinline__ StagedWeights stage_weights(unsigned char *s, const M
 // layer reads them as its first operand, so its batch rows are lanes again.
 // What bounds it is the epilogue: 384 tanh per row at 16 per SM and clock, 83 us for 1M rows,
 // against 43 us of tensor work and 20 us of memory traffic. Measured on a B200: 137 us for 1M rows (152 with
-// the batch rows along the lanes; 490 with a block per tile that staged the 72 KB of weights each time), the
-// tanh unit about 60 % busy; without its tanh the kernel takes 106 us, without its tensor work 130. Two warps a
+// the batch rows along the lanes; 490 with a block per tile that staged the 72 KB of weights each time), 60 %
+// of it the tanh unit's own time; without its tanh the kernel takes 106 us, without its tensor work 130. Two warps a
 // TMEM quarter (142 us) and two half tiles a group in turn (148) have shorter waits but more of them.
 constexpr int kGroups = 4;
 constexpr size_t kFwdSmem = kWeightBytes + kGroups * 32768 + (kGroups + 1) * 16 + 4 * kBiasFloats;

@@ -24,8 +24,8 @@ __global__ void k_pack_positions(const double *pos, int64_t n, double4 *xv) {
 // A row's bonds are dealt out to 1, 2, 4 or 8 lanes, whose partial sums a fixed shuffle tree joins. Many lanes read a
 // long row's neighbour indices as consecutive words and fill the GPU where points are few; with one lane per row the
 // lanes of a warp share the lines of short rows, and neighbouring rows of a regular lattice gather consecutive points.
-// The next bond's index is read before the current bond's gathers are used. What bounds the sums is L1 (93 % of its
-// wavefronts at 154,000 jittered points): the gathers of 32 bonds touch about eight lines a load in any arrangement
+// The next bond's index is read before the current bond's gathers are used. What bounds the sums is L1 (90 to 96 % of
+// its throughput at 154,000 jittered points): the gathers of 32 bonds touch about eight lines a load in any arrangement
 // tried.
 constexpr int kRowThreads = 256;
 
