@@ -69,3 +69,12 @@ def test_neighbour_lists_of_one_cell_take_at_most_six_times_those_of_many():
     pos = np.stack(np.meshgrid(*[np.arange(15.0)] * 3, indexing="ij"), -1).reshape(-1, 3)
     x = torch.as_tensor(pos).cuda()
     assert seconds(lambda: vpd.build_neighbor_list(x, 30.0)) <= 6.0 * seconds(lambda: vpd.build_neighbor_list(x, 3.015))
+
+
+def test_neighbour_lists_of_plates_and_lines_take_less_time_than_those_of_a_body():
+    """1M points at two spacings: 12 bonds and nine cells to look into in a plate, 4 and 3 in a line, 31 and 27 in a body."""
+    x, y, z = (torch.as_tensor(np.stack(np.meshgrid(*[np.arange(float(k)) for k in shape], indexing="ij"), -1).reshape(-1, 3)).cuda()
+               for shape in ((1000, 1000, 1), (100, 100, 100), (1000000, 1, 1)))
+    body = seconds(lambda: vpd.build_neighbor_list(y, 2.015), 5)
+    assert seconds(lambda: vpd.build_neighbor_list(x, 2.015), 5) <= 0.95 * body
+    assert seconds(lambda: vpd.build_neighbor_list(z, 2.015), 5) <= 0.95 * body

@@ -29,3 +29,15 @@ def test_lists_equal_the_oracle(kind):
     row_ptr, col = vpd.build_neighbor_list(torch.as_tensor(np.ascontiguousarray(pos)).cuda(), horizon)
     assert np.array_equal(row_ptr.cpu().numpy(), want_ptr)
     assert np.array_equal(col.cpu().numpy(), want_col[:len(col)])
+
+
+# points a cell on either side of where the search by cell begins, in bodies, plates and lines
+@pytest.mark.parametrize("shape,horizon", [((14, 14, 14), 1.7), ((14, 14, 14), 1.72), ((14, 14, 14), 2.015),
+                                           ((60, 40, 1), 2.8), ((60, 40, 1), 2.9), ((60, 40, 1), 3.015),
+                                           ((1, 3000, 1), 13.5), ((1, 3000, 1), 14.5), ((4, 4, 4), 9.0)])
+def test_lists_on_either_side_of_the_search_by_cell(shape, horizon):
+    pos = np.stack(np.meshgrid(*[np.arange(float(k)) for k in shape], indexing="ij"), -1).reshape(-1, 3)
+    want_ptr, want_col = O.neighbor_list(np.ascontiguousarray(pos), horizon)
+    row_ptr, col = vpd.build_neighbor_list(torch.as_tensor(pos).cuda(), horizon)
+    assert np.array_equal(row_ptr.cpu().numpy(), want_ptr)
+    assert np.array_equal(col.cpu().numpy(), want_col[:len(col)])

@@ -369,7 +369,11 @@ __global__ void k_nb_fill(const double4 *xv, int64_t n, const long long *cc, Gri
 
 // ------------------------------------------------------------------ search by cell
 constexpr int kMaxCandidates = 4096;  // 99 KB of shared memory
-constexpr int kMinCellPoints = 4;
+// Points per cell from which on a block per cell (38 ns each) is quicker than a warp per point (11, 5.5 and 2.8 ns a point in
+// bodies, plates and lines of 1M points, which look into 27, 9 and 3 cells), by the number of directions with more
+// than one cell. Lists of 1M points, milliseconds, by cell | by point: 3, 5.7 and 11.7 points a cell of a body 14.1 | 11.3,
+// 8.9 | 12.2 and 6.2 | 13.2, 6 and 9 of a plate 6.9 | 5.7 and 5.4 | 6.0, 9 and 20 of a line 3.8 | 3.0 and 2.5 | 3.6.
+constexpr int kMinCellPoints[4] = {1, 14, 8, 5};
 constexpr int kCellThreads = 256;
 
 // The nine runs of `sorted` that hold the points of the 27 cells around cell c (the three along the last
@@ -773,7 +777,8 @@ int neighbor_count(const double4 *xv, int64_t n, double horizon, int64_t *row_pt
   // the search by cell needs a few points a cell, candidates that fit shared memory, and a cell width whose
   // reciprocal and square are ordinary numbers
   grid.candidates = 0;
-  if (grid.ncells * kMinCellPoints <= n && grid.cell_width > 1.0e-100 && grid.cell_width < 1.0e100) {
+  const int directions = (grid.dims[0] > 1) + (grid.dims[1] > 1) + (grid.dims[2] > 1);
+  if (grid.ncells * kMinCellPoints[directions] <= n && grid.cell_width > 1.0e-100 && grid.cell_width < 1.0e100) {
     k_cell_load<<<(unsigned)((grid.ncells + 255) / 256), 256, 0, s>>>(grid.ncells, g, scr.cell_start, scr.reduce + 8);
     VPD_CUDA(cudaMemcpyAsync(red, scr.reduce, sizeof red, cudaMemcpyDeviceToHost, s));
     VPD_CUDA(cudaStreamSynchronize(s));
