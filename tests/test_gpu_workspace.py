@@ -58,7 +58,7 @@ def free_bytes():
 
 def loaded():
     """Every kernel of the step's calls loaded (CUDA loads them lazily)."""
-    for n in (64, 60_000):
+    for n in (64, 65_000):
         body = Step(n)
         body.shape(), body.deformation(), body.damage(), body.noalloc_force()
 

@@ -37,18 +37,20 @@ constexpr int kRowThreads = 256;
 // with 28, 38 | 87 | 36 and 73 | 88 | 53; 1M points with 6, 61 | 200 | 63 and 52 | 163 | 52, with 118,
 // 548 | 770 | 533 and 1210 | 838 | 651; 108,000 points with 229, 198 | 133 | 122 and 394 | 169 | 164; the force sum of
 // 1M points with 6, eight always | now, 263 | 145.
-// With packed records (calls over long rows) eight lanes serve up to 100,000 points: damage of 50,000 points with 109
-// bonds, four | eight lanes 47 | 41, of 82,000 with 230, 135 | 124, of 108,000 with 229, 156 | 152.
-constexpr int64_t kLargeBody = 40000, kLargePackedBody = 100000, kShortRowBody = 150000, kTwoLaneGrid = 500000;
+// With packed records (calls over long rows) eight lanes serve up to 100,000 points, in the shape tensors up to 500,000:
+// damage of 50,000 points with 109 bonds, four | eight lanes 47 | 41, of 82,000 with 230, 135 | 124, of 108,000 with 229,
+// 156 | 152; shape tensors of 154,000 with 230, 158 | 145, of 250,000 with 239, 205 | 205, of 1M with 245, 665 | 723.
+constexpr int64_t kLargeBody = 60000, kLargePackedBody = 100000, kLargePackedShapes = 500000;
+constexpr int64_t kShortRowBody = 150000, kTwoLaneGrid = 500000;
 __device__ __forceinline__ int row_lanes(int64_t n, const int64_t *row_ptr) {
   const int64_t bonds = __ldg(row_ptr + n) - __ldg(row_ptr);
   if (n < kShortRowBody)
     return bonds < 24 * n ? 2 : 4;
   return bonds < 20 * n ? 1 : (bonds < 64 * n ? 2 : 4);
 }
-// launch(LARGE, blocks): the sums' kernels come in both forms.
-template <typename F> static void launch_rows(int64_t n, bool packed, F &&launch) {
-  const bool large = n >= (packed ? kLargePackedBody : kLargeBody);
+// launch(LARGE, blocks): the sums' kernels come in both forms, LARGE from large_body points on.
+template <typename F> static void launch_rows(int64_t n, int64_t large_body, F &&launch) {
+  const bool large = n >= large_body;
   const int64_t lanes = !large ? 8 : (n < kTwoLaneGrid ? 4 : 2);
   const unsigned blocks = (unsigned)((n * lanes + kRowThreads - 1) / kRowThreads);
   if (large)
@@ -612,7 +614,7 @@ int launch_csr_force(const double *positions, const double *volumes, int64_t n, 
                      const int32_t *col, const double *kinv, const double *defgrad, const double *cauchy_stress,
                      const double *bond_damage, double *force, double *M, unsigned *status, cudaStream_t s) {
   k_csr_force_map<<<blocks(n), 128, 0, s>>>(cauchy_stress, defgrad, kinv, n, M, status);
-  launch_rows(n, false, [&](auto large, unsigned blocks) {
+  launch_rows(n, kLargeBody, [&](auto large, unsigned blocks) {
     k_csr_force<decltype(large)::value><<<blocks, kRowThreads, 0, s>>>(PointsPlain{positions, volumes}, n,
         row_ptr, col, M, bond_damage, force);
   });
@@ -637,12 +639,12 @@ static int shape_tensor_inverse(const double *positions, const double *volumes, 
   VPD_CUDA(cudaMemsetAsync(st, 0, sizeof(unsigned), s));
   if (rec) {
     k_pack_points<false><<<blocks(n), 128, 0, s>>>(positions, volumes, nullptr, n, rec, nullptr);
-    launch_rows(n, true, [&](auto large, unsigned blocks) {
+    launch_rows(n, kLargePackedShapes, [&](auto large, unsigned blocks) {
       k_csr_shape_inverse<decltype(large)::value><<<blocks, kRowThreads, 0, s>>>(Packed{rec}, n, row_ptr,
           col, kinv, st);
     });
   } else {
-    launch_rows(n, false, [&](auto large, unsigned blocks) {
+    launch_rows(n, kLargeBody, [&](auto large, unsigned blocks) {
       k_csr_shape_inverse<decltype(large)::value><<<blocks, kRowThreads, 0, s>>>(PointsPlain{positions,
           volumes}, n, row_ptr, col, kinv, st);
     });
@@ -658,12 +660,12 @@ static int deformation_gradients(const double *positions, const double *displace
     return VPD_OK;
   if (rec) {
     k_pack_points<false><<<blocks(n), 128, 0, s>>>(positions, volumes, displacement, n, rec, rec + n);
-    launch_rows(n, true, [&](auto large, unsigned blocks) {
+    launch_rows(n, kLargePackedBody, [&](auto large, unsigned blocks) {
       k_csr_deformation<decltype(large)::value><<<blocks, kRowThreads, 0, s>>>(Packed{rec}, Packed{rec + n},
           n, row_ptr, col, kinv, defgrad);
     });
   } else {
-    launch_rows(n, false, [&](auto large, unsigned blocks) {
+    launch_rows(n, kLargeBody, [&](auto large, unsigned blocks) {
       k_csr_deformation<decltype(large)::value><<<blocks, kRowThreads, 0, s>>>(PointsPlain{positions,
           volumes}, VectorsPlain<false>{positions, displacement}, n, row_ptr, col, kinv, defgrad);
     });
@@ -682,12 +684,12 @@ static int damage_update(const double *positions, const double *displacement, co
   const StretchTest test = stretch_test(initiation, failure);
   if (rec) {
     k_pack_points<true><<<blocks(n), 128, 0, s>>>(positions, volumes, displacement, n, rec, rec + n);
-    launch_rows(n, true, [&](auto large, unsigned blocks) {
+    launch_rows(n, kLargePackedBody, [&](auto large, unsigned blocks) {
       k_csr_damage<decltype(large)::value><<<blocks, kRowThreads, 0, s>>>(Packed{rec}, Packed{rec + n}, n,
           row_ptr, col, test, bond_damage, damage_index);
     });
   } else {
-    launch_rows(n, false, [&](auto large, unsigned blocks) {
+    launch_rows(n, kLargeBody, [&](auto large, unsigned blocks) {
       k_csr_damage<decltype(large)::value><<<blocks, kRowThreads, 0, s>>>(PointsPlain{positions, volumes},
           VectorsPlain<true>{positions, displacement}, n, row_ptr, col, test, bond_damage, damage_index);
     });
