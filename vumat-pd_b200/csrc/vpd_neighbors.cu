@@ -419,9 +419,11 @@ __global__ void k_cell_load(int64_t ncells, GridDev g, const int64_t *cell_start
 // a few cells, or a cluster among sparse points); each block then searches for some of the cell's points, 32 or more, and
 // sorts the candidates again. The two calls that build the list, microseconds, a block per cell | so: 3,375 points in one
 // cell 9938 | 467, 2,744 points in eight cells 5376 | 442 (3200 both with a warp per point and allocations in the calls).
-static int cell_blocks(const unsigned long long *load) {
+// At most 65,536 blocks in all: those without points end at once, but each takes its nanoseconds.
+static int cell_blocks(const unsigned long long *load, int64_t ncells) {
   const unsigned long long share = std::max(load[3] / 148, 32 * load[0]);
-  return (int)std::max(1ull, std::min(load[2] / share, (load[1] + 31) / 32));
+  const unsigned long long wanted = std::min(load[2] / share, (load[1] + 31) / 32);
+  return (int)std::max(1ull, std::min(wanted, (unsigned long long)(65536 / ncells)));
 }
 
 // Ascending bitonic sort of `width` (a power of two, at least 32) shared-memory ints by the whole block.
@@ -783,7 +785,7 @@ int neighbor_count(const double4 *xv, int64_t n, double horizon, int64_t *row_pt
     VPD_CUDA(cudaMemcpyAsync(red, scr.reduce, sizeof red, cudaMemcpyDeviceToHost, s));
     VPD_CUDA(cudaStreamSynchronize(s));
     if (red[8] <= (unsigned long long)kMaxCandidates)
-      grid.candidates = (int)red[8], grid.cell_blocks = cell_blocks(red + 8);
+      grid.candidates = (int)red[8], grid.cell_blocks = cell_blocks(red + 8, grid.ncells);
   }
   if (grid.candidates) {
     if ((rc = launch_cells<false>(xv, grid, scr, nullptr, nullptr, s)))
